@@ -642,17 +642,17 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // Byte sizes of the arena regions, in carve order.
 struct ArenaPlan {
     size_t control, sims, simout, chunk, tiles, keys, vals, sbody, base, cell_u, groups,
-        cell_d, cell_child, cell_parent, cell_counter, err, stats;
+        cell_d, cell_child, cell_parent, agg_words, err, stats;
     size_t total() const {
         return control + sims + simout + chunk + tiles + 2 * keys + 2 * vals + sbody + base +
-               cell_u + groups + cell_d + cell_child + cell_parent + cell_counter +
+               cell_u + groups + cell_d + cell_child + cell_parent + agg_words +
                err + stats;
     }
 };
 
 static ArenaPlan plan_arena(const Layout& L, uint32_t nsims) {
     ArenaPlan a;
-    a.control = align256(4ull * nsims * 4 + 4ull * nsims * kRadixPasses * kRadixDigits + 4ull * 16 +
+    a.control = align256(4ull * nsims * 4 + 4ull * nsims * kRadixPasses * kRadixDigits + 4ull * 32 +
                          4ull * kRadixPasses * L.ntiles * kRadixDigits) +
                 align256(8ull * L.nscan_tiles);
     a.sims = align256(sizeof(SimDesc) * nsims);
@@ -668,7 +668,7 @@ static ArenaPlan plan_arena(const Layout& L, uint32_t nsims) {
     a.cell_d = align256(32ull * L.cells);
     a.cell_child = align256(16ull * L.cells);
     a.cell_parent = align256(4ull * L.cells);
-    a.cell_counter = align256(4ull * L.cells);
+    a.agg_words = align256(4ull * L.cells);
     a.err = 256;
     a.stats = 256;
     return a;
@@ -758,7 +758,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.hist = (uint32_t*)cp;
     cp += 4ull * count * kRadixPasses * kRadixDigits;
     bb.counters = (uint32_t*)cp;
-    cp += 4ull * 16;
+    cp += 4ull * 32;
     bb.sort_flags = (uint32_t*)cp;
     cp += 4ull * kRadixPasses * L.ntiles * kRadixDigits;
     bb.scan_flags = (unsigned long long*)((char*)b->control +
@@ -779,7 +779,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.cell_d = (double4*)take(A.cell_d);
     bb.cell_child = (uint4*)take(A.cell_child);
     bb.cell_parent = (uint32_t*)take(A.cell_parent);
-    bb.cell_counter = (uint32_t*)take(A.cell_counter);
+    bb.agg_words = (uint32_t*)take(A.agg_words);
     bb.err = (uint32_t*)take(A.err);
     bb.force_stats = (unsigned long long*)take(A.stats);
     bb.nsims = count;

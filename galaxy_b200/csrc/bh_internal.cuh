@@ -53,7 +53,7 @@ struct SimDesc {
 // Per-simulation results of the last rebuild.
 struct SimOut {
     double cx, cy, half;  // f64 root bounds (nbody/src/lib.rs:137-154)
-    double reserved;
+    double crit0;         // root width / theta (+inf at theta 0)
 };
 
 // Traversal record of one cell, its slot in the parent's node group
@@ -93,7 +93,8 @@ struct BatchBuffers {
     // zeroed once per rebuild (one memset): control block
     uint32_t* minmax;      // nsims * 4 (atomicMax of encoded floats; mins stored inverted)
     uint32_t* hist;        // nsims * 4 * 256
-    uint32_t* counters;    // 16: radix tile counters (one per pass, <= 8), scan tile counter [8]
+    uint32_t* counters;    // 32: radix tile counters (one per pass, <= 8), scan tile counter [8],
+                           // cells that span outer cuts [16]
     uint32_t* sort_flags;  // 4 * ntiles * 256
     unsigned long long* scan_flags;  // nscan_tiles
     // transient per rebuild
@@ -111,7 +112,7 @@ struct BatchBuffers {
                         // com_x, com_y (float2 bits): com - (float)com
     uint4* cell_child;  // children (global cell indices)
     uint32_t* cell_parent;
-    uint32_t* cell_counter;
+    uint32_t* agg_words;  // the aggregates' cuts and list of cells across outer cuts
     // persistent
     uint32_t* err;                   // error bits
     unsigned long long* force_stats; // 4 counters

@@ -15,7 +15,8 @@
 //                 reference's recursive preorder, nbody/src/flat.rs:127-177)
 //   k_cells       ranges, children, skip pointers of every cell
 //   k_aggregate   bottom-up f64 mass / centre of mass, identical arithmetic
-//                 and order to nbody/src/flat.rs:179-215
+//                 and order to nbody/src/flat.rs:179-215, in blocks of about
+//                 256 positions; k_aggregate_spans the cells across blocks
 //   k_traverse    lane-parallel theta-MAC walk over node groups with per-warp
 //                 interaction lists (nbody/src/flat.rs:270-346 decisions per
 //                 body), f32 forces, exact f64 MAC in the guard band
@@ -97,6 +98,11 @@ __device__ __forceinline__ RootBounds root_bounds_from(const uint32_t* mm) {
     r.cy = __dmul_rn(__dadd_rn(min_y, max_y), 0.5);
     r.half = __dadd_rn(__dmul_rn(span, 0.500000000001), 1e-12);
     return r;
+}
+
+// Root width / theta, +inf at theta = 0 (every cell opens).
+__device__ __forceinline__ double crit_of(double root_half, double theta) {
+    return theta > 0.0 ? __dmul_rn(root_half, 2.0) / theta : INFINITY;
 }
 
 // nbody/src/flat.rs:82-87
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const SimDesc* __rest
         simout[t.sim].cx = rb.cx;
         simout[t.sim].cy = rb.cy;
         simout[t.sim].half = rb.half;
+        simout[t.sim].crit0 = crit_of(rb.half, sd.theta);
     }
 #pragma unroll
     for (int k = 0; k < kMortonItems; ++k) {
@@ -801,12 +808,34 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(
 // bases of the next kCellsWin positions sit in shared memory, so the range
 // searches of almost every cell (all but the few that span more than the
 // window) never touch global memory.
-// Positions per k_aggregate block: cells whose range crosses a multiple of it
-// are finished by cross-block climbs (the only users of the cell counters).
+// k_aggregate's blocks own [cut_b, cut_b+1): cut b is the first position of the
+// kAggCutWindow ones from b * kAggPositions on that starts a group of the least
+// depth, so that few cells, and only shallow ones, span two blocks.
 #ifndef GBH_AGG_POSITIONS
 #define GBH_AGG_POSITIONS 256
 #endif
-constexpr uint32_t kAggBlockPositions = GBH_AGG_POSITIONS;
+#ifndef GBH_AGG_CUT_WINDOW
+#define GBH_AGG_CUT_WINDOW 128
+#endif
+constexpr uint32_t kAggPositions = GBH_AGG_POSITIONS;
+constexpr uint32_t kAggCutWindow = GBH_AGG_CUT_WINDOW;
+// The cuts (one more than blocks, from k_cells) and the internal cells that
+// span one (from k_aggregate), as (cell, depth << 26 | simulation) at most one
+// per cut and depth.  Every kAggRange-th cut is an outer cut: a list per range
+// between two of them, and one of the cells that span an outer cut.
+#ifndef GBH_AGG_RANGE
+#define GBH_AGG_RANGE 128
+#endif
+constexpr uint32_t kAggRange = GBH_AGG_RANGE;
+constexpr uint32_t kAggRangeCells = 16u * kAggRange;
+struct AggPlan {
+    uint32_t* cuts;
+    uint32_t* inner_n;  // [range], zeroed by k_cells
+    uint32_t* outer_n;  // zeroed with the control block
+    uint2* inner;       // [range][kAggRangeCells]
+    uint2* outer;       // [16 ranges]
+    uint32_t blocks, ranges;
+};
 #ifndef GBH_CELLS_THREADS
 #define GBH_CELLS_THREADS 256
 #endif
@@ -905,13 +934,14 @@ __global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(c
                                                          const uint32_t* __restrict__ base,
                                                          uint4* cell_u,
                                                          uint4* cell_child, uint32_t* cell_parent,
-                                                         uint32_t* cell_counter, CellRec* groups,
+                                                         AggPlan plan, CellRec* groups,
                                                          uint32_t* err) {
     wait_for_predecessor();
     __shared__ uint32_t s_code[kCellsWin];
     __shared__ uint32_t s_base[kCellsWin + 1];
     __shared__ uint8_t s_owner[kCellsThreads * kMaxChain];  // cell -> position in block
     __shared__ uint16_t s_end[kCellsThreads * kMaxChain];   // cell -> min(end - P0, 0xffff)
+    __shared__ uint32_t s_cut;  // least dmin << 16 | position - P0 of the cut window
     const uint32_t t = threadIdx.x;
     const uint32_t P0 = blockIdx.x * kCellsThreads;
     for (uint32_t j = t; j <= kCellsWin; j += kCellsThreads) {
@@ -930,7 +960,27 @@ __global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(c
         const uint32_t c0 = s_base[t] - kb, c = s_base[t + 1] - s_base[t];
         for (uint32_t j = 0; j < c; ++j) s_owner[c0 + j] = (uint8_t)t;
     }
+    // this block's cut: the first position of the window whose dmin is least
+    if (t == 0) s_cut = kNone;
     __syncthreads();
+    if (t < kAggCutWindow) {
+        const uint32_t p = P0 + t;
+        uint32_t dmin = 0xffu;  // past the last position: no cut
+        if (p < npos) {
+            const SimDesc& sd = sims[chunk_sim[p >> 5]];
+            dmin = 0;
+            if (p != sd.off && p < sd.off + sd.n)
+                dmin = shared_levels(t ? s_code[t - 1u] : codes[p - 1u], s_code[t]) + 1u;
+        }
+        const uint32_t key = __reduce_min_sync(kFull, dmin << 16 | t);
+        if (lane_id() == 0) atomicMin(&s_cut, key);
+    }
+    __syncthreads();
+    if (t == 0) {
+        plan.cuts[blockIdx.x] = P0 + (s_cut & 0xffffu);
+        if (P1 == npos) plan.cuts[blockIdx.x + 1u] = npos;
+        if (blockIdx.x < plan.ranges) plan.inner_n[blockIdx.x] = 0;
+    }
     const CellsWindow w{s_code, s_base, codes, base, P0};
     const uint4 absent = make_uint4(0u, 0u, 0u, kNone);  // u.z == 0: no child in this slot
     // Position, depth and deepest chain depth of cell k of this block.
@@ -969,8 +1019,6 @@ __global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(c
             rg[3].u = absent;
         }
         cell_u[k] = make_uint4(end, w.base_at(end), p, d);
-        // counters serve only cells that span aggregate blocks (cross-block climbs)
-        if ((p / kAggBlockPositions) != ((end - 1u) / kAggBlockPositions)) cell_counter[k] = 0;
         s_end[k - kb] = (uint16_t)min(end - P0, 0xffffu);
     }
     __syncthreads();
@@ -1020,13 +1068,11 @@ __global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(c
 #pragma unroll
             for (uint32_t qd = 0; qd < 4; ++qd) {
                 const uint32_t child = chp[qd];
-                if (child == kNone) {
-                    groups[4ull * k + qd].u = absent;
-                } else if (child < capacity) {
+                if (child == kNone) continue;
+                if (child < capacity)
                     cell_parent[child] = k;
-                } else {
+                else
                     set_err(err, kErrCapacity);
-                }
             }
         }
         cell_child[k] = ch;
@@ -1043,26 +1089,25 @@ __global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(c
 // linear in d^2: |d2_f32 - d^2| <= d^2 * r + u*C*crit, r = u*C/crit + 4u.
 // So d2_f32 > hi proves "approximate" and d2_f32 < lo proves "open" (with a
 // 4x margin and 1e-4 relative slack); in between the traversal decides in f64.
-__device__ __forceinline__ void mac_band(double width, double theta, float com_x, float com_y,
+// With r = u C/crit + 4 u the slack 4 r + 1e-4 on crit^2 and 4 u C crit beside
+// it make crit^2 (16 u + 1e-4) + 8 u C crit on either side of crit^2; here in
+// f32 with every rounding away from crit^2, so the band only widens.
+struct Crit {
+    float up, down;  // width/theta rounded up and down; +inf at theta = 0
+};
+__device__ __forceinline__ Crit crit_f32(double crit) {
+    return Crit{__double2float_ru(crit), __double2float_rd(crit)};
+}
+__device__ __forceinline__ void mac_band(Crit root, uint32_t depth, float com_x, float com_y,
                                          float* lo, float* hi) {
-    if (!(theta > 0.0)) {  // theta = 0: every cell opens
-        *lo = INFINITY;
-        *hi = INFINITY;
-        return;
-    }
-    const double crit = width / theta;
-    const double crit2 = crit * crit;
-    if (!(crit2 < 1e38)) {  // beyond any f32 distance: always open
-        *lo = INFINITY;
-        *hi = INFINITY;
-        return;
-    }
-    const double u = 5.9604644775390625e-8;
-    const double C = fabs((double)com_x) + fabs((double)com_y);
-    const double r = u * C / crit + 4.0 * u;
-    const double slack = 4.0 * r + 1e-4;
-    *hi = __double2float_ru(crit2 * (1.0 + slack) + 4.0 * u * C * crit);
-    *lo = __double2float_rd(crit2 * (1.0 - slack) - 4.0 * u * C * crit);
+    const float scale = __uint_as_float((127u - depth) << 23);  // 2^-depth
+    const float up = __fmul_ru(root.up, scale), down = __fmul_rd(root.down, scale);
+    const float up2 = __fmul_ru(up, up);
+    const float wide = __fmul_ru(__fmul_ru(up, 4.76837159e-7f), __fadd_ru(fabsf(com_x), fabsf(com_y)));
+    const float down2 = __fmul_rd(down, down);
+    const bool always_open = !(down2 < 1e38f);  // beyond any f32 distance
+    *hi = always_open ? INFINITY : __fmaf_ru(up2, 1.000101f, wide);
+    *lo = always_open ? INFINITY : __fmaf_rd(down2, 0.999899f, -wide);
 }
 
 // hi with the depth in its low 5 bits, rounded away from zero to make room:
@@ -1072,93 +1117,33 @@ __device__ __forceinline__ float pack_depth(float hi, uint32_t depth) {
     return __uint_as_float(((__float_as_uint(hi) + 32u) & ~31u) | depth);
 }
 
-// Writes the MAC fields of record k: internal cells get (hi|depth, lo); a
-// leaf (count >= 1 bodies) is always summed directly: one body -> hi = -1 (it
-// passes as a point mass at its own position, which is its f32 centre of
-// mass exactly) and u.x = 1; several bodies -> hi = +inf (no point-mass
-// term) and u.x = count, summed body by body.
-// Where a cell sits for the traversal: slot `quadrant` of its parent's node
-// group, or slot 0 of its simulation's root group (index capacity + sim).
-struct SlotRef {
-    uint32_t parent;      // kNone for a root
-    uint32_t quadrant;
-    uint32_t root_group;  // capacity + sim
-};
-
-__device__ __forceinline__ CellRec* slot_of(CellRec* groups, const SlotRef& r) {
-    return groups + (r.parent == kNone ? 4ull * r.root_group : 4ull * r.parent + r.quadrant);
+// Where a cell sits for the traversal: slot `quadrant` (the 2-bit digit of
+// its codes at the parent's depth) of its parent's node group, or slot 0 of
+// its simulation's root group (index capacity + sim).
+__device__ __forceinline__ unsigned long long slot_index(uint32_t parent, uint32_t depth,
+                                                         uint32_t code, uint32_t root_group) {
+    return depth == 0u ? 4ull * root_group
+                       : 4ull * parent + ((code >> (32u - 2u * depth)) & 3u);
 }
 
-// Writes the MAC fields of cell k into its slot of the parent's node group
-// (the traversal's record of the cell): internal cells get (hi|depth, lo); a leaf
-// (count >= 1 bodies) is always summed directly: one body -> hi = -1 (it
-// passes as a point mass at its own position, which is its f32 centre of
-// mass exactly); several bodies -> hi = +inf (no point-mass term), summed
-// body by body.  The slot's u = (lo | body count, start, body count, k or
-// kNone for a leaf).
-__device__ __forceinline__ void store_mac_fields(CellRec* groups, uint32_t k,
-                                                 float fx, float fy, float gm, uint32_t depth,
-                                                 uint32_t start, uint32_t count, bool leaf,
-                                                 const SlotRef& slot, double root_half,
-                                                 double theta) {
-    float lo = 0.f, hi;
-    uint32_t ux;
-    if (leaf) {
-        hi = count == 1u ? -1.0f : INFINITY;
-        ux = count;
-    } else {
-        const double width = __dmul_rn(__dmul_rn(root_half, pow2_neg(depth)), 2.0);
-        mac_band(width, theta, fx, fy, &lo, &hi);
-        ux = __float_as_uint(lo);
-    }
-    const float4 f = make_float4(fx, fy, gm, pack_depth(hi, depth));
-    CellRec* sl = slot_of(groups, slot);
-    sl->f = f;
-    sl->u = make_uint4(ux, start, count, leaf ? kNone : k);
-}
-
-// Writes a cell's f64 aggregates (centre of mass = weighted sums / mass, as
-// flat.rs:193-212) and its traversal records.
-__device__ __forceinline__ void store_cell_values(uint32_t k, double mass, double wx, double wy,
-                                                  uint32_t depth, uint32_t start, uint32_t count,
-                                                  bool leaf, const SlotRef& slot,
-                                                  double root_half, double theta, float g,
-                                                  double4* cell_d, CellRec* groups) {
-    const double com_x = __ddiv_rn(wx, mass);
-    const double com_y = __ddiv_rn(wy, mass);
-    const float hx = (float)com_x, hy = (float)com_y;
-    // the f32 residuals com - (float)com ride in the record's spare word: the
-    // compensated traversal adds them back to its differences
-    const float lo_x = (float)(com_x - (double)hx), lo_y = (float)(com_y - (double)hy);
-    const unsigned long long lo_bits =
-        ((unsigned long long)__float_as_uint(lo_y) << 32) | __float_as_uint(lo_x);
-    cell_d[k] = make_double4(com_x, com_y, mass, __longlong_as_double((long long)lo_bits));
-    store_mac_fields(groups, k, hx, hy, __fmul_rn(g, (float)mass),
-                     depth, start, count, leaf, slot, root_half, theta);
-}
-
-// Slot of cell k given its parent: the quadrant is the 2-bit digit of the
-// cell's codes at the parent's depth.
-__device__ __forceinline__ SlotRef slot_ref(uint32_t parent, uint32_t depth, uint32_t start_code,
-                                            uint32_t root_group) {
-    SlotRef r;
-    r.parent = parent;
-    r.quadrant = depth ? (start_code >> (32u - 2u * depth)) & 3u : 0u;
-    r.root_group = root_group;
-    return r;
-}
-
-// Acquire-release fetch-add at GPU scope: the writes before it (this
-// thread's cell values) are visible to whichever thread reads the counter's
-// final value, and this thread sees the writes released before the
-// increments it reads.
-__device__ __forceinline__ uint32_t atomic_add_acq_rel(uint32_t* p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "l"(p), "r"(v)
-                 : "memory");
-    return old;
+// Cell k's record for its slot of the parent's node group: internal cells get
+// (hi|depth, lo); a leaf (count >= 1 bodies) is always summed directly: one
+// body -> hi = -1 (it passes as a point mass at its own position, which is its
+// f32 centre of mass exactly); several bodies -> hi = +inf (no point-mass
+// term), summed body by body.  The slot's u = (lo | body count, start, body
+// count, k or kNone for a leaf).  crit: the root's width/theta (halved at each
+// depth).
+__device__ __forceinline__ CellRec slot_record(uint32_t k, float fx, float fy, float gm,
+                                               uint32_t depth, uint32_t start, uint32_t count,
+                                               bool leaf, Crit crit) {
+    float lo, hi;
+    mac_band(crit, depth, fx, fy, &lo, &hi);
+    if (leaf) hi = count == 1u ? -1.0f : INFINITY;
+    const uint32_t ux = leaf ? count : __float_as_uint(lo);
+    CellRec rec;
+    rec.f = make_float4(fx, fy, gm, pack_depth(hi, depth));
+    rec.u = make_uint4(ux, start, count, leaf ? kNone : k);
+    return rec;
 }
 
 struct AggArgs {
@@ -1170,135 +1155,452 @@ struct AggArgs {
     uint32_t capacity;
     const uint4* cell_u;
     const uint4* cell_child;
-    const uint32_t* cell_parent;
-    uint32_t* cell_counter;
     double4* cell_d;
     CellRec* groups;
 };
 
-// Aggregates of cell k (u = its links (end, skip, start, depth)): a leaf
-// sums its bodies in Morton order, an internal cell its children in quadrant
-// order 0..3 (nbody/src/flat.rs:179-215).
-__device__ __forceinline__ void aggregate_cell(const AggArgs& a, uint32_t k, uint4 u, bool leaf) {
-    const uint32_t start = u.z, depth = u.w, end = u.x;
-    const uint32_t s = a.chunk_sim[start >> 5];
-    const SimDesc& sd = a.sims[s];
-    double mass = 0.0, wx = 0.0, wy = 0.0;
-    if (leaf) {
-        for (uint32_t q = start; q < end; ++q) {
-            const float4 b = a.sbody[q];
-            const double m = (double)b.z;
-            mass = __dadd_rn(mass, m);
-            wx = __dadd_rn(wx, __dmul_rn(m, (double)b.x));
-            wy = __dadd_rn(wy, __dmul_rn(m, (double)b.y));
-        }
-    } else {
-        const uint4 ch = a.cell_child[k];
-        const uint32_t chv[4] = {ch.x, ch.y, ch.z, ch.w};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (chv[q] == kNone) continue;
-            const double2 cxy = __ldcg(reinterpret_cast<const double2*>(a.cell_d + chv[q]));
-            const double cm = __ldcg(reinterpret_cast<const double*>(a.cell_d + chv[q]) + 2);
-            mass = __dadd_rn(mass, cm);
-            wx = __dadd_rn(wx, __dmul_rn(cm, cxy.x));
-            wy = __dadd_rn(wy, __dmul_rn(cm, cxy.y));
-        }
+// The simulation a chunk of 32 positions belongs to, as the aggregates need it.
+struct AggSim {
+    Crit crit;            // root width / theta
+    uint32_t off, end;    // its positions (end = 0: an unused chunk)
+    uint32_t root_group;  // capacity + sim
+    float g;
+};
+
+// Mass and centre of mass of a cell from its weighted sums, as
+// nbody/src/flat.rs:193-212, in f64.
+struct CellSum {
+    double mass = 0.0, wx = 0.0, wy = 0.0;  // then wx, wy become the centre of mass
+    __device__ __forceinline__ void add(double m, double x, double y) {
+        mass = __dadd_rn(mass, m);
+        wx = __dadd_rn(wx, __dmul_rn(m, x));
+        wy = __dadd_rn(wy, __dmul_rn(m, y));
     }
-    store_cell_values(k, mass, wx, wy, depth, start, end - start, leaf,
-                      slot_ref(a.cell_parent[k], depth, a.codes[start], a.capacity + s),
-                      a.simout[s].half, sd.theta, sd.g_f, a.cell_d, a.groups);
+    __device__ __forceinline__ void finish() {
+        wx = __ddiv_rn(wx, mass);
+        wy = __ddiv_rn(wy, mass);
+    }
+};
+
+// Writes a finished cell's f64 record; returns its centre of mass in f32.
+__device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const CellSum& c) {
+    const float hx = (float)c.wx, hy = (float)c.wy;
+    // the f32 residuals com - (float)com ride in the record's spare word: the
+    // compensated traversal adds them back to its differences
+    const float lo_x = (float)(c.wx - (double)hx), lo_y = (float)(c.wy - (double)hy);
+    const unsigned long long lo_bits =
+        ((unsigned long long)__float_as_uint(lo_y) << 32) | __float_as_uint(lo_x);
+    cell_d[k] = make_double4(c.wx, c.wy, c.mass, __longlong_as_double((long long)lo_bits));
+    return make_float2(hx, hy);
 }
 
-// Cell k is done and its parent spans several blocks: count k in at the
-// parent; the thread that completes a parent's last child computes the
-// parent and carries on upwards.
-__device__ void climb(const AggArgs& a, uint32_t k) {
-    while (true) {
-        const uint32_t par = a.cell_parent[k];
-        if (par == kNone) return;
-        const uint4 ch = a.cell_child[par];
-        const uint32_t nchild =
-            (ch.x != kNone) + (ch.y != kNone) + (ch.z != kNone) + (ch.w != kNone);
-        if (atomic_add_acq_rel(a.cell_counter + par, 1u) + 1u != nchild) return;
-        aggregate_cell(a, par, a.cell_u[par], false);
-        k = par;
-    }
-}
-
-// Bottom-up f64 aggregates.  A block covers the cells of 256 positions
-// [P0, P1), the preorder range [kb, ke).  A cell whose positions lie inside
-// [P0, P1) is local: the block computes every leaf first, then its local
-// internal cells depth by depth, deepest first, with a block barrier between
-// depths, so no local cell needs an atomic.  The other cells span several
-// blocks (ancestors of block boundaries, about 1% of the internal cells);
-// each is computed by the thread that completes its last child, found with
-// one acquire-release counter per cell.  Same arithmetic and order as the
-// reference, so the f64 mass and centre of mass equal its values bit for bit.
-// 64 threads per 256 positions: a depth holds few cells, and small blocks
-// let many blocks hide each other's per-depth latency.
-constexpr uint32_t kAggPositions = kAggBlockPositions;
+// Bottom-up f64 aggregates.  The structure below a run of positions needs no
+// links: position p starts a group at every depth >= dmin(p) (one more than
+// the levels it shares with p - 1), its cells are numbered base[p] + d -
+// dmin(p), and a group ends at the next position whose dmin is at most its
+// depth.  A block owns the cells that start between two cuts.  It computes
+// every leaf, then the internal cells that end before the next cut, depth by
+// depth, deepest first, with a block barrier between depths.  The sum and end
+// of the last cell done at each position stay in shared memory, so a cell
+// hops over its children there (the first at its own start, the next at each
+// child's end), and it writes its whole node group, a 128-byte line; nothing
+// is loaded from global memory after the block's codes, bases and bodies.  The
+// cells that span a cut (few, and shallow: the cuts lie at the coarsest group
+// starts near every kAggPositions) are listed for k_aggregate_spans.  A leaf sums
+// its bodies in Morton order, an internal cell its children in quadrant order
+// 0..3 (nbody/src/flat.rs:179-215): the f64 mass and centre of mass equal the
+// reference's bit for bit.
 #ifndef GBH_AGG_THREADS
-#define GBH_AGG_THREADS 64
+#define GBH_AGG_THREADS 128
+#endif
+#ifndef GBH_AGG_MIN_BLOCKS
+#define GBH_AGG_MIN_BLOCKS 8
 #endif
 constexpr uint32_t kAggThreads = GBH_AGG_THREADS;
+constexpr uint32_t kAggItems = kAggPositions + kAggCutWindow;  // positions of a block, at most
+constexpr uint32_t kAggGroups = (kAggItems + 31u) / 32u;
+static_assert(kAggPositions == kCellsThreads, "k_cells' blocks find the cuts");
+static_assert(kAggCutWindow <= kCellsThreads && kAggCutWindow % 32u == 0u, "cut windows");
 
-__global__ void __launch_bounds__(kAggThreads) k_aggregate(const AggArgs a, uint32_t npos,
-                                                           const uint32_t* __restrict__ base,
-                                                           uint32_t* err) {
+__device__ __forceinline__ AggSim agg_sim(const AggArgs& a, uint32_t sim) {
+    AggSim si{};
+    if (sim != kNone) {
+        const SimDesc& sd = a.sims[sim];
+        si.crit = crit_f32(a.simout[sim].crit0);
+        si.off = sd.off;
+        si.end = sd.off + sd.n;
+        si.root_group = a.capacity + sim;
+        si.g = sd.g_f;
+    }
+    return si;
+}
+
+// One child of a cell, or none, as its slot of the cell's node group: an
+// absent child takes the lowest quadrant left in `missing`.
+__device__ __forceinline__ void store_child(CellRec* group, bool have, uint32_t quadrant,
+                                            uint32_t* missing, uint32_t k, float x, float y,
+                                            float gm, uint32_t depth, uint32_t start, uint32_t end,
+                                            bool leaf, Crit crit) {
+    CellRec rec = slot_record(k, x, y, gm, depth, start, end - start, leaf, crit);
+    if (!have) {
+        rec.f = make_float4(0.f, 0.f, 0.f, 0.f);
+        rec.u = make_uint4(0u, 0u, 0u, kNone);
+        quadrant = __ffs(*missing) - 1u;
+        *missing &= *missing - 1u;
+    }
+    group[quadrant].f = rec.f;
+    group[quadrant].u = rec.u;
+}
+
+struct AggShared {
+    // the last finished cell that starts at position i: centre of mass x, y and
+    // mass (f64), then its end | dmin of that end << 16 (positions of the block)
+    double x[kAggItems], y[kAggItems], m[kAggItems];
+    float fx[kAggItems], fy[kAggItems], gm[kAggItems];  // in f32, with G*mass
+    uint32_t link[kAggItems];
+    uint32_t code[kAggItems];
+    uint32_t base[kAggItems + 1];
+    // dmin | depth of the chain's leaf << 8 | first depth whose group ends
+    // inside the block << 16
+    uint32_t info[kAggItems + 1];
+    AggSim sim[kAggGroups + 1];  // by chunk of 32 positions
+    // local internal cells by depth, as positions: those of one depth hold
+    // disjoint ranges of at least two positions
+    uint16_t level[kMortonDepth][kAggItems / 2u];
+    uint16_t count[kAggGroups][kMortonDepth], total[kMortonDepth];
+    uint32_t depths;  // depths that have some
+};
+
+__global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
+    k_aggregate(const AggArgs a, const uint32_t* __restrict__ base, const AggPlan plan,
+                uint32_t* err) {
     wait_for_predecessor();
-    // local internal cells by depth (offsets from kb), internal depths
-    // 0..15: those of one depth hold disjoint ranges of at least two
-    // positions, so at most half the block's positions per depth
-    __shared__ uint16_t s_level[kMortonDepth][kAggPositions / 2];
-    __shared__ uint32_t s_count[kMortonDepth];
-    __shared__ uint32_t s_code[kAggPositions + 2];  // codes of positions P0-1 .. P0+256
-    const uint32_t t = threadIdx.x;
-    const uint32_t P0 = blockIdx.x * kAggPositions;
-    const uint32_t P1 = min(P0 + kAggPositions, npos);
-    if (t < kMortonDepth) s_count[t] = 0;
-    for (uint32_t j = t; j < kAggPositions + 2; j += kAggThreads) {
-        const uint32_t gp = P0 + j - 1u;
-        s_code[j] = (j > 0 || P0 > 0) && gp < npos ? a.codes[gp] : 0u;
+    __shared__ AggShared s;
+    const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
+    const uint32_t R0 = plan.cuts[blockIdx.x], R1 = plan.cuts[blockIdx.x + 1u];
+    const uint32_t npos = plan.cuts[plan.blocks];
+    const uint32_t n = R1 - R0;
+    if (n - 1u >= kAggItems) {  // cannot be: the cuts lie in windows
+        if (t == 0) set_err(err, kErrCapacity);
+        return;
+    }
+    const uint32_t chunk0 = R0 >> 5;
+    for (uint32_t j = t; j < n; j += kAggThreads) {
+        s.code[j] = a.codes[R0 + j];
+        s.base[j] = base[R0 + j];
+    }
+    if (t <= (R1 - 1u) / 32u - chunk0) s.sim[t] = agg_sim(a, a.chunk_sim[chunk0 + t]);
+    const uint32_t before = R0 > 0u ? a.codes[R0 - 1u] : 0u;
+    const uint32_t after = R1 < npos ? a.codes[R1] : 0u;
+    const uint32_t range = blockIdx.x / kAggRange;
+    const uint32_t R2 = plan.cuts[min((range + 1u) * kAggRange, plan.blocks)];  // the outer cut
+    const uint32_t beyond = R2 < npos ? a.codes[R2] : 0u;
+    if (t == 0) {
+        s.depths = 0;
+        s.info[n] = 0;
+        s.base[n] = base[R1];
     }
     __syncthreads();
-    const uint32_t kb = base[P0], ke = base[P1];
-    // whether the depth-dd group holding position p lies inside [P0, P1):
-    // its neighbours outside the block (within the simulation) differ in
-    // the first dd levels
-    auto inside = [&](uint32_t p, uint32_t dd, const SimDesc& sd) {
-        const uint32_t c = s_code[p - P0 + 1u];
-        const bool left = sd.off >= P0 || shared_levels(s_code[0], c) < dd;
-        const bool right = sd.off + sd.n <= P1 || shared_levels(c, s_code[P1 - P0 + 1u]) < dd;
-        return left && right;
+    const uint32_t groups = (n + 31u) / 32u;
+    auto local = [](uint32_t info, uint32_t d) {
+        return d >= ((info >> 16) & 0xffu) && d < ((info >> 8) & 0xffu);
     };
-    // the next cell's links are loaded while this one is summed
-    uint4 u_next = kb + t < ke ? a.cell_u[kb + t] : make_uint4(0u, 0u, 0u, 0u);
-    for (uint32_t k = kb + t; k < ke; k += kAggThreads) {
-        const uint4 u = u_next;  // (end, skip, start, depth)
-        if (k + kAggThreads < ke) u_next = a.cell_u[k + kAggThreads];
-        const SimDesc& sd = a.sims[a.chunk_sim[u.z >> 5]];
-        if (u.y == k + 1u) {
-            aggregate_cell(a, k, u, true);
-            if (u.w > 0 && !inside(u.z, u.w - 1u, sd)) climb(a, k);
-        } else if (inside(u.z, u.w, sd)) {
-            const uint32_t slot = u.w < kMortonDepth ? atomicAdd(&s_count[u.w], 1u) : kNone;
-            if (slot < kAggPositions / 2)
-                s_level[u.w][slot] = (uint16_t)(k - kb);
-            else
-                set_err(err, kErrCapacity);
+    auto sim_of = [&](uint32_t j) -> const AggSim& { return s.sim[((R0 + j) >> 5) - chunk0]; };
+    for (uint32_t g = warp; g < groups; g += kAggThreads / 32u) {
+        const uint32_t j = g * 32u + lane, p = R0 + j;
+        uint32_t depths = 0;
+        if (j < n) {
+            const AggSim& si = sim_of(j);
+            const uint32_t code = s.code[j], cells = s.base[j + 1u] - s.base[j];
+            // positions past the simulation's end head every depth: they end its groups
+            uint32_t dmin = 0, deepest = 0;
+            if (p < si.end && p != si.off)
+                dmin = shared_levels(j ? s.code[j - 1u] : before, code) + 1u;
+            if (cells) deepest = dmin + cells - 1u;
+            const uint32_t dlo = si.end > R1 ? max(dmin, shared_levels(code, after) + 1u) : dmin;
+            s.info[j] = dmin | deepest << 8 | dlo << 16;
+            if (deepest > dlo) depths = ((1u << deepest) - 1u) & ~((1u << dlo) - 1u);
+            for (uint32_t d = dmin; d < min(dlo, deepest); ++d) {  // the cells that span R1
+                const uint2 rec = make_uint2(s.base[j] + d - dmin,
+                                             d << 26 | (si.root_group - a.capacity));
+                if (si.end > R2 && shared_levels(code, beyond) >= d)
+                    plan.outer[atomicAdd(plan.outer_n, 1u)] = rec;
+                else
+                    plan.inner[(size_t)range * kAggRangeCells + atomicAdd(plan.inner_n + range, 1u)] =
+                        rec;
+            }
+        }
+        depths = __reduce_or_sync(kFull, depths);
+        if (lane == 0 && depths) atomicOr(&s.depths, depths);
+    }
+    __syncthreads();
+    for (uint32_t j = t; j < n; j += kAggThreads) {
+        const uint32_t k = s.base[j + 1u] - 1u;
+        if (s.base[j + 1u] == s.base[j]) continue;
+        const uint32_t info = s.info[j], d = (info >> 8) & 0xffu;
+        const AggSim& si = sim_of(j);
+        const float4 body = a.sbody[R0 + j];
+        CellSum sum;
+        sum.add((double)body.z, (double)body.x, (double)body.y);
+        uint32_t q = j + 1u;
+        for (; (s.info[q] & 0xffu) > d; ++q) {  // s.info[n] = 0 ends the walk
+            const float4 b = a.sbody[R0 + q];
+            sum.add((double)b.z, (double)b.x, (double)b.y);
+        }
+        s.link[j] = q | (s.info[q] & 0xffu) << 16;
+        uint32_t end = R0 + q;
+        if (q == n && d < ((info >> 16) & 0xffu)) {  // the leaf goes on past the block
+            end = a.cell_u[k].x;
+            for (uint32_t g = R0 + q; g < end; ++g) {
+                const float4 b = a.sbody[g];
+                sum.add((double)b.z, (double)b.x, (double)b.y);
+            }
+        }
+        float2 com = make_float2(body.x + 0.f, body.y + 0.f);
+        float mass = body.z;
+        if (end == R0 + j + 1u) {
+            // one body: m x of two f32 values is exact in f64, so (m x) / m is x
+            // (+0.0 for -0.0, as the sum that starts at +0.0)
+            sum.wx = (double)com.x;
+            sum.wy = (double)com.y;
+            a.cell_d[k] = make_double4(sum.wx, sum.wy, sum.mass, 0.0);
+        } else {
+            sum.finish();
+            com = store_cell(a.cell_d, k, sum);
+            mass = (float)sum.mass;
+        }
+        s.x[j] = sum.wx;
+        s.y[j] = sum.wy;
+        s.m[j] = sum.mass;
+        s.fx[j] = com.x;
+        s.fy[j] = com.y;
+        s.gm[j] = __fmul_rn(si.g, mass);
+        if (d == 0u)  // the simulation is one leaf
+            a.groups[4ull * si.root_group] = slot_record(
+                k, com.x, com.y, s.gm[j], 0u, R0 + j, end - (R0 + j), true, si.crit);
+    }
+    // the cells of each depth, in position order: counts by group of 32
+    // positions, then every group's places
+    const uint32_t depths = s.depths;
+    for (uint32_t g = warp; g < groups; g += kAggThreads / 32u) {
+        const uint32_t info = g * 32u + lane < n ? s.info[g * 32u + lane] : 0u;
+        uint32_t count = 0;
+        for (uint32_t m = depths; m; m &= m - 1u) {
+            const uint32_t d = __ffs(m) - 1u;
+            const uint32_t votes = __popc(__ballot_sync(kFull, local(info, d)));
+            if (lane == d) count = votes;
+        }
+        if (lane < kMortonDepth) s.count[g][lane] = (uint16_t)count;
+    }
+    __syncthreads();
+    for (uint32_t g = warp; g < groups; g += kAggThreads / 32u) {
+        const uint32_t info = g * 32u + lane < n ? s.info[g * 32u + lane] : 0u;
+        uint32_t place = 0;
+        if (lane < kMortonDepth) {
+            for (uint32_t q = 0; q < g; ++q) place += s.count[q][lane];
+            if (g + 1u == groups) s.total[lane] = (uint16_t)(place + s.count[g][lane]);
+        }
+        for (uint32_t m = depths; m; m &= m - 1u) {
+            const uint32_t d = __ffs(m) - 1u;
+            const uint32_t votes = __ballot_sync(kFull, local(info, d));
+            const uint32_t at = __shfl_sync(kFull, place, d) + __popc(votes & ((1u << lane) - 1u));
+            if ((votes >> lane) & 1u) s.level[d][at] = (uint16_t)(g * 32u + lane);
         }
     }
     __syncthreads();
-    for (int d = (int)kMortonDepth - 1; d >= 0; --d) {
-        const uint32_t cnt = min(s_count[d], kAggPositions / 2);
-        if (cnt == 0) continue;
-        for (uint32_t j = t; j < cnt; j += kAggThreads) {
-            const uint32_t k = kb + s_level[d][j];
-            const uint4 u = a.cell_u[k];
-            aggregate_cell(a, k, u, false);
-            if (d > 0 && !inside(u.z, (uint32_t)d - 1u, a.sims[a.chunk_sim[u.z >> 5]])) climb(a, k);
+    // The cells of one depth, a thread each.  No branch on the children: an
+    // absent one stands in as the first and adds 0 (lanes taking turns at four
+    // ways through the code cost more than the arithmetic).  The node group is
+    // written after the depth's barrier, and the next depth's cells go to other
+    // warps first, so the stores are off the way from depth to depth: children
+    // but the first are final, and the first's values are kept (`first`).
+    struct {
+        uint32_t d = kNone, c0 = 0, c1 = 0, c2 = 0, c3 = 0, kids = 0, link0 = 0;
+        float fx = 0.f, fy = 0.f, gm = 0.f;
+    } first;
+    auto store_group = [&]() {
+        const uint32_t d = first.d;
+        if (d == kNone) return;
+        const uint32_t c[4] = {first.c0, first.c1, first.c2, first.c3};
+        const uint32_t k = s.base[first.c0] + d - (s.info[first.c0] & 0xffu);
+        const AggSim& sim = sim_of(first.c0);
+        uint32_t quadrant[4], missing = 15u;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            quadrant[q] = (s.code[c[q]] >> (30u - 2u * d)) & 3u;
+            missing &= ~(1u << quadrant[q]);  // (an absent child repeats the first)
         }
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const uint32_t kid = s.base[c[q]] + d + 1u - (s.info[c[q]] & 0xffu);
+            const uint32_t link = q ? s.link[c[q]] : first.link0;
+            store_child(a.groups + 4ull * k, q < first.kids, quadrant[q], &missing, kid,
+                        q ? s.fx[c[q]] : first.fx, q ? s.fy[c[q]] : first.fy,
+                        q ? s.gm[c[q]] : first.gm, d + 1u, R0 + c[q], R0 + (link & 0xffffu),
+                        kid + 1u == s.base[c[q] + 1u], sim.crit);
+        }
+        first.d = kNone;
+    };
+    uint32_t turn = 0;
+    for (uint32_t todo = depths; todo != 0u;) {
+        const uint32_t d = 31u - __clz(todo);
+        todo &= ~(1u << d);
+        const uint32_t cells = s.total[d];
+        for (uint32_t i = (t + turn) % kAggThreads; i < cells; i += kAggThreads) {
+            store_group();
+            const uint32_t c0 = s.level[d][i];
+            const uint32_t k = s.base[c0] + d - (s.info[c0] & 0xffu);
+            const uint32_t link0 = s.link[c0];
+            const bool two = (link0 >> 16) > d;
+            const uint32_t c1 = two ? link0 & 0xffffu : c0;
+            const uint32_t link1 = s.link[c1];
+            const bool three = two && (link1 >> 16) > d;
+            const uint32_t c2 = three ? link1 & 0xffffu : c0;
+            const uint32_t link2 = s.link[c2];
+            const bool four = three && (link2 >> 16) > d;
+            const uint32_t c3 = four ? link2 & 0xffffu : c0;
+            const uint32_t link3 = s.link[c3];
+            const uint32_t c[4] = {c0, c1, c2, c3};
+            const bool have[4] = {true, two, three, four};
+            CellSum sum;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                // (adding 0.0 leaves a sum: it starts at +0.0 and is never -0.0)
+                const double m = s.m[c[q]];
+                sum.mass = __dadd_rn(sum.mass, have[q] ? m : 0.0);
+                sum.wx = __dadd_rn(sum.wx, have[q] ? __dmul_rn(m, s.x[c[q]]) : 0.0);
+                sum.wy = __dadd_rn(sum.wy, have[q] ? __dmul_rn(m, s.y[c[q]]) : 0.0);
+            }
+            first.d = d;
+            first.c0 = c0;
+            first.c1 = c1;
+            first.c2 = c2;
+            first.c3 = c3;
+            first.kids = 1u + two + three + four;
+            first.link0 = link0;
+            first.fx = s.fx[c0];
+            first.fy = s.fy[c0];
+            first.gm = s.gm[c0];
+            sum.finish();
+            s.x[c0] = sum.wx;
+            s.y[c0] = sum.wy;
+            s.m[c0] = sum.mass;
+            const uint32_t link = four ? link3 : three ? link2 : two ? link1 : link0;
+            s.link[c0] = link;
+            const AggSim& sim = sim_of(c0);
+            const float2 com = store_cell(a.cell_d, k, sum);
+            const float gm = __fmul_rn(sim.g, (float)sum.mass);
+            s.fx[c0] = com.x;
+            s.fy[c0] = com.y;
+            s.gm[c0] = gm;
+            if (d == 0u)
+                a.groups[4ull * sim.root_group] = slot_record(
+                    k, com.x, com.y, gm, 0u, R0 + c0, (link & 0xffffu) - c0, false, sim.crit);
+        }
+        __syncthreads();
+        store_group();
+        turn += kAggThreads / 2u;
+    }
+}
+
+// One cell that spans a cut, from its children's f64 records.
+struct SpanCell {
+    uint32_t k, start, count, c[4];
+    uint32_t kid_start[4], kid_end[4];
+    bool kid_leaf[4];
+    AggSim sim;
+
+    __device__ __forceinline__ void load(const AggArgs& a, uint2 rec) {
+        k = rec.x;
+        sim = agg_sim(a, rec.y & 0x3ffffffu);
+        const uint4 u = a.cell_u[k];
+        const uint4 ch = a.cell_child[k];
+        start = u.z;
+        count = u.x - u.z;
+        c[0] = ch.x;
+        c[1] = ch.y;
+        c[2] = ch.z;
+        c[3] = ch.w;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t kid = c[q] == kNone ? k + 1u : c[q];  // absent: its first child
+            const uint4 cu = a.cell_u[kid];
+            kid_start[q] = cu.z;
+            kid_end[q] = cu.x;
+            kid_leaf[q] = cu.y == kid + 1u;
+        }
+    }
+    __device__ __forceinline__ void combine(const AggArgs& a, uint32_t d) const {
+        CellSum sum;
+        double2 com[4];
+        double m[4];
+        uint32_t missing = 15u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double4* rec = a.cell_d + (c[q] == kNone ? k + 1u : c[q]);
+            com[q] = __ldcg(reinterpret_cast<const double2*>(rec));
+            m[q] = __ldcg(reinterpret_cast<const double*>(rec) + 2);
+            if (c[q] != kNone) missing &= ~(1u << q);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (c[q] != kNone) sum.add(m[q], com[q].x, com[q].y);
+        sum.finish();
+        const float2 own = store_cell(a.cell_d, k, sum);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            store_child(a.groups + 4ull * k, c[q] != kNone, (uint32_t)q, &missing, c[q],
+                        (float)com[q].x, (float)com[q].y, __fmul_rn(sim.g, (float)m[q]), d + 1u,
+                        kid_start[q], kid_end[q], kid_leaf[q], sim.crit);
+        if (d == 0u)
+            a.groups[4ull * sim.root_group] =
+                slot_record(k, own.x, own.y, __fmul_rn(sim.g, (float)sum.mass), 0u, start, count,
+                            false, sim.crit);
+    }
+};
+
+// Lists of cells that span cuts, a block each (list stride `capacity`), depth
+// by depth: each depth waits for the one below, and a barrier of one block is
+// the cheapest wait.  A thread per cell, everything but the children's sums
+// loaded before the first depth (the further cells of a list longer than the
+// block are loaded in turn).  All lists of the inner cuts run at once, then
+// the one of the outer cuts: in a single list the 64-range tree of 2^20 bodies
+// took 70 us.
+#ifndef GBH_SPAN_THREADS
+#define GBH_SPAN_THREADS 512
+#endif
+constexpr uint32_t kSpanThreads = GBH_SPAN_THREADS;
+
+__global__ void __launch_bounds__(kSpanThreads) k_aggregate_spans(const AggArgs a,
+                                                                  const uint2* lists,
+                                                                  const uint32_t* counts,
+                                                                  uint32_t capacity) {
+    wait_for_predecessor();
+    __shared__ uint32_t s_depths;
+    const uint32_t t = threadIdx.x;
+    const uint2* list = lists + (size_t)blockIdx.x * capacity;
+    const uint32_t n = min(counts[blockIdx.x], capacity);
+    if (n == 0u) return;
+    if (t == 0) s_depths = 0;
+    __syncthreads();
+    uint32_t depth = kNone;
+    SpanCell cell;
+    if (t < n) {
+        depth = list[t].y >> 26;
+        cell.load(a, list[t]);
+    }
+    for (uint32_t i = t; i < n; i += kSpanThreads) atomicOr(&s_depths, 1u << (list[i].y >> 26));
+    __syncthreads();
+    for (uint32_t todo = s_depths; todo != 0u;) {
+        const uint32_t d = 31u - __clz(todo);
+        todo &= ~(1u << d);
+        if (depth == d) cell.combine(a, d);
+        for (uint32_t i = t + kSpanThreads; i < n; i += kSpanThreads)
+            if (list[i].y >> 26 == d) {
+                SpanCell more;
+                more.load(a, list[i]);
+                more.combine(a, d);
+            }
         __syncthreads();
     }
 }
@@ -1319,10 +1621,9 @@ __global__ void k_refresh_mac(const SimDesc* __restrict__ sims, const SimOut* __
     const double4 v = cell_d[k];
     const bool leaf = u.y == k + 1u;
     const uint32_t start = u.z;
-    store_mac_fields(groups, k, (float)v.x, (float)v.y, __fmul_rn(sd.g_f, (float)v.z), u.w, start,
-                     u.x - start, leaf,
-                     slot_ref(cell_parent[k], u.w, codes[start], capacity + sim),
-                     simout[sim].half, sd.theta);
+    groups[slot_index(cell_parent[k], u.w, codes[start], capacity + sim)] =
+        slot_record(k, (float)v.x, (float)v.y, __fmul_rn(sd.g_f, (float)v.z), u.w, start, u.x - start,
+                    leaf, crit_f32(crit_of(simout[sim].half, sd.theta)));
 }
 
 // ============================================================ traverse ====
@@ -2423,18 +2724,40 @@ cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
                        b.npos, b.keys_a, b.base, b.counters + 8, b.scan_flags, b.err);
 }
 
+// The counts, the outer list and the cuts (about 5 bytes per kAggPositions) have
+// their own words; the inner lists lie in the sort's spent value buffers, 8
+// bytes a position: a range of kAggRange blocks may hold 16 KB of them, and the
+// last range's list has at most 128 bytes per cut.
+static AggPlan agg_plan(const BatchBuffers& b) {
+    AggPlan p;
+    p.blocks = (b.npos + kAggPositions - 1) / kAggPositions;
+    p.ranges = (p.blocks + kAggRange - 1) / kAggRange;
+    p.outer = reinterpret_cast<uint2*>(b.agg_words);
+    p.inner_n = b.agg_words + 2u * kMortonDepth * p.ranges;
+    p.cuts = p.inner_n + p.ranges;
+    p.inner = reinterpret_cast<uint2*>(b.vals_a);
+    p.outer_n = b.counters + 16;
+    return p;
+}
+
 cudaError_t launch_cells(const BatchBuffers& b, cudaStream_t s) {
     return launch_step(k_cells, (b.npos + kCellsThreads - 1) / kCellsThreads, kCellsThreads, 0, s,
                        b.sims, b.chunk_sim, b.npos, b.cell_capacity, b.keys_a, b.base, b.cell_u,
-                       b.cell_child, b.cell_parent, b.cell_counter, b.groups, b.err);
+                       b.cell_child, b.cell_parent, agg_plan(b), b.groups, b.err);
 }
 
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s) {
-    const AggArgs a{b.sims,          b.simout, b.chunk_sim, b.sbody,      b.keys_a,
-                    b.cell_capacity, b.cell_u, b.cell_child, b.cell_parent,
-                    b.cell_counter,  b.cell_d, b.groups};
-    return launch_step(k_aggregate, (b.npos + kAggPositions - 1) / kAggPositions, kAggThreads, 0,
-                       s, a, b.npos, b.base, b.err);
+    const AggArgs a{b.sims,          b.simout, b.chunk_sim,  b.sbody, b.keys_a,
+                    b.cell_capacity, b.cell_u, b.cell_child, b.cell_d, b.groups};
+    const AggPlan plan = agg_plan(b);
+    cudaError_t e = launch_step(k_aggregate, plan.blocks, kAggThreads, 0, s, a, b.base, plan, b.err);
+    if (e == cudaSuccess && plan.blocks > 1)
+        e = launch_step(k_aggregate_spans, plan.ranges, kSpanThreads, 0, s, a, plan.inner,
+                        plan.inner_n, kAggRangeCells);
+    if (e == cudaSuccess && plan.ranges > 1)
+        e = launch_step(k_aggregate_spans, 1, kSpanThreads, 0, s, a, plan.outer, plan.outer_n,
+                        kMortonDepth * plan.ranges);
+    return e;
 }
 
 cudaError_t launch_wait_probe(const uint32_t* flags, uint32_t* err, long long limit,

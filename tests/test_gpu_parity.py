@@ -676,3 +676,36 @@ def test_large_n_tree_and_sampled_forces(gpu, rt, oracle):
     force_check(oracle, acc, b32, ot, oc, targets=targets)
     rt.step(gpu, ev, tree, cfg, 5e-4, 2)
     assert np.isfinite(gpu.read_evolving_state(ev)[0]).all()
+
+
+@pytest.mark.parametrize("layout,bucket", [("random", 1), ("random", 40), ("runs", 1), ("runs", 3),
+                                           ("one_point", 1), ("one_point", 300)])
+def test_aggregates_at_block_edges(gpu, rt, oracle, layout, bucket):
+    """The aggregates work in blocks of about 256 positions, cut at the coarsest
+    group start of each 128 positions, and join them over 128 blocks: sizes at
+    the edges of a block, of a cut window and of a range of blocks, with leaves
+    of many bodies and chains to depth 16 across the cuts.  Trees bit-exact, and
+    the forces (which read the node groups) the reference's."""
+    rng = np.random.default_rng(3)
+    for n in (2, 31, 32, 33, 127, 128, 129, 255, 256, 257, 383, 384, 385, 511, 513, 4097, 32767,
+              32768, 32769, 33153):
+        pts = rng.uniform(-1, 1, (n, 2))
+        if layout == "runs":  # runs of coincident bodies, some longer than a block
+            lengths = rng.choice([1, 2, 5, 70, 300], n, p=[0.5, 0.3, 0.17, 0.02, 0.01])
+            pts = np.repeat(pts, lengths, axis=0)[:n]
+        elif layout == "one_point":
+            pts[: n - n // 8] = pts[0]
+        bodies = np.zeros((n, 5))
+        bodies[:, :2] = pts
+        bodies[:, 4] = rng.uniform(0.5, 2.0, n) / n
+        cfg = Config(theta=0.6, softening_kpc=0.05, g=1.0, bucket=bucket)
+        ev, tree, evid, ot, b32, oc = build_both(gpu, rt, oracle, bodies, cfg)
+        assert_tree_bit_exact(oracle, evid, ot, b32, oc, cfg)
+        rt.force(gpu, ev, tree, cfg)
+        acc, _ = gpu.read_evolving_accelerations(ev)
+        targets = rng.choice(n, min(n, 200), replace=False).astype(np.uint64)
+        ref, _, s = oracle.flat_accelerations(b32, ot, oc, targets=targets, abs_sum=True)
+        err = np.hypot(*(acc[targets.astype(np.int64)] - ref).T)
+        # an f32 sum of k terms is off by at most k 2^-24 of their magnitudes (and a
+        # term by a few 2^-24): the layouts of long leaves sum up to n of them
+        assert (err <= (8.0 + n) * 2.0 ** -24 * s).all(), n
