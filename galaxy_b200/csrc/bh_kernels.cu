@@ -1210,6 +1210,14 @@ __device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const 
 // its bodies in Morton order, an internal cell its children in quadrant order
 // 0..3 (nbody/src/flat.rs:179-215): the f64 mass and centre of mass equal the
 // reference's bit for bit.
+//
+// What bounds it: the chain of depths (about 700 cycles each: a few dependent
+// shared loads, four sums, two divisions, a barrier), at 8 blocks of 4 warps
+// per SM.  Links and values read from global memory per cell, with a climb
+// through an acquire-release counter wherever a parent crossed a block, took
+// 156 us at 2^20 bodies (458 at 2^22, 61 at 2^14, 45 at 2^10); this and
+// k_aggregate_spans take 110 (331, 28, 20).  256 threads: 130 us at 2^20, 64:
+// 140; four lanes per cell: 168; cut windows of 64 and 256 positions: 112, 118.
 #ifndef GBH_AGG_THREADS
 #define GBH_AGG_THREADS 128
 #endif
@@ -1563,9 +1571,10 @@ struct SpanCell {
 // by depth: each depth waits for the one below, and a barrier of one block is
 // the cheapest wait.  A thread per cell, everything but the children's sums
 // loaded before the first depth (the further cells of a list longer than the
-// block are loaded in turn).  All lists of the inner cuts run at once, then
-// the one of the outer cuts: in a single list the 64-range tree of 2^20 bodies
-// took 70 us.
+// block are loaded in turn).  The lists of the inner cuts run at once, then the
+// one of the outer cuts: 11 and 14 us at 2^20 bodies with 64 cuts a range (128:
+// 1 to 5 % less aggregate time from 2^20 on; 16: 22 % more), where one list of
+// all cuts took 70.
 #ifndef GBH_SPAN_THREADS
 #define GBH_SPAN_THREADS 512
 #endif
