@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -212,6 +213,15 @@ static uint64_t cell_bound(uint32_t n, const bh_config& c) {
     for (uint32_t d = 0; d < eff_depth(c); ++d, squares *= 4)
         internal += std::min(squares, per_depth);
     return (uint64_t)n + internal + 1;
+}
+
+// Whether the f32 softening squared is a normal number (k_traverse's rule).
+static bool normal_eps2(const bh_config* cfgs, size_t count) {
+    for (size_t s = 0; s < count; ++s) {
+        const float eps = (float)cfgs[s].softening;
+        if (!(eps * eps >= FLT_MIN)) return false;
+    }
+    return true;
 }
 
 static void fill_physics(SimDesc& sd, const bh_config& c) {
@@ -790,6 +800,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.cell_capacity = (uint32_t)L.cells;
     bb.radix_bits = 8;
     bb.trav_warps = 4;
+    bb.normal_eps2 = normal_eps2(cfgs, count);
 
     b->h_sims.resize(count);
     b->h_chunk_sim.assign(L.nchunks, kNone);
@@ -916,6 +927,7 @@ static int apply_configs(Batch* b, const bh_config* cfgs, bool for_rebuild) {
         b->h_sims[s].potential = b->states[s]->d_potential;
         fill_physics(b->h_sims[s], cfgs[s]);
     }
+    b->bb.normal_eps2 = normal_eps2(b->cfgs.data(), b->cfgs.size());
     return upload_sims(b);
 }
 
@@ -923,7 +935,8 @@ static int run_graphs(Batch* b, uint32_t nsteps) {
     cudaStream_t s = b->dev->stream;
     const uint32_t flags = (any_flag(b, BH_FLAG_COMPENSATED) ? 1u : 0u) |
                            (any_flag(b, BH_FLAG_POTENTIAL) ? 2u : 0u) |
-                           (any_without_flag(b, BH_FLAG_COMPENSATED) ? 4u : 0u);
+                           (any_without_flag(b, BH_FLAG_COMPENSATED) ? 4u : 0u) |
+                           (b->bb.normal_eps2 ? 8u : 0u);
     if (b->graph_flags != flags) {
         for (auto& g : b->graphs)
             if (g) {

@@ -1737,7 +1737,25 @@ constexpr uint32_t kTravStack = 17u * 32u;
 constexpr uint32_t kTravList = 64u;
 static_assert(kTravList >= 64u, "the mixed cells of a step park in list[32, 64)");
 
-template <bool COMP, bool POT, bool STATS, int WARPS>
+// Reciprocal square root of a softened squared distance.  NORMAL: the squared
+// softening is a normal number, so no such distance is subnormal, and the
+// instruction without the subnormals' rescaling (about three more instructions
+// of the ~15 of a term) gives the same bits.  The traversal is issue-bound: at
+// 2^20 bodies 588 -> 541 us (theta 0.5), 2^22 compensated 3818 -> 3614, 700,001
+// at theta 0.12 2704 -> 2469.  A template of the
+// kernel, chosen on the host: both forms in one kernel spilled (609 us).
+template <bool NORMAL>
+__device__ __forceinline__ float rsqrt_r2(float r2) {
+    if constexpr (NORMAL) {
+        float r;
+        asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(r2));
+        return r;
+    } else {
+        return rsqrtf(r2);
+    }
+}
+
+template <bool COMP, bool POT, bool STATS, int WARPS, bool NORMAL>
 __global__ void __launch_bounds__(WARPS * 32, GBH_TRAVERSE_MIN_BLOCKS * kTravWarps / WARPS)
     k_traverse(
     const SimDesc* __restrict__ sims, const SimOut* __restrict__ simout,
@@ -1791,7 +1809,7 @@ __global__ void __launch_bounds__(WARPS * 32, GBH_TRAVERSE_MIN_BLOCKS * kTravWar
     const float2 txy = make_float2(tx, ty);
     // one point-mass term at difference d, scale 0 for lanes that do not take it
     auto term = [&](float2 d, float d2, float gm, bool take) {
-        const float inv_r = rsqrtf(d2 + eps2);
+        const float inv_r = rsqrt_r2<NORMAL>(d2 + eps2);
         const float scale = take ? gm * inv_r * inv_r * inv_r : 0.f;
         acc.add_scaled(d, scale);
         if (POT) phi -= take ? gm * inv_r : 0.f;
@@ -1806,7 +1824,7 @@ __global__ void __launch_bounds__(WARPS * 32, GBH_TRAVERSE_MIN_BLOCKS * kTravWar
             const float4 e = list[i];
             float2 d = sub2<COMP>(make_float2(e.x, e.y), txy);
             if constexpr (COMP) d = __fadd2_rn(d, s_lo[warp][i]);
-            const float inv_r = rsqrtf(__fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, eps2)));
+            const float inv_r = rsqrt_r2<NORMAL>(__fmaf_rn(d.x, d.x, __fmaf_rn(d.y, d.y, eps2)));
             const bool take = (__float_as_uint(e.w) & lane_bit) != 0u;
             const float scale = e.z * inv_r * inv_r * inv_r;
             if constexpr (!COMP && !POT) {
@@ -2782,7 +2800,7 @@ cudaError_t launch_refresh_mac(const BatchBuffers& b, uint32_t sim, cudaStream_t
     return cudaGetLastError();
 }
 
-template <int WARPS>
+template <int WARPS, bool NORMAL>
 static cudaError_t traverse_launch(const BatchBuffers& b, bool compensated, bool potential,
                                    bool stats, cudaStream_t s) {
     // The compensated form keeps a residual per list entry; with it 8 warps'
@@ -2790,7 +2808,7 @@ static cudaError_t traverse_launch(const BatchBuffers& b, bool compensated, bool
     // block (each warp does the same work at any block size).
     constexpr int CW = WARPS > 4 ? 4 : WARPS;
 #define GBH_TRAVERSE(C, P, S)                                                                   \
-    return launch_step(k_traverse<C, P, S, (C ? CW : WARPS)>,                                   \
+    return launch_step(k_traverse<C, P, S, (C ? CW : WARPS), NORMAL>,                           \
                        (b.nchunks + (C ? CW : WARPS) - 1) / (C ? CW : WARPS),                   \
                        (C ? CW : WARPS) * 32, 0, s, b.sims, b.simout, b.chunk_sim, b.nchunks,  \
                        b.sbody, b.groups, b.cell_d, b.cell_capacity, b.force_stats, b.err)
@@ -2811,11 +2829,14 @@ static cudaError_t traverse_launch(const BatchBuffers& b, bool compensated, bool
 #undef GBH_TRAVERSE
 }
 
+// A softening whose square is subnormal (or zero) in some simulation of the
+// batch: the general form, at one block size.
 static cudaError_t traverse_form(const BatchBuffers& b, bool compensated, bool potential,
                                  bool stats, cudaStream_t s) {
-    if (b.trav_warps == 2) return traverse_launch<2>(b, compensated, potential, stats, s);
-    if (b.trav_warps == 4) return traverse_launch<4>(b, compensated, potential, stats, s);
-    return traverse_launch<kTravWarps>(b, compensated, potential, stats, s);
+    if (!b.normal_eps2) return traverse_launch<4, false>(b, compensated, potential, stats, s);
+    if (b.trav_warps == 2) return traverse_launch<2, true>(b, compensated, potential, stats, s);
+    if (b.trav_warps == 4) return traverse_launch<4, true>(b, compensated, potential, stats, s);
+    return traverse_launch<kTravWarps, true>(b, compensated, potential, stats, s);
 }
 
 cudaError_t launch_traverse(const BatchBuffers& b, bool compensated, bool plain, bool potential,

@@ -709,3 +709,29 @@ def test_aggregates_at_block_edges(gpu, rt, oracle, layout, bucket):
         # an f32 sum of k terms is off by at most k 2^-24 of their magnitudes (and a
         # term by a few 2^-24): the layouts of long leaves sum up to n of them
         assert (err <= (8.0 + n) * 2.0 ** -24 * s).all(), n
+
+
+@pytest.mark.parametrize("compensated", [False, True])
+@pytest.mark.parametrize("eps", [1e-20, 2.0 ** -63.5, 2.0 ** -63, 1e-6])
+def test_softening_about_the_smallest_normal_square(gpu, rt, oracle, eps, compensated):
+    """The traversal takes the reciprocal square root without subnormal inputs
+    where the f32 softening squared is a normal number (2^-63 and up): forces of
+    a group 1e-19 across, whose squared distances are subnormal, on both sides
+    of that limit, against the reference traversal (whose softening is f64)."""
+    rng = np.random.default_rng(8)
+    n = 40
+    bodies = np.zeros((n, 5))
+    bodies[:, :2] = rng.uniform(-1.0, 1.0, (n, 2))
+    bodies[:8, :2] = rng.uniform(-1e-19, 1e-19, (8, 2))
+    bodies[:, 4] = 1e-30
+    cfg = Config(theta=0.5, softening_kpc=eps, g=1.0, bucket=8, compensated=compensated)
+    ev, tree, evid, ot, b32, oc = build_both(gpu, rt, oracle, bodies, cfg)
+    rt.force(gpu, ev, tree, cfg)
+    acc, _ = gpu.read_evolving_accelerations(ev)
+    ref, _, s = oracle.flat_accelerations(b32, ot, oc, abs_sum=True)
+    err = np.hypot(acc[:, 0] - ref[:, 0], acc[:, 1] - ref[:, 1])
+    # f32 terms: (8 + n) 2^-24 of their magnitudes, except that a squared distance
+    # or softening below 2^-126 itself carries 2^-149 of absolute rounding, at
+    # most 3 2^-23 of the power 3/2 at 2^-128 (1e-20 squared, the smallest here,
+    # adds to squared distances of about 1e-38)
+    assert (err <= (8.0 + n) * 2.0 ** -24 * s + 1e-5 * s).all()
