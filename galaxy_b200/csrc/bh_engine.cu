@@ -793,6 +793,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.err = (uint32_t*)take(A.err);
     bb.force_stats = (unsigned long long*)take(A.stats);
     bb.nsims = count;
+    bb.max_bodies = *std::max_element(counts.begin(), counts.end());
     bb.npos = L.npos;
     bb.nchunks = L.nchunks;
     bb.ntiles = L.ntiles;
@@ -877,11 +878,12 @@ static int enqueue_rebuild(Batch* b, int integrate_mode, cudaEvent_t* ev) {
     CK(cudaMemsetAsync(b->control, 0, b->control_bytes, s), "control memset");
     CK(launch_integrate(b->bb, integrate_mode, s), "integrate launch");
     if (ev) CK(cudaEventRecord(ev[1], s), "event");
-    CK(launch_morton(b->bb, s), "morton launch");
+    const bool small = small_sort(b->bb);  // one launch, timed as the radix stage
+    if (!small) CK(launch_morton(b->bb, s), "morton launch");
     if (ev) CK(cudaEventRecord(ev[2], s), "event");
-    CK(launch_radix(b->bb, s), "radix launch");
+    CK(small ? launch_sort_small(b->bb, s) : launch_radix(b->bb, s), "radix launch");
     if (ev) CK(cudaEventRecord(ev[3], s), "event");
-    CK(launch_count_scan(b->bb, s), "count/scan launch");
+    if (!small || b->bb.nsims > 1) CK(launch_count_scan(b->bb, s), "count/scan launch");
     CK(launch_cells(b->bb, s), "cells launch");
     if (ev) CK(cudaEventRecord(ev[4], s), "event");
     CK(launch_aggregate(b->bb, s), "aggregate launch");

@@ -20,6 +20,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;  // 1024-position scan tiles: a shorter per-tile chain
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // positions per scan tile
 constexpr uint32_t kMortonDepth = 16;
+constexpr uint32_t kSmallSort = 4096;  // bodies one block sorts (k_sort_small)
 
 // Error bits accumulated in the device error word until the host reads it.
 enum : uint32_t {
@@ -83,6 +84,7 @@ struct BatchBuffers {
     const uint32_t* chunk_sim;  // P/32 entries, kNone for unused chunks
     const Tile* tiles;
     uint32_t nsims;
+    uint32_t max_bodies;  // of one simulation
     uint32_t npos;     // P, multiple of 32
     uint32_t nchunks;  // P / 32
     uint32_t ntiles;
@@ -124,6 +126,10 @@ struct BatchBuffers {
 cudaError_t launch_integrate(const BatchBuffers& b, int mode, cudaStream_t s);
 cudaError_t launch_morton(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s);
+// Whether Morton codes, sort and gather run as launch_sort_small (which also
+// does launch_count_scan's work for a single simulation).
+bool small_sort(const BatchBuffers& b);
+cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_cells(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s);

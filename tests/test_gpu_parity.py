@@ -735,3 +735,32 @@ def test_softening_about_the_smallest_normal_square(gpu, rt, oracle, eps, compen
     # most 3 2^-23 of the power 3/2 at 2^-128 (1e-20 squared, the smallest here,
     # adds to squared distances of about 1e-38)
     assert (err <= (8.0 + n) * 2.0 ** -24 * s + 1e-5 * s).all()
+
+
+@pytest.mark.parametrize("bucket", [1, 5])
+def test_one_block_sort_at_its_edges(gpu, rt, oracle, bucket):
+    """Simulations of at most 4,096 bodies are sorted by one block, 1, 2 or 4
+    keys a thread: sizes at those edges, half the bodies on a lattice of equal
+    codes (the stable order), alone and in a batch (whose chain counts are
+    scanned by another kernel).  Bit for bit, so no tolerance."""
+    import dataclasses as dc
+
+    from galaxy_b200.batch import Batch
+    rng = np.random.default_rng(12)
+    cfg = Config(theta=0.5, softening_kpc=0.02, g=1.0, bucket=bucket)
+    states, alone = [], []
+    for n in (2, 33, 1000, 1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096):
+        bodies = np.zeros((n, 5))
+        bodies[:, :2] = rng.uniform(-1, 1, (n, 2))
+        half = n // 2
+        bodies[:half, :2] = rng.integers(0, 5, (half, 2)) / 4.0
+        bodies = bodies[rng.permutation(n)]
+        bodies[:, 4] = rng.uniform(0.5, 2.0, n) / n
+        ev, tree, evid, ot, b32, oc = build_both(gpu, rt, oracle, bodies, cfg)
+        assert_tree_bit_exact(oracle, evid, ot, b32, oc, cfg)
+        rt.force(gpu, ev, tree, dc.replace(cfg, force_stats=False))
+        alone.append(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32))
+        states.append(gpu.create_evolving_state(bodies)[0])
+    Batch(gpu, states, [dc.replace(cfg, force_stats=False)] * len(states)).solve()
+    for ev, want in zip(states, alone):
+        assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
