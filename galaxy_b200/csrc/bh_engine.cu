@@ -548,7 +548,7 @@ extern "C" int galaxy_bh_direct_probes(bh_device* dev, bh_state* st, const bh_co
     uint32_t* d_p = nullptr;
     double* d_o = nullptr;
     cudaError_t e = cudaMalloc(&d_p, 4ull * nprobes);
-    if (!e) e = cudaMalloc(&d_o, 16ull * nprobes);
+    if (!e) e = cudaMalloc(&d_o, 16ull * nprobes * probe_slices(st->n, nprobes));
     if (!e) e = cudaMemcpyAsync(d_p, probes, 4ull * nprobes, cudaMemcpyHostToDevice, dev->stream);
     if (!e)
         e = launch_direct_probes(st->d_state, st->n, d_p, nprobes, cfg->softening, cfg->g, d_o,

@@ -151,7 +151,10 @@ cudaError_t launch_traverse_packed(const BhSettings* settings, const GpuBody* bo
                                    const GpuEntry* entries, const GpuCell* cells, uint32_t n,
                                    uint32_t ncells, float4* accel, uint32_t* err,
                                    cudaStream_t s);
-// FP64 direct accelerations of nprobes probe bodies (out: 2 doubles each).
+// FP64 direct accelerations of nprobes probe bodies: out holds 2 nprobes
+// doubles for each of probe_slices(n, nprobes) slices, the first of which get
+// the results.
+uint32_t probe_slices(uint32_t n, uint32_t nprobes);
 cudaError_t launch_direct_probes(const GpuEvolveState* state, uint32_t n, const uint32_t* probes,
                                  uint32_t nprobes, double eps, double g, double* out,
                                  cudaStream_t s);

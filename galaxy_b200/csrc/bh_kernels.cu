@@ -2613,11 +2613,15 @@ constexpr int kProbesPerBlock = 8;
 // FP64 direct sums for probe bodies (direct_acceleration_for,
 // nbody/src/lib.rs:315-329, over the f32 state promoted to f64): every term
 // is nbody/src/lib.rs:247-255 with explicit round-to-nearest f64 operations;
-// each thread sums a strided slice of the sources and the block adds the
-// slices in a fixed order.
+// each thread sums a strided share of a slice of the sources, the block adds
+// the shares in a fixed order and k_add_slices the slices.  The slices (grid.y)
+// fill the chip whatever the number of probes: with every source in one block
+// 4,096 probes were 512 blocks, 1.15 waves of the 444 resident ones, and 12
+// probes 2 blocks; 4,096 probes of 2^20 bodies, a whole call, 16.3 -> 10.0 ms.
+// The f64 pipe bounds it (a square root and a division per term).
 __global__ void __launch_bounds__(kProbeThreads) k_direct_probes(
     const GpuEvolveState* __restrict__ state, uint32_t n, const uint32_t* __restrict__ probes,
-    uint32_t nprobes, double eps, double g, double* __restrict__ out) {
+    uint32_t nprobes, uint32_t slice, double eps, double g, double* __restrict__ out) {
     __shared__ double sh[kProbesPerBlock][2][kProbeThreads];
     double tx[kProbesPerBlock], ty[kProbesPerBlock], ax[kProbesPerBlock], ay[kProbesPerBlock];
     uint32_t ti[kProbesPerBlock];
@@ -2631,7 +2635,8 @@ __global__ void __launch_bounds__(kProbeThreads) k_direct_probes(
         ax[k] = ay[k] = 0.0;
     }
     const double eps2 = __dmul_rn(eps, eps);
-    for (uint32_t j = threadIdx.x; j < n; j += kProbeThreads) {
+    const uint32_t end = min(n - blockIdx.y * slice, slice) + blockIdx.y * slice;
+    for (uint32_t j = blockIdx.y * slice + threadIdx.x; j < end; j += kProbeThreads) {
         const float4 pm = *reinterpret_cast<const float4*>(state + j);
         const double x = pm.x, y = pm.y, m = pm.z;
         const double gm = __dmul_rn(g, m);
@@ -2665,17 +2670,42 @@ __global__ void __launch_bounds__(kProbeThreads) k_direct_probes(
     if (threadIdx.x < kProbesPerBlock) {
         const uint32_t q = blockIdx.x * kProbesPerBlock + threadIdx.x;
         if (q < nprobes) {
-            out[2 * q] = sh[threadIdx.x][0][0];
-            out[2 * q + 1] = sh[threadIdx.x][1][0];
+            double* slot = out + 2 * ((size_t)blockIdx.y * nprobes + q);
+            slot[0] = sh[threadIdx.x][0][0];
+            slot[1] = sh[threadIdx.x][1][0];
         }
     }
+}
+
+// out[i] = the sum of the slices' values, in slice order; values[0] may be out.
+__global__ void __launch_bounds__(256) k_add_slices(const double* values, uint32_t count,
+                                                    uint32_t slices, double* out) {
+    const uint32_t i = blockIdx.x * 256u + threadIdx.x;
+    if (i >= count) return;
+    double sum = values[i];
+    for (uint32_t k = 1; k < slices; ++k) sum += values[(size_t)k * count + i];
+    out[i] = sum;
+}
+
+// Slices of the sources: enough blocks for about ten waves (a last one that is
+// nearly empty then costs little), of at least 2,048 sources each.
+uint32_t probe_slices(uint32_t n, uint32_t nprobes) {
+    const uint64_t blocks = (nprobes + kProbesPerBlock - 1ull) / kProbesPerBlock;
+    const uint64_t want = 4440ull / blocks, most = (n + 2047ull) / 2048ull;
+    const uint64_t slices = want < most ? want : most;
+    return slices ? (uint32_t)slices : 1u;
 }
 
 cudaError_t launch_direct_probes(const GpuEvolveState* state, uint32_t n, const uint32_t* probes,
                                  uint32_t nprobes, double eps, double g, double* out,
                                  cudaStream_t s) {
     const uint32_t blocks = (nprobes + kProbesPerBlock - 1) / kProbesPerBlock;
-    k_direct_probes<<<blocks, kProbeThreads, 0, s>>>(state, n, probes, nprobes, eps, g, out);
+    const uint32_t want = probe_slices(n, nprobes);
+    const uint32_t slice = (n + want - 1) / want, slices = (n + slice - 1) / slice;
+    k_direct_probes<<<dim3(blocks, slices), kProbeThreads, 0, s>>>(state, n, probes, nprobes, slice,
+                                                                  eps, g, out);
+    if (slices > 1)
+        k_add_slices<<<(2 * nprobes + 255) / 256, 256, 0, s>>>(out, 2 * nprobes, slices, out);
     return cudaGetLastError();
 }
 

@@ -764,3 +764,24 @@ def test_one_block_sort_at_its_edges(gpu, rt, oracle, bucket):
     Batch(gpu, states, [dc.replace(cfg, force_stats=False)] * len(states)).solve()
     for ev, want in zip(states, alone):
         assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
+
+
+@pytest.mark.parametrize("n,probes", [(2, 1), (2047, 2), (2049, 8), (4097, 9), (30001, 64),
+                                      (30001, 30001)])
+def test_direct_probes_in_slices(gpu, oracle, n, probes):
+    """The sources are summed in slices of at least 2,048: sizes at a slice's
+    edge, few probes (many slices) and as many as bodies (few).  A sum of n f64
+    terms in any order is off by at most n 2^-53 of their magnitudes, and a
+    term by a few 2^-53 in either code."""
+    cfg = Config(theta=0.5, softening_kpc=0.01, g=1.0, bucket=1)
+    bodies = scenarios.exponential_disc(n, 4)
+    ev, _ = gpu.create_evolving_state(bodies)
+    b32 = f32_bodies(bodies)
+    index = np.random.default_rng(2).choice(n, probes, replace=False).astype(np.uint32)
+    got = gpu.direct_probes(ev, cfg, index)
+    want = oracle.direct_accelerations_for(b32, ocfg(oracle, cfg), index[:200])
+    d = b32[None, :, :2] - b32[index[:200], None, :2]
+    r2 = (d ** 2).sum(-1) + 0.01 ** 2
+    mags = (b32[None, :, 4] * np.sqrt((d ** 2).sum(-1)) / r2 ** 1.5).sum(1)
+    err = np.hypot(*(got[:200] - want).T)
+    assert (err <= (n + 16) * 2.0 ** -52 * mags).all()
