@@ -2816,7 +2816,8 @@ constexpr int kConsThreads = 256;
 constexpr int kConsTerms = 9;
 
 // Per-block f64 partial sums in a fixed order, then one block adds the
-// partials in block order: the result does not depend on scheduling.
+// partials, a warp per term, in a fixed order: the result does not depend on
+// scheduling.
 __global__ void __launch_bounds__(kConsThreads) k_conservation_partial(
     const GpuEvolveState* __restrict__ state, const float* __restrict__ potential, uint32_t n,
     double* partials) {
@@ -2849,11 +2850,17 @@ __global__ void __launch_bounds__(kConsThreads) k_conservation_partial(
     if (threadIdx.x < kConsTerms) partials[blockIdx.x * kConsTerms + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-__global__ void k_conservation_final(const double* partials, uint32_t nblocks, double* out) {
-    if (threadIdx.x >= kConsTerms) return;
+// A warp per term: lane l adds partials l, l + 32, ..., the lanes pairwise.  (One
+// thread per term was a chain of 592 additions behind their loads: a call at
+// 262,147 bodies 51 -> 36 us, at 2^22 83 -> 53.)
+__global__ void __launch_bounds__(32 * kConsTerms) k_conservation_final(
+    const double* __restrict__ partials, uint32_t nblocks, double* out) {
+    const uint32_t term = threadIdx.x >> 5;
     double acc = 0.0;
-    for (uint32_t b = 0; b < nblocks; ++b) acc += partials[b * kConsTerms + threadIdx.x];
-    out[threadIdx.x] = acc;
+    for (uint32_t b = lane_id(); b < nblocks; b += 32u) acc += partials[b * kConsTerms + term];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(kFull, acc, o);
+    if (lane_id() == 0) out[term] = acc;
 }
 
 // ============================================================ launchers ===
@@ -3106,7 +3113,7 @@ cudaError_t launch_conservation(const GpuEvolveState* state, const float* potent
                                 double* partials, uint32_t nblocks, double* out,
                                 cudaStream_t s) {
     k_conservation_partial<<<nblocks, kConsThreads, 0, s>>>(state, potential, n, partials);
-    k_conservation_final<<<1, 32, 0, s>>>(partials, nblocks, out);
+    k_conservation_final<<<1, 32 * kConsTerms, 0, s>>>(partials, nblocks, out);
     return cudaGetLastError();
 }
 

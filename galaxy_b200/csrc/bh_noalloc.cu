@@ -73,12 +73,16 @@ __global__ void __launch_bounds__(kThreads) k_conservation_slices(const GpuEvolv
     if (threadIdx.x < kTerms) partials[blockIdx.x * kTerms + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-// Adds the rows of this call's blocks in block order into out[0..kTerms).
-__global__ void k_conservation_rows(const double* partials, uint32_t nblocks, double* out) {
-    if (threadIdx.x >= kTerms) return;
+// Adds the rows of this call's blocks in a fixed order into out[0..kTerms): a
+// warp per term, lane l rows l, l + 32, ..., then the lanes pairwise.
+__global__ void __launch_bounds__(32 * kTerms) k_conservation_rows(
+    const double* __restrict__ partials, uint32_t nblocks, double* out) {
+    const uint32_t term = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     double acc = 0.0;
-    for (uint32_t b = 0; b < nblocks; ++b) acc += partials[b * kTerms + threadIdx.x];
-    out[threadIdx.x] = acc;
+    for (uint32_t b = lane; b < nblocks; b += 32u) acc += partials[b * kTerms + term];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) out[term] = acc;
 }
 
 static std::mutex g_setup_mutex;
@@ -154,7 +158,7 @@ extern "C" int galaxy_bh_conservation_noalloc(const GpuEvolveState* state, const
         }
     }
     k_conservation_slices<<<blocks, kThreads, 0, s>>>(state, potential, n, scratch);
-    k_conservation_rows<<<1, 32, 0, s>>>(scratch, blocks, sums);
+    k_conservation_rows<<<1, 32 * kTerms, 0, s>>>(scratch, blocks, sums);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         char msg[256];
