@@ -19,6 +19,7 @@
 #include <cstring>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "bh_internal.cuh"
@@ -66,6 +67,136 @@ extern "C" size_t galaxy_bh_last_error(char* buf, size_t len) {
 
 extern "C" uint32_t galaxy_bh_abi_version(void) { return GALAXY_BH_ABI_VERSION; }
 
+// ------------------------------------------------------------ host copies --
+
+// Copies between device memory and a caller's pageable arrays, through pinned
+// slots and with a few threads: the driver's own staging is one thread that
+// faults in the caller's pages one by one.  Each thread takes every W-th chunk
+// and has two slots, so its memcpy of one chunk runs beside the transfer of the
+// next: read-back of 2^20 states 7.6 -> 3.3 ms, of 2^22 27.8 -> 13.0, upload of
+// 2^22 12 -> 5.3.  The slots (4 MB) belong to the device handle and are made by
+// its first copy that uses them (about 8 ms, once).  Arrays that are pinned
+// already are copied as they are, and so are those below 16 MB: from 4 to 8 MB
+// the threads cost up to a fifth more than they save, at 12 MB 10 % less, and a
+// handle that moves no more than that need not pay for the slots.
+class HostCopies {
+public:
+    // Returns once a device-to-host copy is complete; a host-to-device one may
+    // still be running on the stream, but its source can be reused.
+    cudaError_t run(void* dst, const void* src, size_t bytes, bool to_host, cudaStream_t stream,
+                    int ordinal) {
+        const void* host = to_host ? dst : src;
+        cudaPointerAttributes at{};
+        const bool pageable = cudaPointerGetAttributes(&at, host) != cudaSuccess ||
+                              at.type == cudaMemoryTypeUnregistered;
+        cudaGetLastError();
+        if (!pageable || bytes < kStagedBytes || !ready())
+            return cudaMemcpyAsync(dst, src, bytes,
+                                   to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream);
+        const size_t chunks = (bytes + kChunk - 1) / kChunk;
+        const int workers = (int)std::min<size_t>(kWorkers, chunks);
+        cudaError_t result[kWorkers] = {};
+        auto work = [&](int w) {
+            result[w] = cudaSetDevice(ordinal);
+            if (result[w] == cudaSuccess)
+                result[w] = to_host ? down(w, workers, (char*)dst, (const char*)src, bytes, stream)
+                                    : up(w, workers, (char*)dst, (const char*)src, bytes, stream);
+        };
+        std::thread threads[kWorkers];
+        for (int w = 1; w < workers; ++w) {
+            try {
+                threads[w] = std::thread(work, w);
+            } catch (...) {  // no thread to be had: its share is done here
+                work(w);
+            }
+        }
+        work(0);
+        cudaError_t e = result[0];
+        for (int w = 1; w < workers; ++w) {
+            if (threads[w].joinable()) threads[w].join();
+            if (e == cudaSuccess) e = result[w];
+        }
+        return e;
+    }
+
+    void release() {
+        for (auto& s : slots_)
+            if (s.done) cudaEventDestroy(s.done);
+        if (pinned_) cudaFreeHost(pinned_);
+        *this = HostCopies();
+    }
+
+private:
+    static constexpr size_t kChunk = 512u << 10, kStagedBytes = 16u << 20;
+    static constexpr int kWorkers = 4;
+    struct Slot {
+        char* at = nullptr;
+        cudaEvent_t done = nullptr;
+        bool used = false;
+    };
+
+    bool ready() {
+        if (pinned_) return true;
+        if (cudaMallocHost((void**)&pinned_, kChunk * 2 * kWorkers) != cudaSuccess) {
+            cudaGetLastError();
+            pinned_ = nullptr;
+            return false;
+        }
+        for (int k = 0; k < 2 * kWorkers; ++k) {
+            slots_[k].at = pinned_ + kChunk * k;
+            if (cudaEventCreateWithFlags(&slots_[k].done, cudaEventDisableTiming) != cudaSuccess) {
+                cudaGetLastError();
+                release();
+                return false;
+            }
+        }
+        return true;
+    }
+
+    cudaError_t down(int w, int workers, char* dst, const char* src, size_t bytes,
+                     cudaStream_t stream) {
+        size_t pending = bytes;  // offset of the chunk in the other slot
+        int k = 0;
+        auto finish = [&](int slot, size_t at) -> cudaError_t {
+            const cudaError_t e = cudaEventSynchronize(slots_[slot].done);
+            if (e == cudaSuccess)
+                memcpy(dst + at, slots_[slot].at, std::min(kChunk, bytes - at));
+            return e;
+        };
+        for (size_t at = (size_t)w * kChunk; at < bytes; at += workers * kChunk, k ^= 1) {
+            Slot& s = slots_[2 * w + k];
+            cudaError_t e = cudaMemcpyAsync(s.at, src + at, std::min(kChunk, bytes - at),
+                                            cudaMemcpyDeviceToHost, stream);
+            if (e == cudaSuccess) e = cudaEventRecord(s.done, stream);
+            if (e == cudaSuccess && pending < bytes) e = finish(2 * w + (k ^ 1), pending);
+            if (e != cudaSuccess) return e;
+            s.used = false;  // waited for below or in the next turn
+            pending = at;
+        }
+        return pending < bytes ? finish(2 * w + (k ^ 1), pending) : cudaSuccess;
+    }
+
+    cudaError_t up(int w, int workers, char* dst, const char* src, size_t bytes,
+                   cudaStream_t stream) {
+        int k = 0;
+        for (size_t at = (size_t)w * kChunk; at < bytes; at += workers * kChunk, k ^= 1) {
+            Slot& s = slots_[2 * w + k];
+            cudaError_t e = s.used ? cudaEventSynchronize(s.done) : cudaSuccess;
+            if (e != cudaSuccess) return e;
+            const size_t size = std::min(kChunk, bytes - at);
+            memcpy(s.at, src + at, size);
+            e = cudaMemcpyAsync(dst + at, s.at, size, cudaMemcpyHostToDevice, stream);
+            if (e == cudaSuccess) e = cudaEventRecord(s.done, stream);
+            if (e != cudaSuccess) return e;
+            s.used = true;
+        }
+        return cudaSuccess;
+    }
+
+    char* pinned_ = nullptr;
+    Slot slots_[2 * kWorkers];
+};
+
 // ------------------------------------------------------------------ device --
 
 struct bh_device {
@@ -81,11 +212,45 @@ struct bh_device {
     // unmaps pages, which cost a serving loop seconds per burst of finished
     // requests and would stall it on its stager's work.
     cudaMemPool_t pool = nullptr;
+    HostCopies copies;
+};
+
+static cudaError_t copy_down(bh_device* dev, void* host, const void* device, size_t bytes) {
+    return dev->copies.run(host, device, bytes, true, dev->stream, dev->ordinal);
+}
+static cudaError_t copy_up(bh_device* dev, void* device, const void* host, size_t bytes) {
+    return dev->copies.run(device, host, bytes, false, dev->stream, dev->ordinal);
+}
+
+// Device memory of one call from the handle's pool (no device-wide
+// synchronisation, as cudaMalloc and cudaFree have), given back in stream order.
+struct PoolBlock {
+    bh_device* dev;
+    char* at = nullptr;
+    explicit PoolBlock(bh_device* d) : dev(d) {}
+    PoolBlock(const PoolBlock&) = delete;
+    PoolBlock& operator=(const PoolBlock&) = delete;
+    cudaError_t get(size_t bytes) {
+        cudaError_t e = cudaMallocFromPoolAsync((void**)&at, bytes, dev->pool, dev->stream);
+        if (e == cudaErrorMemoryAllocation) {
+            // give back what the pool keeps unused, then retry
+            cudaGetLastError();
+            cudaStreamSynchronize(dev->stream);
+            cudaMemPoolTrimTo(dev->pool, 0);
+            e = cudaMallocFromPoolAsync((void**)&at, bytes, dev->pool, dev->stream);
+        }
+        if (e != cudaSuccess) at = nullptr;
+        return e;
+    }
+    ~PoolBlock() {
+        if (at) cudaFreeAsync(at, dev->stream);
+    }
 };
 
 static void device_free(bh_device* dev) {
     cudaSetDevice(dev->ordinal);
     cudaStreamSynchronize(dev->stream);
+    dev->copies.release();
     if (dev->pool) cudaMemPoolDestroy(dev->pool);
     for (auto& ev : dev->ev) cudaEventDestroy(ev);
     cudaStreamDestroy(dev->stream);
@@ -298,8 +463,7 @@ extern "C" int galaxy_bh_state_create(bh_device* dev, const GpuEvolveState* host
     st->h_sim.accel = st->d_accel;
     st->h_sim.off = 0;
     st->h_sim.n = n;
-    if ((e = cudaMemcpyAsync(st->d_state, host, sizeof(GpuEvolveState) * (size_t)n,
-                             cudaMemcpyHostToDevice, dev->stream)) ||
+    if ((e = copy_up(dev, st->d_state, host, sizeof(GpuEvolveState) * (size_t)n)) ||
         (e = cudaMemsetAsync(st->d_accel, 0, sizeof(float4) * (size_t)n, dev->stream)) ||
         (e = cudaMemcpyAsync(st->d_chunk_sim, chunk.data(), 4 * chunk.size(),
                              cudaMemcpyHostToDevice, dev->stream)) ||
@@ -463,9 +627,7 @@ extern "C" int galaxy_bh_read_state(bh_device* dev, bh_state* st, GpuEvolveState
     // device records (bitwise the same values) while they are copied out
     if ((rc = enqueue_check(st, st->d_state, 0, n))) return rc;
     CK(cudaEventRecord(dev->ev[0], dev->stream), "event record");
-    CK(cudaMemcpyAsync(out, st->d_state, sizeof(GpuEvolveState) * (size_t)n,
-                       cudaMemcpyDeviceToHost, dev->stream),
-       "state readback");
+    CK(copy_down(dev, out, st->d_state, sizeof(GpuEvolveState) * (size_t)n), "state readback");
     CK(cudaEventRecord(dev->ev[1], dev->stream), "event record");
     uint32_t bad = kNone;
     if ((rc = fetch_check(st, &bad))) return rc;
@@ -488,9 +650,7 @@ extern "C" int galaxy_bh_read_accel(bh_device* dev, bh_state* st, GpuAccel* out,
     // nbody_gpu.rs:1097-1101, evaluated on the device records
     if ((rc = enqueue_check(st, st->d_accel, 1, n))) return rc;
     CK(cudaEventRecord(dev->ev[0], dev->stream), "event record");
-    CK(cudaMemcpyAsync(out, st->d_accel, sizeof(float4) * (size_t)n, cudaMemcpyDeviceToHost,
-                       dev->stream),
-       "acceleration readback");
+    CK(copy_down(dev, out, st->d_accel, sizeof(float4) * (size_t)n), "acceleration readback");
     CK(cudaEventRecord(dev->ev[1], dev->stream), "event record");
     uint32_t bad = kNone;
     if ((rc = fetch_check(st, &bad))) return rc;
@@ -514,9 +674,7 @@ extern "C" int galaxy_bh_write_state(bh_device* dev, bh_state* st, const GpuEvol
     // replace the resident state: an invalid upload leaves it untouched.
     if (!st->d_stage)
         CK(cudaMalloc(&st->d_stage, sizeof(GpuEvolveState) * (size_t)n), "staging allocation");
-    CK(cudaMemcpyAsync(st->d_stage, host, sizeof(GpuEvolveState) * (size_t)n,
-                       cudaMemcpyHostToDevice, dev->stream),
-       "state upload");
+    CK(copy_up(dev, st->d_stage, host, sizeof(GpuEvolveState) * (size_t)n), "state upload");
     if ((rc = enqueue_check(st, st->d_stage, 0, n))) return rc;
     uint32_t bad = kNone;
     if ((rc = fetch_check(st, &bad))) return rc;
@@ -545,18 +703,17 @@ extern "C" int galaxy_bh_direct_probes(bh_device* dev, bh_state* st, const bh_co
     if (nprobes == 0) return BH_OK;
     for (uint32_t k = 0; k < nprobes; ++k)
         if (probes[k] >= st->n) return set_error(BH_INVALID_ARG, "body index is out of range");
-    uint32_t* d_p = nullptr;
-    double* d_o = nullptr;
-    cudaError_t e = cudaMalloc(&d_p, 4ull * nprobes);
-    if (!e) e = cudaMalloc(&d_o, 16ull * nprobes * probe_slices(st->n, nprobes));
+    const size_t sums = 16ull * nprobes * probe_slices(st->n, nprobes);
+    PoolBlock block(dev);
+    cudaError_t e = block.get(sums + 4ull * nprobes);
+    double* d_o = reinterpret_cast<double*>(block.at);
+    uint32_t* d_p = reinterpret_cast<uint32_t*>(block.at + sums);
     if (!e) e = cudaMemcpyAsync(d_p, probes, 4ull * nprobes, cudaMemcpyHostToDevice, dev->stream);
     if (!e)
         e = launch_direct_probes(st->d_state, st->n, d_p, nprobes, cfg->softening, cfg->g, d_o,
                                  dev->stream);
-    if (!e) e = cudaMemcpyAsync(out, d_o, 16ull * nprobes, cudaMemcpyDeviceToHost, dev->stream);
+    if (!e) e = copy_down(dev, out, d_o, 16ull * nprobes);
     if (!e) e = cudaStreamSynchronize(dev->stream);
-    cudaFree(d_p);
-    cudaFree(d_o);
     if (e) return cuda_fail(e, "direct probes");
     return BH_OK;
 }
@@ -1136,8 +1293,9 @@ extern "C" int galaxy_bh_force_f64(bh_device* dev, bh_state* st, bh_tree* tree,
     if (!tree->built) return set_error(BH_INVALID_ARG, "force requires a rebuilt tree");
     const size_t n = st->n;
     const size_t bytes = 16 * n + (abs_sum ? 8 * n : 0) + 32;
-    char* d = nullptr;
-    CK(cudaMalloc(&d, bytes), "f64 traversal allocation");
+    PoolBlock block(dev);
+    CK(block.get(bytes), "f64 traversal allocation");
+    char* d = block.at;
     double* d_acc = reinterpret_cast<double*>(d);
     double* d_abs = abs_sum ? reinterpret_cast<double*>(d + 16 * n) : nullptr;
     unsigned long long* d_stats = reinterpret_cast<unsigned long long*>(d + bytes - 32);
@@ -1146,12 +1304,10 @@ extern "C" int galaxy_bh_force_f64(bh_device* dev, bh_state* st, bh_tree* tree,
     if (!e)
         e = launch_traverse_f64(tree->batch->bb, 0, st->n, cfg->theta, cfg->softening, cfg->g,
                                 d_acc, d_abs, d_stats, dev->stream);
-    if (!e) e = cudaMemcpyAsync(accel, d_acc, 16 * n, cudaMemcpyDeviceToHost, dev->stream);
-    if (!e && abs_sum)
-        e = cudaMemcpyAsync(abs_sum, d_abs, 8 * n, cudaMemcpyDeviceToHost, dev->stream);
+    if (!e) e = copy_down(dev, accel, d_acc, 16 * n);
+    if (!e && abs_sum) e = copy_down(dev, abs_sum, d_abs, 8 * n);
     if (!e) e = cudaMemcpyAsync(h_stats, d_stats, 24, cudaMemcpyDeviceToHost, dev->stream);
     if (!e) e = cudaStreamSynchronize(dev->stream);
-    cudaFree(d);
     if (e) return cuda_fail(e, "f64 traversal");
     if (stats) {
         *stats = bh_force_stats{};
@@ -1220,21 +1376,22 @@ extern "C" int galaxy_bh_read_tree_evidence(bh_device* dev, bh_tree* tree, TreeM
     if (cells && cell_capacity < ncell)
         return set_error(BH_CAPACITY_OVERFLOW, "cell buffer holds %u records, tree has %u",
                          cell_capacity, ncell);
-    GpuEntry* d_e = nullptr;
-    GpuBody* d_b = nullptr;
-    GpuCell* d_c = nullptr;
-    cudaError_t e = cudaSuccess;
-    if (entries) e = cudaMalloc(&d_e, sizeof(GpuEntry) * (size_t)sn);
-    if (!e && bodies) e = cudaMalloc(&d_b, sizeof(GpuBody) * (size_t)sn);
-    if (!e && cells && ncell) e = cudaMalloc(&d_c, sizeof(GpuCell) * (size_t)ncell);
-    if (!e) e = launch_export(b->bb, 0, d_e, d_b, d_c, s);
-    if (!e && entries) e = cudaMemcpyAsync(entries, d_e, sizeof(GpuEntry) * (size_t)sn, cudaMemcpyDeviceToHost, s);
-    if (!e && bodies) e = cudaMemcpyAsync(bodies, d_b, sizeof(GpuBody) * (size_t)sn, cudaMemcpyDeviceToHost, s);
-    if (!e && cells && ncell) e = cudaMemcpyAsync(cells, d_c, sizeof(GpuCell) * (size_t)ncell, cudaMemcpyDeviceToHost, s);
+    const size_t cells_bytes = cells ? sizeof(GpuCell) * (size_t)ncell : 0;
+    const size_t bodies_bytes = bodies ? sizeof(GpuBody) * (size_t)sn : 0;
+    const size_t entries_bytes = entries ? sizeof(GpuEntry) * (size_t)sn : 0;
+    if (cells_bytes + bodies_bytes + entries_bytes == 0) return BH_OK;
+    PoolBlock block(dev);
+    cudaError_t e = block.get(cells_bytes + bodies_bytes + entries_bytes);
+    GpuCell* d_c = reinterpret_cast<GpuCell*>(block.at);
+    GpuBody* d_b = reinterpret_cast<GpuBody*>(block.at + cells_bytes);
+    GpuEntry* d_e = reinterpret_cast<GpuEntry*>(block.at + cells_bytes + bodies_bytes);
+    if (!e)
+        e = launch_export(b->bb, 0, entries_bytes ? d_e : nullptr, bodies_bytes ? d_b : nullptr,
+                          cells_bytes ? d_c : nullptr, s);
+    if (!e && entries_bytes) e = copy_down(dev, entries, d_e, entries_bytes);
+    if (!e && bodies_bytes) e = copy_down(dev, bodies, d_b, bodies_bytes);
+    if (!e && cells_bytes) e = copy_down(dev, cells, d_c, cells_bytes);
     if (!e) e = cudaStreamSynchronize(s);
-    cudaFree(d_e);
-    cudaFree(d_b);
-    cudaFree(d_c);
     if (e) return cuda_fail(e, "tree evidence");
     return BH_OK;
 }
@@ -1283,50 +1440,62 @@ static int packed_checks(const BhSettings* settings, const GpuBody* bodies, uint
     return BH_OK;
 }
 
+// Uploads the packed records and walks them; d_out: the accelerations, or null
+// to keep them in the call's own block and copy them to `out`.
 static int run_packed(bh_device* dev, const BhSettings* settings, const GpuBody* bodies,
                       uint32_t n, const GpuEntry* entries, const GpuCell* cells,
-                      uint32_t cell_count, float4* d_out, bh_stage_timing* timing) {
+                      uint32_t cell_count, float4* d_out, GpuAccel* out,
+                      bh_stage_timing* timing) {
     cudaStream_t s = dev->stream;
-    BhSettings* d_s = nullptr;
-    GpuBody* d_b = nullptr;
-    GpuEntry* d_e = nullptr;
-    GpuCell* d_c = nullptr;
-    uint32_t* d_err = nullptr;
-    cudaError_t e = cudaSuccess;
-    uint32_t err = 0;
-    float t_up = 0.f, t_k = 0.f;
-    if ((e = cudaMalloc(&d_s, sizeof(BhSettings))) ||
-        (e = cudaMalloc(&d_b, sizeof(GpuBody) * (size_t)n)) ||
-        (e = cudaMalloc(&d_e, sizeof(GpuEntry) * (size_t)n)) ||
-        (e = cudaMalloc(&d_c, sizeof(GpuCell) * (size_t)cell_count)) ||
-        (e = cudaMalloc(&d_err, 8)))
-        goto done;
+    const size_t body_bytes = sizeof(GpuBody) * (size_t)n, entry_bytes = sizeof(GpuEntry) * (size_t)n;
+    const size_t cell_bytes = sizeof(GpuCell) * (size_t)cell_count;
+    const size_t out_bytes = d_out ? 0 : sizeof(float4) * (size_t)n;
+    PoolBlock block(dev);
+    // cells, bodies, settings (32 bytes), entries, accelerations, the walk's two
+    // error words and the first non-finite result
+    CK(block.get(cell_bytes + body_bytes + sizeof(BhSettings) + entry_bytes + out_bytes + 16),
+       "packed traversal allocation");
+    GpuCell* d_c = reinterpret_cast<GpuCell*>(block.at);
+    GpuBody* d_b = reinterpret_cast<GpuBody*>(block.at + cell_bytes);
+    BhSettings* d_s = reinterpret_cast<BhSettings*>((char*)d_b + body_bytes);
+    GpuEntry* d_e = reinterpret_cast<GpuEntry*>(d_s + 1);
+    char* rest = (char*)d_e + entry_bytes;
+    if (!d_out) {
+        d_out = reinterpret_cast<float4*>(rest);
+        CK(cudaMemsetAsync(d_out, 0, out_bytes, s), "memset");
+    }
+    uint32_t* d_err = reinterpret_cast<uint32_t*>(rest + out_bytes);
+    uint32_t err[3] = {0, 0, kNone};
     cudaEventRecord(dev->ev[0], s);
+    cudaError_t e = cudaSuccess;
     if ((e = cudaMemcpyAsync(d_s, settings, sizeof(BhSettings), cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_b, bodies, sizeof(GpuBody) * (size_t)n, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_e, entries, sizeof(GpuEntry) * (size_t)n, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemcpyAsync(d_c, cells, sizeof(GpuCell) * (size_t)cell_count, cudaMemcpyHostToDevice, s)) ||
-        (e = cudaMemsetAsync(d_err, 0, 8, s)))
-        goto done;
+        (e = copy_up(dev, d_b, bodies, body_bytes)) || (e = copy_up(dev, d_e, entries, entry_bytes)) ||
+        (e = copy_up(dev, d_c, cells, cell_bytes)) || (e = cudaMemsetAsync(d_err, 0, 8, s)) ||
+        (e = cudaMemsetAsync(d_err + 2, 0xff, 4, s)))
+        return cuda_fail(e, "packed traversal");
     cudaEventRecord(dev->ev[1], s);
-    if ((e = launch_traverse_packed(d_s, d_b, d_e, d_c, n, cell_count, d_out, d_err, s))) goto done;
+    if ((e = launch_traverse_packed(d_s, d_b, d_e, d_c, n, cell_count, d_out, d_err, s)))
+        return cuda_fail(e, "packed traversal");
     cudaEventRecord(dev->ev[2], s);
-    if ((e = cudaMemcpyAsync(&err, d_err, 4, cudaMemcpyDeviceToHost, s)) ||
+    if (out && ((e = launch_check_records(d_out, 1, n, d_err + 2, s)) ||
+                (e = copy_down(dev, out, d_out, out_bytes))))
+        return cuda_fail(e, "acceleration readback");
+    cudaEventRecord(dev->ev[3], s);
+    if ((e = cudaMemcpyAsync(err, d_err, sizeof err, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
-        goto done;
-    cudaEventElapsedTime(&t_up, dev->ev[0], dev->ev[1]);
-    cudaEventElapsedTime(&t_k, dev->ev[1], dev->ev[2]);
-    if (timing) *timing = bh_stage_timing{t_up * 1e-3, t_k * 1e-3, 0.0};
-done:
-    cudaFree(d_s);
-    cudaFree(d_b);
-    cudaFree(d_e);
-    cudaFree(d_c);
-    cudaFree(d_err);
-    if (e) return cuda_fail(e, "packed traversal");
-    if (err & kErrPackedStack)
+        return cuda_fail(e, "packed traversal");
+    if (timing) {
+        float up = 0.f, walk = 0.f, down = 0.f;
+        cudaEventElapsedTime(&up, dev->ev[0], dev->ev[1]);
+        cudaEventElapsedTime(&walk, dev->ev[1], dev->ev[2]);
+        if (out) cudaEventElapsedTime(&down, dev->ev[2], dev->ev[3]);
+        *timing = bh_stage_timing{up * 1e-3, walk * 1e-3, down * 1e-3};
+    }
+    if (err[0] & kErrPackedStack)
         return set_error(BH_CAPACITY_OVERFLOW, "packed traversal stack exceeded 64 entries");
-    if (err) return set_error(BH_INVALID_ARG, "packed tree holds an out-of-range index");
+    if (err[0]) return set_error(BH_INVALID_ARG, "packed tree holds an out-of-range index");
+    if (out && err[2] != kNone)
+        return set_error(BH_NONFINITE, "GPU produced non-finite acceleration for body %u", err[2]);
     return BH_OK;
 }
 
@@ -1339,31 +1508,7 @@ extern "C" int galaxy_bh_traverse_packed(bh_device* dev, const BhSettings* setti
     if (rc) return rc;
     if (!out) return set_error(BH_INVALID_ARG, "null argument");
     if ((rc = packed_checks(settings, bodies, n, entries, cells, cell_count))) return rc;
-    float4* d_out = nullptr;
-    CK(cudaMalloc(&d_out, sizeof(float4) * (size_t)n), "output allocation");
-    cudaMemsetAsync(d_out, 0, sizeof(float4) * (size_t)n, dev->stream);
-    rc = run_packed(dev, settings, bodies, n, entries, cells, cell_count, d_out, timing);
-    cudaEvent_t* ev = dev->ev;
-    if (!rc) {
-        cudaEventRecord(ev[3], dev->stream);
-        cudaError_t e = cudaMemcpyAsync(out, d_out, sizeof(float4) * (size_t)n,
-                                        cudaMemcpyDeviceToHost, dev->stream);
-        if (!e) e = cudaStreamSynchronize(dev->stream);
-        if (e) rc = cuda_fail(e, "acceleration readback");
-        if (!rc && timing) {
-            float ms = 0.f;
-            cudaEventRecord(ev[4], dev->stream);
-            cudaEventSynchronize(ev[4]);
-            cudaEventElapsedTime(&ms, ev[3], ev[4]);
-            timing->readback_seconds = ms * 1e-3;
-        }
-    }
-    cudaFree(d_out);
-    if (rc) return rc;
-    for (uint32_t i = 0; i < n; ++i)
-        if (!std::isfinite(out[i].value[0]) || !std::isfinite(out[i].value[1]))
-            return set_error(BH_NONFINITE, "GPU produced non-finite acceleration for body %u", i);
-    return BH_OK;
+    return run_packed(dev, settings, bodies, n, entries, cells, cell_count, nullptr, out, timing);
 }
 
 extern "C" int galaxy_bh_force_into(bh_device* dev, bh_state* st, const BhSettings* settings,
@@ -1375,7 +1520,8 @@ extern "C" int galaxy_bh_force_into(bh_device* dev, bh_state* st, const BhSettin
     if (!st) return set_error(BH_INVALID_ARG, "null state");
     if ((rc = packed_checks(settings, bodies, st->n, entries, cells, cell_count)))
         return set_error(rc, "Barnes-Hut force/tree count does not match evolving state");
-    return run_packed(dev, settings, bodies, st->n, entries, cells, cell_count, st->d_accel, timing);
+    return run_packed(dev, settings, bodies, st->n, entries, cells, cell_count, st->d_accel, nullptr,
+                      timing);
 }
 
 // ------------------------------------------------------------ batch API ----

@@ -785,3 +785,19 @@ def test_direct_probes_in_slices(gpu, oracle, n, probes):
     mags = (b32[None, :, 4] * np.sqrt((d ** 2).sum(-1)) / r2 ** 1.5).sum(1)
     err = np.hypot(*(got[:200] - want).T)
     assert (err <= (n + 16) * 2.0 ** -52 * mags).all()
+
+
+@pytest.mark.parametrize("n", [524287, 524288, 524289, 540673])
+def test_large_copies_keep_every_record(gpu, n):
+    """States of 16 MB and more go up and down in chunks of 512 KB over several
+    threads: sizes about that limit and with a short last chunk, twice over."""
+    rng = np.random.default_rng(n)
+    rec = bodies_to_state(np.concatenate([rng.normal(size=(n, 4)), rng.uniform(1, 2, (n, 1))], 1))
+    ev, _ = gpu.create_evolving_state_records(rec)
+    assert np.array_equal(gpu.read_evolving_state_records(ev)[0].view(np.uint32),
+                          rec.view(np.uint32))
+    again = rng.normal(size=(n, 5))
+    again[:, 4] = 1.0
+    gpu.write_evolving_state(ev, again)
+    assert np.array_equal(gpu.read_evolving_state_records(ev)[0].view(np.uint32),
+                          bodies_to_state(again).view(np.uint32))
