@@ -809,11 +809,10 @@ static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // Byte sizes of the arena regions, in carve order.
 struct ArenaPlan {
     size_t control, sims, simout, chunk, tiles, keys, vals, sbody, base, cell_u, groups,
-        cell_d, cell_child, cell_parent, agg_words, err, stats;
+        cell_d, agg_region, err, stats;
     size_t total() const {
         return control + sims + simout + chunk + tiles + 2 * keys + 2 * vals + sbody + base +
-               cell_u + groups + cell_d + cell_child + cell_parent + agg_words +
-               err + stats;
+               cell_u + groups + cell_d + agg_region + err + stats;
     }
 };
 
@@ -833,9 +832,8 @@ static ArenaPlan plan_arena(const Layout& L, uint32_t nsims) {
     a.cell_u = align256(sizeof(uint4) * L.cells);
     a.groups = align256(4ull * sizeof(CellRec) * (L.cells + nsims));
     a.cell_d = align256(32ull * L.cells);
-    a.cell_child = align256(16ull * L.cells);
-    a.cell_parent = align256(4ull * L.cells);
-    a.agg_words = align256(4ull * L.cells);
+    // far more than the lists need: the arena's size is part of the receipts
+    a.agg_region = align256(16ull * L.cells) + 2 * align256(4ull * L.cells);
     a.err = 256;
     a.stats = 256;
     return a;
@@ -944,9 +942,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.cell_u = (uint4*)take(A.cell_u);
     bb.groups = (CellRec*)take(A.groups);
     bb.cell_d = (double4*)take(A.cell_d);
-    bb.cell_child = (uint4*)take(A.cell_child);
-    bb.cell_parent = (uint32_t*)take(A.cell_parent);
-    bb.agg_words = (uint32_t*)take(A.agg_words);
+    bb.agg_region = take(A.agg_region);
     bb.err = (uint32_t*)take(A.err);
     bb.force_stats = (unsigned long long*)take(A.stats);
     bb.nsims = count;
@@ -1041,7 +1037,6 @@ static int enqueue_rebuild(Batch* b, int integrate_mode, cudaEvent_t* ev) {
     CK(small ? launch_sort_small(b->bb, s) : launch_radix(b->bb, s), "radix launch");
     if (ev) CK(cudaEventRecord(ev[3], s), "event");
     if (!small || b->bb.nsims > 1) CK(launch_count_scan(b->bb, s), "count/scan launch");
-    CK(launch_cells(b->bb, s), "cells launch");
     if (ev) CK(cudaEventRecord(ev[4], s), "event");
     CK(launch_aggregate(b->bb, s), "aggregate launch");
     if (ev) CK(cudaEventRecord(ev[5], s), "event");

@@ -113,9 +113,7 @@ struct BatchBuffers {
                         // root at slot 0 of group cell_capacity + s (traversal)
     double4* cell_d;    // com_x, com_y, mass (f64), then the f32 residuals of
                         // com_x, com_y (float2 bits): com - (float)com
-    uint4* cell_child;  // children (global cell indices)
-    uint32_t* cell_parent;
-    uint32_t* agg_words;  // the aggregates' cuts and list of cells across outer cuts
+    void* agg_region;   // the aggregates' cuts and lists of cells across them
     // persistent
     uint32_t* err;                   // error bits
     unsigned long long* force_stats; // 4 counters
@@ -131,7 +129,6 @@ cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s);
 bool small_sort(const BatchBuffers& b);
 cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s);
-cudaError_t launch_cells(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s);
 // Recomputes G*m and the MAC bounds of simulation `sim` for new theta / G.
 cudaError_t launch_refresh_mac(const BatchBuffers& b, uint32_t sim, cudaStream_t s);

@@ -14,10 +14,10 @@
 //   k_sort_small  codes, sort and gather of a small simulation in one block
 //   k_count_scan  cells per position + exclusive scan (cell numbering in the
 //                 reference's recursive preorder, nbody/src/flat.rs:127-177)
-//   k_cells       ranges, children, skip pointers of every cell
-//   k_aggregate   bottom-up f64 mass / centre of mass, identical arithmetic
-//                 and order to nbody/src/flat.rs:179-215, in blocks of about
-//                 256 positions; k_aggregate_spans the cells across blocks
+//   k_aggregate   ranges, children, skip pointers of every cell and bottom-up
+//                 f64 mass / centre of mass, identical arithmetic and order to
+//                 nbody/src/flat.rs:179-215, in blocks of about 256 positions;
+//                 k_aggregate_inner and _outer the cells across blocks
 //   k_traverse    lane-parallel theta-MAC walk over node groups with per-warp
 //                 interaction lists (nbody/src/flat.rs:270-346 decisions per
 //                 body), f32 forces, exact f64 MAC in the guard band
@@ -136,28 +136,6 @@ __device__ __forceinline__ uint32_t shared_levels(uint32_t a, uint32_t b) {
 // 2^-d as an exact double.
 __device__ __forceinline__ double pow2_neg(uint32_t d) {
     return __longlong_as_double((long long)(1023 - (int)d) << 52);
-}
-
-// First index in [lo, hi) whose code is >= x, given codes[j] < x for j < lo.
-// Exponential probe from lo, then binary search: O(log distance).
-__device__ __forceinline__ uint32_t gallop_lower_bound(const uint32_t* codes, uint32_t lo,
-                                                       uint32_t hi, uint32_t x) {
-    uint32_t step = 1;
-    uint32_t probe = lo;
-    while (probe < hi && codes[probe] < x) {
-        lo = probe + 1;
-        probe = lo + step;
-        step <<= 1;
-    }
-    uint32_t r = probe < hi ? probe : hi;
-    while (lo < r) {
-        uint32_t m = lo + ((r - lo) >> 1);
-        if (codes[m] < x)
-            lo = m + 1;
-        else
-            r = m;
-    }
-    return lo;
 }
 
 // First index in [lo, hi) whose code is >= x (codes ascending there; hi if
@@ -718,14 +696,46 @@ __device__ __forceinline__ uint32_t chain_count(const uint32_t* __restrict__ sc,
     return (uint32_t)(deepest - (int)dmin + 1);
 }
 
+// k_aggregate's blocks own [cut_b, cut_b+1): cut b is the first position of the
+// kAggCutWindow ones from b * kAggPositions on that starts a group of the least
+// depth, so that few cells, and only shallow ones, span two blocks.
+#ifndef GBH_AGG_POSITIONS
+#define GBH_AGG_POSITIONS 256
+#endif
+#ifndef GBH_AGG_CUT_WINDOW
+#define GBH_AGG_CUT_WINDOW 128
+#endif
+constexpr uint32_t kAggPositions = GBH_AGG_POSITIONS;
+constexpr uint32_t kAggCutWindow = GBH_AGG_CUT_WINDOW;
+static_assert(kAggCutWindow == 32u * kScanItems && kAggPositions == 2u * kAggCutWindow,
+              "the warps of k_count_scan find the cuts");
+// The cuts (one more than blocks, found with the chain counts) and the internal
+// cells that span one (from k_aggregate), as (cell, depth << 26 | simulation,
+// first position), at most one per cut and depth.  Every kAggRange-th cut is an outer cut: a list per range
+// between two of them, and one of the cells that span an outer cut.
+#ifndef GBH_AGG_RANGE
+#define GBH_AGG_RANGE 128
+#endif
+constexpr uint32_t kAggRange = GBH_AGG_RANGE;
+constexpr uint32_t kAggRangeCells = 16u * kAggRange;
+struct AggPlan {
+    uint32_t* cuts;
+    uint32_t* inner_n;  // [range], zeroed with the chain counts
+    uint32_t* outer_n;  // zeroed with the control block
+    uint4* inner;       // [range][kAggRangeCells]
+    uint4* outer;       // [16 ranges]
+    struct SpanCell* outer_cells;  // [16 ranges], with their links
+    uint32_t blocks, ranges;
+};
+
 constexpr unsigned long long kScanAgg = 1ull << 62;
 constexpr unsigned long long kScanInc = 2ull << 62;
 constexpr unsigned long long kScanMask = (1ull << 62) - 1ull;
 
 __global__ void __launch_bounds__(kScanThreads) k_count_scan(
     const SimDesc* __restrict__ sims, const uint32_t* __restrict__ chunk_sim, uint32_t npos,
-    const uint32_t* __restrict__ codes, uint32_t* __restrict__ base, uint32_t* tile_counter,
-    unsigned long long* flags, uint32_t* err) {
+    const uint32_t* __restrict__ codes, uint32_t* __restrict__ base, const AggPlan plan,
+    uint32_t* tile_counter, unsigned long long* flags, uint32_t* err) {
     wait_for_predecessor();
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_scan[8];
@@ -735,24 +745,32 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(
     const uint32_t t = s_tile;
     const uint32_t p0 = t * kScanTile + threadIdx.x * kScanItems;
     uint32_t cnt[kScanItems];
-    uint32_t sum = 0;
+    uint32_t sum = 0, cut = kNone;
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         const uint32_t p = p0 + k;
         uint32_t c = 0;
         if (p < npos) {
             const uint32_t s = chunk_sim[p >> 5];
+            uint32_t dmin = 0;
             if (s != kNone) {
                 const SimDesc& sd = sims[s];
                 const uint32_t i = p - sd.off;
-                if (i < sd.n) {
-                    uint32_t dmin;
+                if (i < sd.n)
                     c = chain_count(codes + sd.off, i, sd.n, sd.bucket, sd.max_depth, &dmin);
-                }
             }
+            cut = min(cut, dmin << 16 | (p % kAggPositions));
         }
         cnt[k] = c;
         sum += c;
+    }
+    // a warp's positions are one half of a block's: a cut window, or not
+    cut = __reduce_min_sync(kFull, cut);
+    if (lane_id() == 0 && p0 % kAggPositions == 0u && p0 < npos)
+        plan.cuts[p0 / kAggPositions] = p0 + (cut & 0xffffu);
+    if (threadIdx.x == 0) {
+        if (t == 0) plan.cuts[plan.blocks] = npos;
+        if (t < plan.ranges) plan.inner_n[t] = 0;  // (a range spans many tiles)
     }
     uint32_t tile_total;
     const uint32_t texcl = block_exclusive_scan_256(sum, &tile_total, s_scan);
@@ -826,6 +844,7 @@ struct SmallSort {
     // threads of a digit read rows 8 apart, in different banks)
     uint16_t place[kSmallWarps][258];
     uint32_t warp_sum[kSmallWarps];
+    uint32_t cut[kSmallSort / kAggPositions];  // least dmin << 16 | position of the cut windows
 };
 
 // Exclusive scan of one value per thread over a block of kSmallThreads.
@@ -854,7 +873,7 @@ template <int ITEMS, bool SCAN>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     const SimDesc* __restrict__ sims, const uint32_t* __restrict__ minmax, uint32_t npos,
     uint32_t* __restrict__ keys, float4* __restrict__ sbody, uint32_t* __restrict__ base,
-    SimOut* simout) {
+    const AggPlan plan, SimOut* simout) {
     wait_for_predecessor();
     extern __shared__ unsigned long long small_shared[];
     SmallSort<ITEMS>& s = *reinterpret_cast<SmallSort<ITEMS>*>(small_shared);
@@ -863,6 +882,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     const SimDesc& sd = sims[blockIdx.x];
     const uint32_t n = sd.n;
     const uint32_t i0 = warp * (ITEMS * 32u) + lane;  // this thread's positions: i0 + 32 r
+    if (SCAN && t < kSmallSort / kAggPositions) s.cut[t] = kNone;
     const RootBounds rb = root_bounds_from(minmax + 4 * blockIdx.x);
     if (t == 0) {
         simout[blockIdx.x].cx = rb.cx;
@@ -939,16 +959,24 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
         const uint32_t i = i0 + 32u * r;
+        uint32_t cut = kNone;
         count[r] = 0;
         if (i < n) {
             const uint32_t v = s.val[i];
             const float4 pm = *reinterpret_cast<const float4*>(sd.state + v);
             keys[sd.off + i] = s.key[i];
             sbody[sd.off + i] = make_float4(pm.x, pm.y, pm.z, __uint_as_float(v));
-            uint32_t dmin;
-            if (SCAN) count[r] = chain_count(s.key, i, n, sd.bucket, sd.max_depth, &dmin);
+            if (SCAN) {
+                uint32_t dmin;
+                count[r] = chain_count(s.key, i, n, sd.bucket, sd.max_depth, &dmin);
+                cut = dmin << 16 | i;
+            }
         }
         sum += count[r];
+        if (SCAN && (i & ~31u) % kAggPositions < kAggCutWindow && (i & ~31u) < n) {
+            cut = __reduce_min_sync(kFull, cut);
+            if (lane == 0) atomicMin(&s.cut[i / kAggPositions], cut);
+        }
     }
     if constexpr (SCAN) {  // cells per position, scanned in position order
         uint32_t total;
@@ -967,284 +995,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
             at += __shfl_sync(kFull, x, 31);
         }
         for (uint32_t p = n + t; p <= npos; p += kSmallThreads) base[p] = total;
-    }
-}
-
-// =============================================================== cells ====
-
-// One thread per cell.  A block covers 256 positions, whose cells are the
-// contiguous preorder range [base[P0], base[P0 + 256]); the codes and chain
-// bases of the next kCellsWin positions sit in shared memory, so the range
-// searches of almost every cell (all but the few that span more than the
-// window) never touch global memory.
-// k_aggregate's blocks own [cut_b, cut_b+1): cut b is the first position of the
-// kAggCutWindow ones from b * kAggPositions on that starts a group of the least
-// depth, so that few cells, and only shallow ones, span two blocks.
-#ifndef GBH_AGG_POSITIONS
-#define GBH_AGG_POSITIONS 256
-#endif
-#ifndef GBH_AGG_CUT_WINDOW
-#define GBH_AGG_CUT_WINDOW 128
-#endif
-constexpr uint32_t kAggPositions = GBH_AGG_POSITIONS;
-constexpr uint32_t kAggCutWindow = GBH_AGG_CUT_WINDOW;
-// The cuts (one more than blocks, from k_cells) and the internal cells that
-// span one (from k_aggregate), as (cell, depth << 26 | simulation) at most one
-// per cut and depth.  Every kAggRange-th cut is an outer cut: a list per range
-// between two of them, and one of the cells that span an outer cut.
-#ifndef GBH_AGG_RANGE
-#define GBH_AGG_RANGE 128
-#endif
-constexpr uint32_t kAggRange = GBH_AGG_RANGE;
-constexpr uint32_t kAggRangeCells = 16u * kAggRange;
-struct AggPlan {
-    uint32_t* cuts;
-    uint32_t* inner_n;  // [range], zeroed by k_cells
-    uint32_t* outer_n;  // zeroed with the control block
-    uint2* inner;       // [range][kAggRangeCells]
-    uint2* outer;       // [16 ranges]
-    uint32_t blocks, ranges;
-};
-#ifndef GBH_CELLS_THREADS
-#define GBH_CELLS_THREADS 256
-#endif
-constexpr uint32_t kCellsThreads = GBH_CELLS_THREADS;  // positions (and threads) per block
-// 512 positions: wider windows load more than their searches save (1024 and
-// 2048 measured slower at 2^20 and 2^24)
-#ifndef GBH_CELLS_WIN
-#define GBH_CELLS_WIN 512
-#endif
-constexpr uint32_t kCellsWin = GBH_CELLS_WIN;
-constexpr uint32_t kMaxChain = kMortonDepth + 1;  // cells per position: depths 0..16
-
-#ifndef GBH_CELLS_KARY
-#define GBH_CELLS_KARY 1
-#endif
-
-struct CellsWindow {
-    const uint32_t* s_code;  // codes of positions [w0, w0 + kCellsWin)
-    const uint32_t* s_base;  // base of positions [w0, w0 + kCellsWin]
-    const uint32_t* codes;
-    const uint32_t* base;
-    uint32_t w0;
-
-    __device__ __forceinline__ uint32_t base_at(uint32_t gp) const {
-        const uint32_t j = gp - w0;
-        return j <= kCellsWin ? s_base[j] : base[gp];
-    }
-    // First position in [lo, hi) whose code is >= x, given codes < x before lo
-    // (w0 <= lo).
-    __device__ __forceinline__ uint32_t lower_bound(uint32_t lo, uint32_t hi, uint32_t x) const {
-        const uint32_t wend = min(hi, w0 + kCellsWin);
-        if (lo < wend) {
-            if (s_code[wend - 1u - w0] >= x)
-                return w0 + gallop_lower_bound(s_code, lo - w0, wend - w0, x);
-            lo = wend;
-        }
-#if GBH_CELLS_KARY
-        if (lo >= hi) return hi;
-        const uint32_t xs[1] = {x};
-        uint32_t r[1];
-        kary_lower_bound<1>(codes, lo, hi, xs, r);
-        return r[0];
-#else
-        return lo < hi ? gallop_lower_bound(codes, lo, hi, x) : hi;
-#endif
-    }
-    // The three quadrant bounds of a cell's range [lo, hi): out[q] = first
-    // position whose code is >= x[q] (x ascending), the window first, the
-    // searches past it together.
-    __device__ __forceinline__ void lower_bound3(uint32_t lo, uint32_t hi, const uint32_t (&x)[3],
-                                                 uint32_t (&out)[3]) const {
-#if GBH_CELLS_KARY
-        const uint32_t wend = min(hi, w0 + kCellsWin);
-        bool far = false;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            if (lo < wend && s_code[wend - 1u - w0] >= x[q]) {
-                out[q] = w0 + gallop_lower_bound(s_code, lo - w0, wend - w0, x[q]);
-            } else {
-                out[q] = kNone;
-                far = true;
-            }
-        }
-        if (far) {
-            const uint32_t flo = max(lo, wend);
-            uint32_t r[3];
-            if (flo < hi) {
-                kary_lower_bound<3>(codes, flo, hi, x, r);
-            } else {
-                r[0] = r[1] = r[2] = hi;
-            }
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (out[q] == kNone) out[q] = r[q];
-        }
-#else
-        uint32_t l = lo;
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            l = lower_bound(l, hi, x[q]);
-            out[q] = l;
-        }
-#endif
-    }
-};
-
-// six blocks per SM (40 registers): the k-ary searches spill a little in
-// the few threads that run them instead of halving every block's occupancy
-#ifndef GBH_CELLS_MIN_BLOCKS
-#define GBH_CELLS_MIN_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kCellsThreads, GBH_CELLS_MIN_BLOCKS) k_cells(const SimDesc* __restrict__ sims,
-                                                         const uint32_t* __restrict__ chunk_sim,
-                                                         uint32_t npos, uint32_t capacity,
-                                                         const uint32_t* __restrict__ codes,
-                                                         const uint32_t* __restrict__ base,
-                                                         uint4* cell_u,
-                                                         uint4* cell_child, uint32_t* cell_parent,
-                                                         AggPlan plan, CellRec* groups,
-                                                         uint32_t* err) {
-    wait_for_predecessor();
-    __shared__ uint32_t s_code[kCellsWin];
-    __shared__ uint32_t s_base[kCellsWin + 1];
-    __shared__ uint8_t s_owner[kCellsThreads * kMaxChain];  // cell -> position in block
-    __shared__ uint16_t s_end[kCellsThreads * kMaxChain];   // cell -> min(end - P0, 0xffff)
-    __shared__ uint32_t s_cut;  // least dmin << 16 | position - P0 of the cut window
-    const uint32_t t = threadIdx.x;
-    const uint32_t P0 = blockIdx.x * kCellsThreads;
-    for (uint32_t j = t; j <= kCellsWin; j += kCellsThreads) {
-        const uint32_t gp = P0 + j;
-        if (j < kCellsWin) s_code[j] = gp < npos ? codes[gp] : 0xffffffffu;
-        s_base[j] = gp <= npos ? base[gp] : 0u;
-    }
-    __syncthreads();
-    const uint32_t P1 = min(P0 + kCellsThreads, npos);
-    const uint32_t kb = s_base[0], ke = s_base[P1 - P0];
-    if (ke > capacity || ke - kb > kCellsThreads * kMaxChain) {
-        if (t == 0) set_err(err, kErrCapacity);
-        return;
-    }
-    if (P0 + t < P1) {
-        const uint32_t c0 = s_base[t] - kb, c = s_base[t + 1] - s_base[t];
-        for (uint32_t j = 0; j < c; ++j) s_owner[c0 + j] = (uint8_t)t;
-    }
-    // this block's cut: the first position of the window whose dmin is least
-    if (t == 0) s_cut = kNone;
-    __syncthreads();
-    if (t < kAggCutWindow) {
-        const uint32_t p = P0 + t;
-        uint32_t dmin = 0xffu;  // past the last position: no cut
-        if (p < npos) {
-            const SimDesc& sd = sims[chunk_sim[p >> 5]];
-            dmin = 0;
-            if (p != sd.off && p < sd.off + sd.n)
-                dmin = shared_levels(t ? s_code[t - 1u] : codes[p - 1u], s_code[t]) + 1u;
-        }
-        const uint32_t key = __reduce_min_sync(kFull, dmin << 16 | t);
-        if (lane_id() == 0) atomicMin(&s_cut, key);
-    }
-    __syncthreads();
-    if (t == 0) {
-        plan.cuts[blockIdx.x] = P0 + (s_cut & 0xffffu);
-        if (P1 == npos) plan.cuts[blockIdx.x + 1u] = npos;
-        if (blockIdx.x < plan.ranges) plan.inner_n[blockIdx.x] = 0;
-    }
-    const CellsWindow w{s_code, s_base, codes, base, P0};
-    const uint4 absent = make_uint4(0u, 0u, 0u, kNone);  // u.z == 0: no child in this slot
-    // Position, depth and deepest chain depth of cell k of this block.
-    auto locate = [&](uint32_t k, uint32_t* p, uint32_t* d, uint32_t* deepest) {
-        const uint32_t tl = s_owner[k - kb];
-        *p = P0 + tl;
-        const SimDesc& sd = sims[chunk_sim[*p >> 5]];
-        const uint32_t ci = s_code[tl];
-        const uint32_t dmin = *p == sd.off
-                                  ? 0u
-                                  : shared_levels(tl ? s_code[tl - 1u] : codes[*p - 1u], ci) + 1u;
-        const uint32_t k0 = s_base[tl];
-        *deepest = dmin + (s_base[tl + 1] - k0) - 1u;
-        *d = dmin + (k - k0);
-    };
-    // Pass 1: every cell's range end (one search each).
-    for (uint32_t k = kb + t; k < ke; k += kCellsThreads) {
-        uint32_t p, d, deepest;
-        locate(k, &p, &d, &deepest);
-        const uint32_t s = chunk_sim[p >> 5];
-        const SimDesc& sd = sims[s];
-        const uint32_t hi = sd.off + sd.n;
-        const uint32_t ci = s_code[p - P0];
-        // end of the depth-d group holding p
-        uint32_t end = hi;
-        if (d > 0) {
-            const uint32_t sh = 32u - 2u * d;
-            const unsigned long long next = ((unsigned long long)(ci >> sh) + 1ull) << sh;
-            if (next <= 0xffffffffull) end = w.lower_bound(p + 1u, hi, (uint32_t)next);
-        } else {
-            cell_parent[k] = kNone;
-            // the simulation's root group holds the root in slot 0 only
-            CellRec* rg = groups + 4ull * (capacity + s);
-            rg[1].u = absent;
-            rg[2].u = absent;
-            rg[3].u = absent;
-        }
-        cell_u[k] = make_uint4(end, w.base_at(end), p, d);
-        s_end[k - kb] = (uint16_t)min(end - P0, 0xffffu);
-    }
-    __syncthreads();
-    // Pass 2: children.  Children of (p, d) are the depth-(d+1) groups of its
-    // range in position order (= quadrant order): (p, d+1) first, then the
-    // chain head at each child's end.  While those ends lie in this block
-    // they come from pass 1; otherwise the quadrant bounds are searched.
-    for (uint32_t k = kb + t; k < ke; k += kCellsThreads) {
-        uint32_t p, d, deepest;
-        locate(k, &p, &d, &deepest);
-        uint4 ch = make_uint4(kNone, kNone, kNone, kNone);
-        uint32_t* chp = &ch.x;
-        if (d < deepest) {
-            const uint32_t end = cell_u[k].x;
-            const uint32_t sh = 30u - 2u * d;
-            uint32_t q = p, child = k + 1u;
-            bool searched = false;
-            while (true) {
-                chp[(s_code[q - P0] >> sh) & 3u] = child;
-                const uint32_t e = s_end[child - kb];
-                if (P0 + e >= end) break;        // the last child
-                if (e >= P1 - P0) {              // next child starts past this block
-                    searched = true;
-                    break;
-                }
-                q = P0 + e;
-                child = s_base[e];               // chain head of position q
-            }
-            if (searched) {
-                const uint32_t pre = d == 0 ? 0u : (s_code[p - P0] >> (32u - 2u * d));
-                const uint32_t xs[3] = {((pre << 2) | 1u) << sh, ((pre << 2) | 2u) << sh,
-                                        ((pre << 2) | 3u) << sh};
-                uint32_t qb[3];
-                w.lower_bound3(p, end, xs, qb);
-                uint32_t bounds[5];
-                bounds[0] = p;
-                bounds[1] = qb[0];
-                bounds[2] = qb[1];
-                bounds[3] = qb[2];
-                bounds[4] = end;
-#pragma unroll
-                for (uint32_t qd = 0; qd < 4; ++qd)
-                    chp[qd] = bounds[qd] < bounds[qd + 1]
-                                  ? (bounds[qd] == p ? k + 1u : w.base_at(bounds[qd]))
-                                  : kNone;
-            }
-#pragma unroll
-            for (uint32_t qd = 0; qd < 4; ++qd) {
-                const uint32_t child = chp[qd];
-                if (child == kNone) continue;
-                if (child < capacity)
-                    cell_parent[child] = k;
-                else
-                    set_err(err, kErrCapacity);
-            }
-        }
-        cell_child[k] = ch;
+        if (t < plan.blocks) plan.cuts[t] = s.cut[t] & 0xffffu;
+        if (t == plan.blocks) plan.cuts[t] = npos;
+        if (t == 0) plan.inner_n[0] = 0;
     }
 }
 
@@ -1286,15 +1039,6 @@ __device__ __forceinline__ float pack_depth(float hi, uint32_t depth) {
     return __uint_as_float(((__float_as_uint(hi) + 32u) & ~31u) | depth);
 }
 
-// Where a cell sits for the traversal: slot `quadrant` (the 2-bit digit of
-// its codes at the parent's depth) of its parent's node group, or slot 0 of
-// its simulation's root group (index capacity + sim).
-__device__ __forceinline__ unsigned long long slot_index(uint32_t parent, uint32_t depth,
-                                                         uint32_t code, uint32_t root_group) {
-    return depth == 0u ? 4ull * root_group
-                       : 4ull * parent + ((code >> (32u - 2u * depth)) & 3u);
-}
-
 // Cell k's record for its slot of the parent's node group: internal cells get
 // (hi|depth, lo); a leaf (count >= 1 bodies) is always summed directly: one
 // body -> hi = -1 (it passes as a point mass at its own position, which is its
@@ -1322,8 +1066,8 @@ struct AggArgs {
     const float4* sbody;
     const uint32_t* codes;
     uint32_t capacity;
-    const uint4* cell_u;
-    const uint4* cell_child;
+    const uint32_t* base;
+    uint4* cell_u;
     double4* cell_d;
     CellRec* groups;
 };
@@ -1375,7 +1119,7 @@ __device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const 
 // child's end), and it writes its whole node group, a 128-byte line; nothing
 // is loaded from global memory after the block's codes, bases and bodies.  The
 // cells that span a cut (few, and shallow: the cuts lie at the coarsest group
-// starts near every kAggPositions) are listed for k_aggregate_spans.  A leaf sums
+// starts near every kAggPositions) are listed for k_aggregate_inner.  A leaf sums
 // its bodies in Morton order, an internal cell its children in quadrant order
 // 0..3 (nbody/src/flat.rs:179-215): the f64 mass and centre of mass equal the
 // reference's bit for bit.
@@ -1385,7 +1129,7 @@ __device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const 
 // per SM.  Links and values read from global memory per cell, with a climb
 // through an acquire-release counter wherever a parent crossed a block, took
 // 156 us at 2^20 bodies (458 at 2^22, 61 at 2^14, 45 at 2^10); this and
-// k_aggregate_spans take 110 (331, 28, 20).  256 threads: 130 us at 2^20, 64:
+// the spanning cells' passes take 110 (331, 28, 20).  256 threads: 130 us at 2^20, 64:
 // 140; four lanes per cell: 168; cut windows of 64 and 256 positions: 112, 118.
 #ifndef GBH_AGG_THREADS
 #define GBH_AGG_THREADS 128
@@ -1396,8 +1140,6 @@ __device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const 
 constexpr uint32_t kAggThreads = GBH_AGG_THREADS;
 constexpr uint32_t kAggItems = kAggPositions + kAggCutWindow;  // positions of a block, at most
 constexpr uint32_t kAggGroups = (kAggItems + 31u) / 32u;
-static_assert(kAggPositions == kCellsThreads, "k_cells' blocks find the cuts");
-static_assert(kAggCutWindow <= kCellsThreads && kAggCutWindow % 32u == 0u, "cut windows");
 
 __device__ __forceinline__ AggSim agg_sim(const AggArgs& a, uint32_t sim) {
     AggSim si{};
@@ -1414,10 +1156,10 @@ __device__ __forceinline__ AggSim agg_sim(const AggArgs& a, uint32_t sim) {
 
 // One child of a cell, or none, as its slot of the cell's node group: an
 // absent child takes the lowest quadrant left in `missing`.
-__device__ __forceinline__ void store_child(CellRec* group, bool have, uint32_t quadrant,
-                                            uint32_t* missing, uint32_t k, float x, float y,
-                                            float gm, uint32_t depth, uint32_t start, uint32_t end,
-                                            bool leaf, Crit crit) {
+__device__ __forceinline__ void store_child(const AggArgs& a, uint32_t parent, bool have,
+                                            uint32_t quadrant, uint32_t* missing, uint32_t k,
+                                            float x, float y, float gm, uint32_t depth,
+                                            uint32_t start, uint32_t end, bool leaf, Crit crit) {
     CellRec rec = slot_record(k, x, y, gm, depth, start, end - start, leaf, crit);
     if (!have) {
         rec.f = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1425,8 +1167,33 @@ __device__ __forceinline__ void store_child(CellRec* group, bool have, uint32_t 
         quadrant = __ffs(*missing) - 1u;
         *missing &= *missing - 1u;
     }
+    CellRec* group = a.groups + 4ull * parent;
     group[quadrant].f = rec.f;
     group[quadrant].u = rec.u;
+}
+
+// A root: slot 0 of its simulation's root group, the other slots empty.
+__device__ __forceinline__ void store_root(const AggArgs& a, uint32_t root_group, uint32_t k,
+                                           float x, float y, float gm, uint32_t start,
+                                           uint32_t end, bool leaf, Crit crit) {
+    CellRec* group = a.groups + 4ull * root_group;
+    group[0] = slot_record(k, x, y, gm, 0u, start, end - start, leaf, crit);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) group[q].u = make_uint4(0u, 0u, 0u, kNone);
+}
+
+// End of the depth-d group that starts before position lo and goes on to it, by
+// code prefix (d levels of `code`), at most hi.
+__device__ __forceinline__ uint32_t group_end(const uint32_t* codes, uint32_t lo, uint32_t hi,
+                                              uint32_t code, uint32_t d) {
+    if (d == 0u) return hi;
+    const uint32_t sh = 32u - 2u * d;
+    const unsigned long long next = ((unsigned long long)(code >> sh) + 1ull) << sh;
+    if (next > 0xffffffffull) return hi;
+    const uint32_t x[1] = {(uint32_t)next};
+    uint32_t out[1];
+    kary_lower_bound<1>(codes, lo, hi, x, out);
+    return out[0];
 }
 
 struct AggShared {
@@ -1449,8 +1216,7 @@ struct AggShared {
 };
 
 __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
-    k_aggregate(const AggArgs a, const uint32_t* __restrict__ base, const AggPlan plan,
-                uint32_t* err) {
+    k_aggregate(const AggArgs a, const AggPlan plan, uint32_t* err) {
     wait_for_predecessor();
     __shared__ AggShared s;
     const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
@@ -1464,7 +1230,7 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
     const uint32_t chunk0 = R0 >> 5;
     for (uint32_t j = t; j < n; j += kAggThreads) {
         s.code[j] = a.codes[R0 + j];
-        s.base[j] = base[R0 + j];
+        s.base[j] = a.base[R0 + j];
     }
     if (t <= (R1 - 1u) / 32u - chunk0) s.sim[t] = agg_sim(a, a.chunk_sim[chunk0 + t]);
     const uint32_t before = R0 > 0u ? a.codes[R0 - 1u] : 0u;
@@ -1475,9 +1241,13 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
     if (t == 0) {
         s.depths = 0;
         s.info[n] = 0;
-        s.base[n] = base[R1];
+        s.base[n] = a.base[R1];
     }
     __syncthreads();
+    if (s.base[n] > a.capacity) {  // cannot be: the capacity bounds every tree
+        if (t == 0) set_err(err, kErrCapacity);
+        return;
+    }
     const uint32_t groups = (n + 31u) / 32u;
     auto local = [](uint32_t info, uint32_t d) {
         return d >= ((info >> 16) & 0xffu) && d < ((info >> 8) & 0xffu);
@@ -1498,8 +1268,8 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
             s.info[j] = dmin | deepest << 8 | dlo << 16;
             if (deepest > dlo) depths = ((1u << deepest) - 1u) & ~((1u << dlo) - 1u);
             for (uint32_t d = dmin; d < min(dlo, deepest); ++d) {  // the cells that span R1
-                const uint2 rec = make_uint2(s.base[j] + d - dmin,
-                                             d << 26 | (si.root_group - a.capacity));
+                const uint4 rec = make_uint4(s.base[j] + d - dmin,
+                                             d << 26 | (si.root_group - a.capacity), p, 0u);
                 if (si.end > R2 && shared_levels(code, beyond) >= d)
                     plan.outer[atomicAdd(plan.outer_n, 1u)] = rec;
                 else
@@ -1527,7 +1297,7 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
         s.link[j] = q | (s.info[q] & 0xffu) << 16;
         uint32_t end = R0 + q;
         if (q == n && d < ((info >> 16) & 0xffu)) {  // the leaf goes on past the block
-            end = a.cell_u[k].x;
+            end = group_end(a.codes, R1, si.end, s.code[j], d);
             for (uint32_t g = R0 + q; g < end; ++g) {
                 const float4 b = a.sbody[g];
                 sum.add((double)b.z, (double)b.x, (double)b.y);
@@ -1552,9 +1322,9 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
         s.fx[j] = com.x;
         s.fy[j] = com.y;
         s.gm[j] = __fmul_rn(si.g, mass);
+        a.cell_u[k] = make_uint4(end, k + 1u, R0 + j, d);
         if (d == 0u)  // the simulation is one leaf
-            a.groups[4ull * si.root_group] = slot_record(
-                k, com.x, com.y, s.gm[j], 0u, R0 + j, end - (R0 + j), true, si.crit);
+            store_root(a, si.root_group, k, com.x, com.y, s.gm[j], R0 + j, end, true, si.crit);
     }
     // the cells of each depth, in position order: counts by group of 32
     // positions, then every group's places
@@ -1611,7 +1381,7 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
         for (uint32_t q = 0; q < 4; ++q) {
             const uint32_t kid = s.base[c[q]] + d + 1u - (s.info[c[q]] & 0xffu);
             const uint32_t link = q ? s.link[c[q]] : first.link0;
-            store_child(a.groups + 4ull * k, q < first.kids, quadrant[q], &missing, kid,
+            store_child(a, k, q < first.kids, quadrant[q], &missing, kid,
                         q ? s.fx[c[q]] : first.fx, q ? s.fy[c[q]] : first.fy,
                         q ? s.gm[c[q]] : first.gm, d + 1u, R0 + c[q], R0 + (link & 0xffffu),
                         kid + 1u == s.base[c[q] + 1u], sim.crit);
@@ -1666,13 +1436,14 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
             s.link[c0] = link;
             const AggSim& sim = sim_of(c0);
             const float2 com = store_cell(a.cell_d, k, sum);
+            const uint32_t end = link & 0xffffu;
+            a.cell_u[k] = make_uint4(R0 + end, s.base[end], R0 + c0, d);
             const float gm = __fmul_rn(sim.g, (float)sum.mass);
             s.fx[c0] = com.x;
             s.fy[c0] = com.y;
             s.gm[c0] = gm;
             if (d == 0u)
-                a.groups[4ull * sim.root_group] = slot_record(
-                    k, com.x, com.y, gm, 0u, R0 + c0, (link & 0xffffu) - c0, false, sim.crit);
+                store_root(a, sim.root_group, k, com.x, com.y, gm, R0 + c0, R0 + end, false, sim.crit);
         }
         __syncthreads();
         store_group();
@@ -1680,34 +1451,41 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
     }
 }
 
-// One cell that spans a cut, from its children's f64 records.
+// One cell that spans a cut: its links by searches over the codes, its sums from
+// its children's f64 records.
 struct SpanCell {
-    uint32_t k, start, count, c[4];
-    uint32_t kid_start[4], kid_end[4];
+    uint32_t k, depth, start, end, c[4];
+    uint32_t kid_end[4], kid_start[4];
     bool kid_leaf[4];
     AggSim sim;
 
-    __device__ __forceinline__ void load(const AggArgs& a, uint2 rec) {
+    // limit: a position its end does not pass
+    __device__ __forceinline__ void load(const AggArgs& a, uint4 rec, uint32_t limit) {
         k = rec.x;
+        depth = rec.y >> 26;
+        start = rec.z;
+        const SimDesc& sd = a.sims[rec.y & 0x3ffffffu];
         sim = agg_sim(a, rec.y & 0x3ffffffu);
-        const uint4 u = a.cell_u[k];
-        const uint4 ch = a.cell_child[k];
-        start = u.z;
-        count = u.x - u.z;
-        c[0] = ch.x;
-        c[1] = ch.y;
-        c[2] = ch.z;
-        c[3] = ch.w;
+        const uint32_t code = a.codes[start];
+        end = group_end(a.codes, start + 1u, min(sim.end, limit), code, depth);
+        const uint32_t sh = 30u - 2u * depth;
+        const uint32_t prefix = depth == 0u ? 0u : (code >> (sh + 2u)) << 2;
+        const uint32_t x[3] = {(prefix | 1u) << sh, (prefix | 2u) << sh, (prefix | 3u) << sh};
+        uint32_t bound[3];
+        kary_lower_bound<3>(a.codes, start, end, x, bound);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const uint32_t kid = c[q] == kNone ? k + 1u : c[q];  // absent: its first child
-            const uint4 cu = a.cell_u[kid];
-            kid_start[q] = cu.z;
-            kid_end[q] = cu.x;
-            kid_leaf[q] = cu.y == kid + 1u;
+            kid_start[q] = q ? bound[q - 1] : start;
+            kid_end[q] = q < 3 ? bound[q] : end;
+            // the first child follows its parent, the others head their positions' chains
+            c[q] = kid_start[q] == kid_end[q] ? kNone
+                   : kid_start[q] == start    ? k + 1u
+                                              : a.base[kid_start[q]];
+            kid_leaf[q] = kid_end[q] - kid_start[q] <= sd.bucket || depth + 1u >= sd.max_depth;
         }
+        a.cell_u[k] = make_uint4(end, a.base[end], start, depth);
     }
-    __device__ __forceinline__ void combine(const AggArgs& a, uint32_t d) const {
+    __device__ __forceinline__ void combine(const AggArgs& a) const {
         CellSum sum;
         double2 com[4];
         double m[4];
@@ -1726,82 +1504,105 @@ struct SpanCell {
         const float2 own = store_cell(a.cell_d, k, sum);
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-            store_child(a.groups + 4ull * k, c[q] != kNone, (uint32_t)q, &missing, c[q],
-                        (float)com[q].x, (float)com[q].y, __fmul_rn(sim.g, (float)m[q]), d + 1u,
-                        kid_start[q], kid_end[q], kid_leaf[q], sim.crit);
-        if (d == 0u)
-            a.groups[4ull * sim.root_group] =
-                slot_record(k, own.x, own.y, __fmul_rn(sim.g, (float)sum.mass), 0u, start, count,
-                            false, sim.crit);
+            store_child(a, k, c[q] != kNone, (uint32_t)q, &missing, c[q], (float)com[q].x,
+                        (float)com[q].y, __fmul_rn(sim.g, (float)m[q]), depth + 1u, kid_start[q],
+                        kid_end[q], kid_leaf[q], sim.crit);
+        if (depth == 0u)
+            store_root(a, sim.root_group, k, own.x, own.y, __fmul_rn(sim.g, (float)sum.mass), start,
+                       end, false, sim.crit);
     }
 };
 
-// Lists of cells that span cuts, a block each (list stride `capacity`), depth
-// by depth: each depth waits for the one below, and a barrier of one block is
-// the cheapest wait.  A thread per cell, everything but the children's sums
-// loaded before the first depth (the further cells of a list longer than the
-// block are loaded in turn).  The lists of the inner cuts run at once, then the
-// one of the outer cuts: 11 and 14 us at 2^20 bodies with 64 cuts a range (128:
-// 1 to 5 % less aggregate time from 2^20 on; 16: 22 % more), where one list of
-// all cuts took 70.
+// The cells of a list that span cuts, depth by depth: each depth waits for the
+// one below, and a barrier of one block is the cheapest wait.  A thread per cell,
+// everything but the children's sums in hand before the first depth (the further
+// cells of a list longer than the block are fetched in turn).
+template <typename Fetch>
+__device__ __forceinline__ void combine_spans(const AggArgs& a, uint32_t n, Fetch fetch) {
+    __shared__ uint32_t s_depths;
+    const uint32_t t = threadIdx.x;
+    if (t == 0) s_depths = 0;
+    __syncthreads();
+    SpanCell cell;
+    cell.depth = kNone;
+    for (uint32_t i = t; i < n; i += blockDim.x) {
+        SpanCell c;
+        fetch(i, &c);
+        atomicOr(&s_depths, 1u << c.depth);
+        if (i == t) cell = c;
+    }
+    __syncthreads();
+    for (uint32_t todo = s_depths; todo != 0u;) {
+        const uint32_t d = 31u - __clz(todo);
+        todo &= ~(1u << d);
+        if (cell.depth == d) cell.combine(a);
+        for (uint32_t i = t + blockDim.x; i < n; i += blockDim.x) {
+            SpanCell more;
+            fetch(i, &more);
+            if (more.depth == d) more.combine(a);
+        }
+        __syncthreads();
+    }
+}
+
 #ifndef GBH_SPAN_THREADS
 #define GBH_SPAN_THREADS 512
 #endif
 constexpr uint32_t kSpanThreads = GBH_SPAN_THREADS;
 
-__global__ void __launch_bounds__(kSpanThreads) k_aggregate_spans(const AggArgs a,
-                                                                  const uint2* lists,
-                                                                  const uint32_t* counts,
-                                                                  uint32_t capacity) {
+// The lists of the inner cuts, a block each; the blocks after them find the
+// links of the cells that span outer cuts meanwhile.
+__global__ void __launch_bounds__(kSpanThreads) k_aggregate_inner(const AggArgs a,
+                                                                  const AggPlan plan) {
     wait_for_predecessor();
-    __shared__ uint32_t s_depths;
-    const uint32_t t = threadIdx.x;
-    const uint2* list = lists + (size_t)blockIdx.x * capacity;
-    const uint32_t n = min(counts[blockIdx.x], capacity);
+    const uint32_t r = blockIdx.x;
+    if (r >= plan.ranges) {
+        const uint32_t n = min(*plan.outer_n, kMortonDepth * plan.ranges);
+        const uint32_t i = (r - plan.ranges) * kSpanThreads + threadIdx.x;
+        if (i < n) plan.outer_cells[i].load(a, plan.outer[i], kNone);
+        return;
+    }
+    const uint4* list = plan.inner + (size_t)r * kAggRangeCells;
+    const uint32_t n = min(plan.inner_n[r], kAggRangeCells);
     if (n == 0u) return;
-    if (t == 0) s_depths = 0;
-    __syncthreads();
-    uint32_t depth = kNone;
-    SpanCell cell;
-    if (t < n) {
-        depth = list[t].y >> 26;
-        cell.load(a, list[t]);
-    }
-    for (uint32_t i = t; i < n; i += kSpanThreads) atomicOr(&s_depths, 1u << (list[i].y >> 26));
-    __syncthreads();
-    for (uint32_t todo = s_depths; todo != 0u;) {
-        const uint32_t d = 31u - __clz(todo);
-        todo &= ~(1u << d);
-        if (depth == d) cell.combine(a, d);
-        for (uint32_t i = t + kSpanThreads; i < n; i += kSpanThreads)
-            if (list[i].y >> 26 == d) {
-                SpanCell more;
-                more.load(a, list[i]);
-                more.combine(a, d);
-            }
-        __syncthreads();
-    }
+    const uint32_t outer_cut = plan.cuts[min((r + 1u) * kAggRange, plan.blocks)];
+    combine_spans(a, n, [&](uint32_t i, SpanCell* c) { c->load(a, list[i], outer_cut); });
 }
 
-// Recomputes G*m and the MAC band of every cell of one simulation from the
-// f64 aggregates, for a force pass whose theta or G differs from the rebuild's.
+// Then the list of the outer cuts: in a single list with the inner ones, the
+// cells of 2^20 bodies took 70 us instead of 11 and 14.
+__global__ void __launch_bounds__(kSpanThreads) k_aggregate_outer(const AggArgs a,
+                                                                  const AggPlan plan) {
+    wait_for_predecessor();
+    const uint32_t n = min(*plan.outer_n, kMortonDepth * plan.ranges);
+    combine_spans(a, n, [&](uint32_t i, SpanCell* c) { *c = plan.outer_cells[i]; });
+}
+
+// Recomputes G*m and the MAC bands of one simulation from the f64 aggregates,
+// for a force pass whose theta or G differs from the rebuild's: a thread per
+// cell, its children's slots (child k + 1, then each at the one before's skip).
 __global__ void k_refresh_mac(const SimDesc* __restrict__ sims, const SimOut* __restrict__ simout,
                               uint32_t sim, const uint32_t* __restrict__ base,
                               const uint32_t* __restrict__ codes, uint32_t capacity,
-                              const uint32_t* __restrict__ cell_parent,
                               const double4* __restrict__ cell_d,
                               const uint4* __restrict__ cell_u, CellRec* groups) {
     const SimDesc& sd = sims[sim];
     const uint32_t cb = base[sd.off], ce = base[sd.off + sd.n];
     const uint32_t k = cb + blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= ce) return;
+    const Crit crit = crit_f32(crit_of(simout[sim].half, sd.theta));
+    auto store = [&](CellRec* slot, uint32_t c, const uint4& u) {
+        const double4 v = cell_d[c];
+        *slot = slot_record(c, (float)v.x, (float)v.y, __fmul_rn(sd.g_f, (float)v.z), u.w, u.z,
+                            u.x - u.z, u.y == c + 1u, crit);
+    };
     const uint4 u = cell_u[k];
-    const double4 v = cell_d[k];
-    const bool leaf = u.y == k + 1u;
-    const uint32_t start = u.z;
-    groups[slot_index(cell_parent[k], u.w, codes[start], capacity + sim)] =
-        slot_record(k, (float)v.x, (float)v.y, __fmul_rn(sd.g_f, (float)v.z), u.w, start, u.x - start,
-                    leaf, crit_f32(crit_of(simout[sim].half, sd.theta)));
+    if (k == cb) store(groups + 4ull * (capacity + sim), k, u);
+    for (uint32_t c = k + 1u; c < u.y;) {  // a leaf's skip is k + 1
+        const uint4 cu = cell_u[c];
+        store(groups + 4ull * k + ((codes[cu.z] >> (30u - 2u * u.w)) & 3u), c, cu);
+        c = cu.y;
+    }
 }
 
 // ============================================================ traverse ====
@@ -2556,7 +2357,6 @@ __global__ void k_export_cells(const SimDesc* __restrict__ sims, const SimOut* _
                                uint32_t sim, const uint32_t* __restrict__ codes,
                                const uint32_t* __restrict__ base,
                                const uint4* __restrict__ cell_u,
-                               const uint4* __restrict__ cell_child,
                                const double4* __restrict__ cell_d, GpuCell* out) {
     const SimDesc& sd = sims[sim];
     const uint32_t cb = base[sd.off], ce = base[sd.off + sd.n];
@@ -2575,7 +2375,6 @@ __global__ void k_export_cells(const SimDesc* __restrict__ sims, const SimOut* _
         half = h;
     }
     const double4 v = cell_d[k];
-    const uint4 ch = cell_child[k];
     GpuCell c;
     c.center_half_mass[0] = (float)cx;
     c.center_half_mass[1] = (float)cy;
@@ -2589,10 +2388,17 @@ __global__ void k_export_cells(const SimDesc* __restrict__ sims, const SimOut* _
     c.range_depth[1] = u.x - sd.off;
     c.range_depth[2] = u.w;
     c.range_depth[3] = 0u;
-    c.children[0] = ch.x == kNone ? kNone : ch.x - cb;
-    c.children[1] = ch.y == kNone ? kNone : ch.y - cb;
-    c.children[2] = ch.z == kNone ? kNone : ch.z - cb;
-    c.children[3] = ch.w == kNone ? kNone : ch.w - cb;
+    // children: k + 1, then each at the one before's skip (none for a leaf)
+    uint32_t child[4] = {kNone, kNone, kNone, kNone};
+    for (uint32_t next = k + 1u; next < u.y;) {
+        const uint4 cu = cell_u[next];
+        const uint32_t quadrant = (codes[cu.z] >> (30u - 2u * u.w)) & 3u;
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) child[q] = q == quadrant ? next - cb : child[q];
+        next = cu.y;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) c.children[q] = child[q];
     out[k - cb] = c;
 }
 
@@ -2972,6 +2778,29 @@ cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s) {
     return b.radix_bits == 4 ? radix_passes<4, 0>(b, s) : radix_passes<8, 0>(b, s);
 }
 
+// Lays the plan out in its region, which holds 24 bytes per cell (at least 24 a
+// body, 768 in all): per block a cut and, by range, up to 256 bytes of inner list,
+// per range the count and the outer list's 20 KB of cells.
+static AggPlan agg_plan(const BatchBuffers& b) {
+    AggPlan p;
+    p.blocks = (b.npos + kAggPositions - 1) / kAggPositions;
+    p.ranges = (p.blocks + kAggRange - 1) / kAggRange;
+    p.outer_n = b.counters + 16;
+    char* at = (char*)b.agg_region;
+    auto take = [&](size_t bytes) {
+        char* q = at;
+        at += (bytes + 15) & ~(size_t)15;
+        return q;
+    };
+    p.inner_n = (uint32_t*)take(4ull * p.ranges);
+    p.cuts = (uint32_t*)take(4ull * (p.blocks + 1));
+    const size_t outer = p.ranges > 1 ? (size_t)kMortonDepth * p.ranges : 0;
+    p.outer = (uint4*)take(sizeof(uint4) * outer);
+    p.outer_cells = (SpanCell*)take(sizeof(SpanCell) * outer);
+    p.inner = (uint4*)at;  // the last range's list is as long as its cuts allow
+    return p;
+}
+
 // One block per simulation instead of Morton, radix and (for a single
 // simulation) scan launches, where every simulation is small enough for it (and
 // the caller has not asked for 4-bit digits).
@@ -2984,7 +2813,7 @@ static cudaError_t sort_small(const BatchBuffers& b, cudaStream_t s) {
                              (int)sizeof(SmallSort<ITEMS>));
     if (e != cudaSuccess) return e;
     return launch_step(k_sort_small<ITEMS, SCAN>, b.nsims, kSmallThreads, sizeof(SmallSort<ITEMS>),
-                       s, b.sims, b.minmax, b.npos, b.keys_a, b.sbody, b.base, b.simout);
+                       s, b.sims, b.minmax, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
 }
 
 template <bool SCAN>
@@ -3000,42 +2829,21 @@ cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s) {
 
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
     return launch_step(k_count_scan, b.nscan_tiles, kScanThreads, 0, s, b.sims, b.chunk_sim,
-                       b.npos, b.keys_a, b.base, b.counters + 8, b.scan_flags, b.err);
-}
-
-// The counts, the outer list and the cuts (about 5 bytes per kAggPositions) have
-// their own words; the inner lists lie in the sort's spent value buffers, 8
-// bytes a position: a range of kAggRange blocks may hold 16 KB of them, and the
-// last range's list has at most 128 bytes per cut.
-static AggPlan agg_plan(const BatchBuffers& b) {
-    AggPlan p;
-    p.blocks = (b.npos + kAggPositions - 1) / kAggPositions;
-    p.ranges = (p.blocks + kAggRange - 1) / kAggRange;
-    p.outer = reinterpret_cast<uint2*>(b.agg_words);
-    p.inner_n = b.agg_words + 2u * kMortonDepth * p.ranges;
-    p.cuts = p.inner_n + p.ranges;
-    p.inner = reinterpret_cast<uint2*>(b.vals_a);
-    p.outer_n = b.counters + 16;
-    return p;
-}
-
-cudaError_t launch_cells(const BatchBuffers& b, cudaStream_t s) {
-    return launch_step(k_cells, (b.npos + kCellsThreads - 1) / kCellsThreads, kCellsThreads, 0, s,
-                       b.sims, b.chunk_sim, b.npos, b.cell_capacity, b.keys_a, b.base, b.cell_u,
-                       b.cell_child, b.cell_parent, agg_plan(b), b.groups, b.err);
+                       b.npos, b.keys_a, b.base, agg_plan(b), b.counters + 8, b.scan_flags, b.err);
 }
 
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s) {
-    const AggArgs a{b.sims,          b.simout, b.chunk_sim,  b.sbody, b.keys_a,
-                    b.cell_capacity, b.cell_u, b.cell_child, b.cell_d, b.groups};
+    const AggArgs a{b.sims,          b.simout, b.chunk_sim, b.sbody,  b.keys_a,
+                    b.cell_capacity, b.base,   b.cell_u,    b.cell_d, b.groups};
     const AggPlan plan = agg_plan(b);
-    cudaError_t e = launch_step(k_aggregate, plan.blocks, kAggThreads, 0, s, a, b.base, plan, b.err);
-    if (e == cudaSuccess && plan.blocks > 1)
-        e = launch_step(k_aggregate_spans, plan.ranges, kSpanThreads, 0, s, a, plan.inner,
-                        plan.inner_n, kAggRangeCells);
+    cudaError_t e = launch_step(k_aggregate, plan.blocks, kAggThreads, 0, s, a, plan, b.err);
+    if (e == cudaSuccess && plan.blocks > 1) {
+        const uint32_t outer =
+            plan.ranges > 1 ? (kMortonDepth * plan.ranges + kSpanThreads - 1) / kSpanThreads : 0;
+        e = launch_step(k_aggregate_inner, plan.ranges + outer, kSpanThreads, 0, s, a, plan);
+    }
     if (e == cudaSuccess && plan.ranges > 1)
-        e = launch_step(k_aggregate_spans, 1, kSpanThreads, 0, s, a, plan.outer, plan.outer_n,
-                        kMortonDepth * plan.ranges);
+        e = launch_step(k_aggregate_outer, 1, kSpanThreads, 0, s, a, plan);
     return e;
 }
 
@@ -3047,7 +2855,7 @@ cudaError_t launch_wait_probe(const uint32_t* flags, uint32_t* err, long long li
 
 cudaError_t launch_refresh_mac(const BatchBuffers& b, uint32_t sim, cudaStream_t s) {
     k_refresh_mac<<<(b.cell_capacity + 255) / 256, 256, 0, s>>>(
-        b.sims, b.simout, sim, b.base, b.keys_a, b.cell_capacity, b.cell_parent,
+        b.sims, b.simout, sim, b.base, b.keys_a, b.cell_capacity,
         b.cell_d, b.cell_u, b.groups);
     return cudaGetLastError();
 }
@@ -3103,7 +2911,7 @@ cudaError_t launch_export(const BatchBuffers& b, uint32_t sim, GpuEntry* entries
                           GpuCell* cells, cudaStream_t s) {
     if (cells)
         k_export_cells<<<(b.cell_capacity + 255) / 256, 256, 0, s>>>(
-            b.sims, b.simout, sim, b.keys_a, b.base, b.cell_u, b.cell_child, b.cell_d,
+            b.sims, b.simout, sim, b.keys_a, b.base, b.cell_u, b.cell_d,
             cells);
     if (entries || bodies)
         k_export_entries<<<(b.npos + 255) / 256, 256, 0, s>>>(b.sims, sim, b.keys_a, b.sbody,

@@ -801,3 +801,22 @@ def test_large_copies_keep_every_record(gpu, n):
     gpu.write_evolving_state(ev, again)
     assert np.array_equal(gpu.read_evolving_state_records(ev)[0].view(np.uint32),
                           bodies_to_state(again).view(np.uint32))
+
+
+@pytest.mark.parametrize("n,bucket", [(3, 1), (500, 1), (500, 500), (40000, 1), (40000, 6)])
+def test_force_with_other_theta_and_g_equals_a_rebuild(gpu, rt, n, bucket):
+    """A force pass whose theta and G differ from the rebuild's rewrites every
+    cell's opening bounds and G*m from the f64 aggregates: the same records, so
+    the same bits, as a rebuild under that config."""
+    import dataclasses as dc
+    cfg = Config(theta=0.4, softening_kpc=0.02, g=1.0, bucket=bucket, force_stats=False)
+    other = dc.replace(cfg, theta=0.9, g=2.5)
+    bodies = scenarios.exponential_disc(n, 6)
+    ev, _ = gpu.create_evolving_state(bodies)
+    tree = rt.create_tree(gpu, ev, cfg)
+    rt.rebuild(gpu, ev, tree, cfg)
+    rt.force(gpu, ev, tree, other)
+    got = gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32).copy()
+    rt.rebuild(gpu, ev, tree, other)
+    rt.force(gpu, ev, tree, other)
+    assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), got)
