@@ -954,6 +954,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     bb.cell_capacity = (uint32_t)L.cells;
     bb.radix_bits = 8;
     bb.trav_warps = 4;
+    bb.clusters = true;
     bb.normal_eps2 = normal_eps2(cfgs, count);
 
     b->h_sims.resize(count);
@@ -1165,12 +1166,17 @@ extern "C" int galaxy_bh_tree_destroy(bh_tree* tree) {
 
 // Points *tree at state st under cfg (creating the tree when null), keeping
 // its arena when that is large enough: a serving loop's stager solves each
-// newcomer's boundary on one tree instead of allocating one per request.
+// newcomer's boundary on one tree instead of allocating one per request.  Its
+// rebuilds share the GPU with the loop's rounds, so they use no cluster.
 int gbh::tree_retarget(bh_device* dev, bh_tree** tree, bh_state* st, const bh_config* cfg) {
     if (!tree) return set_error(BH_INVALID_ARG, "null argument");
-    if (!*tree) return galaxy_bh_tree_create(dev, st, cfg, tree);
-    int rc = enter(dev);
-    if (rc) return rc;
+    int rc;
+    if (!*tree) {
+        if ((rc = galaxy_bh_tree_create(dev, st, cfg, tree)) == BH_OK)
+            (*tree)->batch->bb.clusters = false;
+        return rc;
+    }
+    if ((rc = enter(dev))) return rc;
     bh_tree* t = *tree;
     if (!st) return set_error(BH_INVALID_ARG, "null argument");
     if (t->dev != dev || st->dev != dev)
@@ -1185,6 +1191,7 @@ int gbh::tree_retarget(bh_device* dev, bh_tree** tree, bh_state* st, const bh_co
         *tree = nullptr;
         return rc;
     }
+    b->bb.clusters = false;
     t->batch = b;
     t->st = st;
     return BH_OK;

@@ -20,7 +20,7 @@ constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;  // 1024-position scan tiles: a shorter per-tile chain
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // positions per scan tile
 constexpr uint32_t kMortonDepth = 16;
-constexpr uint32_t kSmallSort = 4096;  // bodies one block sorts (k_sort_small)
+constexpr uint32_t kSmallSort = 65536;  // bodies one cluster sorts (k_sort_small)
 
 // Error bits accumulated in the device error word until the host reads it.
 enum : uint32_t {
@@ -93,6 +93,7 @@ struct BatchBuffers {
     uint32_t radix_bits;   // 8 (4 passes) or 4 (8 passes); results do not depend on it
     uint32_t trav_warps;   // warps per traversal block, 2, 4 or 8; results do not depend on it
     bool normal_eps2;      // every simulation's f32 softening squared is a normal number
+    bool clusters;         // sorts may run as clusters; false beside another stream's work
     // zeroed once per rebuild (one memset): control block
     uint32_t* minmax;      // nsims * 4 (atomicMax of encoded floats; mins stored inverted)
     uint32_t* hist;        // nsims * 4 * 256

@@ -11,7 +11,8 @@
 //   k_radix_pass  one stable LSD pass (onesweep: decoupled look-back, warp
 //                 match ranking, shared-memory staged scatter); the last pass
 //                 also gathers the bodies into Morton order
-//   k_sort_small  codes, sort and gather of a small simulation in one block
+//   k_sort_small  codes, sort, gather and chain scan of a simulation of at most
+//                 65,536 bodies in one block or cluster
 //   k_count_scan  cells per position + exclusive scan (cell numbering in the
 //                 reference's recursive preorder, nbody/src/flat.rs:127-177)
 //   k_aggregate   ranges, children, skip pointers of every cell and bottom-up
@@ -44,19 +45,28 @@ constexpr unsigned kFull = 0xffffffffu;
 // Launches a kernel of the step with programmatic stream serialization, so
 // its launch overlaps the previous kernel's tail (see wait_for_predecessor).
 template <typename... KArgs, typename... Args>
-static cudaError_t launch_step(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                               cudaStream_t s, Args... args) {
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), uint32_t cluster, dim3 grid,
+                                   dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = GBH_PDL;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_step(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                               cudaStream_t s, Args... args) {
+    return launch_clusters(kernel, 1, grid, block, smem, s, args...);
 }
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
@@ -670,8 +680,9 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
 // d_min..D).  Cell (d, i) exists iff i starts a depth-d group and its parent
 // group holds more than `bucket` bodies; it is internal iff it holds more
 // than `bucket` bodies and d < max_depth (nbody/src/flat.rs:145).
-__device__ __forceinline__ uint32_t chain_count(const uint32_t* __restrict__ sc, uint32_t i,
-                                                uint32_t n, uint32_t bucket, uint32_t maxd,
+template <typename Codes>
+__device__ __forceinline__ uint32_t chain_count(const Codes sc, uint32_t i, uint32_t n,
+                                                uint32_t bucket, uint32_t maxd,
                                                 uint32_t* dmin_out) {
     const uint32_t ci = sc[i];
     const uint32_t dmin = i == 0 ? 0u : shared_levels(sc[i - 1], ci) + 1u;
@@ -822,32 +833,75 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(
 
 // ========================================================= small sort =====
 
-// A simulation of at most kSmallSort bodies in one block: Morton codes, the
-// four stable 8-bit passes in shared memory, the gather into Morton order and,
-// where the batch is that one simulation (SCAN), the chain counts and their
-// scan.  The passes of k_radix_pass cost 7 us and up each however few keys they
-// have (a launch, a load, a look-back, a store to global memory).  A warp ranks
-// its 32 ITEMS positions in order as k_radix_pass does (the lanes that share a
-// digit by one ballot per digit bit), and one block scan over (digit, warps)
-// turns the counts into places, so the permutation is the same stable one.
-// A step at 1,024 bodies 92.6 -> 70.2 us, at 4,096 121 -> 103; 512 simulations of
-// 2^10 to 2^12 in a batch 731 -> 709.  One SM's issue and load rates bound it (1.3
-// us per 1,024 keys and pass): at 16,384 keys it took 93 us against 47.
-constexpr int kSmallThreads = 1024;
-constexpr int kSmallWarps = kSmallThreads / 32;
+// A simulation of at most kSmallSort bodies in one block or one cluster of up to
+// 16: Morton codes, the four stable 8-bit passes in shared memory (a cluster's
+// blocks write one another's), the gather into Morton order and, where the batch
+// is that one simulation (SCAN), the chain counts and their scan.  Separate
+// launches cost 10 us for the codes, 7 to 10 a pass and 10 for the scan however
+// few keys they have: a launch, a chain of loads, a look-back, global stores.  A
+// warp ranks its positions in order as k_radix_pass does (the lanes that share a
+// digit by one ballot per digit bit); one block scan over (digit, blocks, warps)
+// turns the counts into places, so the permutation is the same stable one.  In a
+// cluster a block gets every block's digit counts before the scan, and an item
+// goes straight to its place in whichever block has it: two barriers a pass, the
+// first also the proof that every block has its items in registers.
+// Bound by the barriers' latency (a pass of 16 blocks of 1,024 keys takes 10,000
+// cycles: ranking 1,500, counts 2,000, the barriers 2,500 and 2,000, places 1,500)
+// and, at 4,096 keys a block, by the 8-byte remote stores (5,000 of 19,000).  512
+// threads have fewer counts to scan and fewer warps to wait for than 1,024, and
+// shorter chains than 256: 92.6, 93.6 and 92.9 us a step at 16,384 bodies, 145, 146
+// and 156 at 65,536.  Steps against separate launches: 4,096 bodies 121 -> 80 us (one
+// block of 1,024 threads: 88), 8,192 112 -> 84, 16,384 117 -> 91, 32,768 128 -> 109,
+// 65,536 154 -> 145.
+constexpr int kSmallThreads = 512;
+constexpr uint32_t kSmallBlocks = 16;  // most blocks of a cluster
+static_assert(kSmallSort == kSmallBlocks * 4096u && kSmallSort <= 65536u,
+              "body indices are kept in 16 bits");
 
-template <int ITEMS>
+template <int LOG>
 struct SmallSort {
-    uint32_t key[kSmallThreads * ITEMS];
-    uint16_t val[kSmallThreads * ITEMS];
-    // digit counts by warp, then first places (rows padded: the scan's four
+    uint64_t item[1 << LOG];  // body index << 32 | code
+    // digit counts by warp, then first places (rows padded: the scan's
     // threads of a digit read rows 8 apart, in different banks)
-    uint16_t place[kSmallWarps][258];
-    uint32_t warp_sum[kSmallWarps];
-    uint32_t cut[kSmallSort / kAggPositions];  // least dmin << 16 | position of the cut windows
+    uint16_t place[kSmallThreads / 32][258];
+    uint32_t digits[kSmallBlocks][264];  // the blocks' digit counts (padded likewise)
+    uint32_t cells[kSmallBlocks];        // the blocks' chain counts
+    uint32_t warp_sum[32];
+    uint32_t cut[(1 << LOG) / kAggPositions];  // least dmin << 16 | position of the cut windows
 };
 
-// Exclusive scan of one value per thread over a block of kSmallThreads.
+// The cluster's barrier in its two halves (a block's exited threads count as
+// arrived), and the address of a shared variable in another of its blocks.
+__device__ __forceinline__ void cluster_arrive() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(const void* shared, uint32_t block) {
+    uint32_t at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(at)
+        : "r"((uint32_t)__cvta_generic_to_shared(shared)), "r"(block));
+    return at;
+}
+
+// The sorted codes, of which block b holds [b << LOG, (b + 1) << LOG).
+template <int LOG>
+struct ClusterCodes {
+    const uint64_t* item;
+    uint32_t block;
+    __device__ __forceinline__ uint32_t operator[](uint32_t i) const {
+        const uint64_t* at = item + (i & ((1u << LOG) - 1u));
+        if (i >> LOG == block) return (uint32_t)*at;
+        uint32_t v;
+        asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_address(at, i >> LOG)));
+        return v;
+    }
+};
+
+// Exclusive scan of one value per thread over a block of WARPS warps.
+template <int WARPS>
 __device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t* warp_sum, uint32_t* total) {
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
     uint32_t x = v;
@@ -858,7 +912,7 @@ __device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t* warp_sum, u
     }
     if (lane == 31u) warp_sum[warp] = x;
     __syncthreads();
-    uint32_t w = warp_sum[lane];  // every warp scans the warps' sums
+    uint32_t w = lane < (uint32_t)WARPS ? warp_sum[lane] : 0u;  // every warp scans the warps' sums
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const uint32_t y = __shfl_up_sync(kFull, w, o);
@@ -869,37 +923,51 @@ __device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t* warp_sum, u
     return x - v + (warp ? before : 0u);
 }
 
-template <int ITEMS, bool SCAN>
+template <int LOG, bool SCAN, bool CLUSTER>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     const SimDesc* __restrict__ sims, const uint32_t* __restrict__ minmax, uint32_t npos,
     uint32_t* __restrict__ keys, float4* __restrict__ sbody, uint32_t* __restrict__ base,
     const AggPlan plan, SimOut* simout) {
     wait_for_predecessor();
     extern __shared__ unsigned long long small_shared[];
-    SmallSort<ITEMS>& s = *reinterpret_cast<SmallSort<ITEMS>*>(small_shared);
+    SmallSort<LOG>& s = *reinterpret_cast<SmallSort<LOG>*>(small_shared);
+    constexpr int ITEMS = (1 << LOG) / kSmallThreads;
+    constexpr int kWarps = kSmallThreads / 32;
+    constexpr int kParts = kSmallThreads / 256;  // threads of a digit, each with 8 warps' counts
     const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
     const uint32_t lanes_below = (1u << lane) - 1u;
-    const SimDesc& sd = sims[blockIdx.x];
-    const uint32_t n = sd.n;
+    uint32_t block = 0, cluster = 1;
+    if constexpr (CLUSTER) {
+        asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(block));
+        asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(cluster));
+    }
+    const uint32_t sim = blockIdx.x / cluster;
+    const SimDesc& sd = sims[sim];
+    const uint32_t first = block << LOG;
+    if (CLUSTER && first >= sd.n) return;  // before any barrier
+    const uint32_t blocks = (sd.n - 1u >> LOG) + 1u;
+    const uint32_t n = min(sd.n - first, 1u << LOG);  // the block's positions
+    if (CLUSTER) cluster_arrive();
     const uint32_t i0 = warp * (ITEMS * 32u) + lane;  // this thread's positions: i0 + 32 r
-    if (SCAN && t < kSmallSort / kAggPositions) s.cut[t] = kNone;
-    const RootBounds rb = root_bounds_from(minmax + 4 * blockIdx.x);
-    if (t == 0) {
-        simout[blockIdx.x].cx = rb.cx;
-        simout[blockIdx.x].cy = rb.cy;
-        simout[blockIdx.x].half = rb.half;
-        simout[blockIdx.x].crit0 = crit_of(rb.half, sd.theta);
+    if (SCAN && t < (1u << LOG) / kAggPositions) s.cut[t] = kNone;
+    const RootBounds rb = root_bounds_from(minmax + 4 * sim);
+    if (t == 0 && block == 0) {
+        simout[sim].cx = rb.cx;
+        simout[sim].cy = rb.cy;
+        simout[sim].half = rb.half;
+        simout[sim].crit0 = crit_of(rb.half, sd.theta);
     }
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
         const uint32_t i = i0 + 32u * r;
         if (i < n) {
-            const float2 xy = *reinterpret_cast<const float2*>(sd.state + i);
-            s.key[i] = morton2(quantize_axis((double)xy.x, rb.cx, rb.half),
-                               quantize_axis((double)xy.y, rb.cy, rb.half));
-            s.val[i] = (uint16_t)i;
+            const float2 xy = *reinterpret_cast<const float2*>(sd.state + first + i);
+            s.item[i] = (uint64_t)(first + i) << 32 |
+                        morton2(quantize_axis((double)xy.x, rb.cx, rb.half),
+                                quantize_axis((double)xy.y, rb.cy, rb.half));
         }
     }
+    if (CLUSTER) cluster_wait();  // every block runs: its shared memory may be written
     // a warp reads back only its own positions until the places are known
 #pragma unroll 1
     for (uint32_t shift = 0; shift < 32u; shift += 8u) {
@@ -911,7 +979,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         for (int r = 0; r < ITEMS; ++r) {
             const uint32_t i = i0 + 32u * r;
             const bool valid = i < n;
-            key[r] = valid ? s.key[i] : 0u;
+            const uint64_t item = valid ? s.item[i] : 0u;
+            key[r] = (uint32_t)item;
             const uint32_t d = (key[r] >> shift) & 255u;
             uint32_t peers = __ballot_sync(kFull, valid);
 #pragma unroll
@@ -926,19 +995,51 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
                 s.place[warp][d] = (uint16_t)(b + __popc(peers));
             }
             b = __shfl_sync(kFull, b, leader & 31u);
-            val_rank[r] = (valid ? s.val[i] : 0u) | (b + __popc(peers & lanes_below)) << 16;
+            val_rank[r] = (uint32_t)(item >> 32) | (b + __popc(peers & lanes_below)) << 16;
             __syncwarp();
         }
         __syncthreads();
-        // thread 4 d + q: digit d of warps 8 q .. 8 q + 7
-        const uint32_t d = t >> 2, w0 = (t & 3u) * 8u;
+        // thread kParts d + q: digit d of warps 8 q .. 8 q + 7
+        const uint32_t d = t / kParts, q = t % kParts, w0 = q * 8u;
         uint32_t c[8], sum = 0;
 #pragma unroll
         for (int w = 0; w < 8; ++w) c[w] = s.place[w0 + w][d];
 #pragma unroll
         for (int w = 0; w < 8; ++w) sum += c[w];
-        uint32_t total;
-        uint32_t at = small_scan(sum, s.warp_sum, &total);
+        uint32_t total, at;
+        if constexpr (CLUSTER) {
+            // to the earlier threads of the digit in this block, those of the
+            // blocks before it and the digits before it in all blocks
+            uint32_t upto = sum;
+#pragma unroll
+            for (int o = 1; o < kParts; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, upto, o, kParts);
+                if (q >= (uint32_t)o) upto += y;
+            }
+            const uint32_t mine = __shfl_sync(kFull, upto, kParts - 1, kParts);
+            for (uint32_t to = q; to < blocks; to += kParts)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                                 peer_address(&s.digits[block][d], to)),
+                             "r"(mine)
+                             : "memory");
+            cluster_arrive();
+            cluster_wait();
+            uint32_t all = 0, before = 0;
+            for (uint32_t b = q; b < blocks; b += kParts) {
+                const uint32_t v = s.digits[b][d];
+                all += v;
+                if (b < block) before += v;
+            }
+#pragma unroll
+            for (int o = 1; o < kParts; o <<= 1) {
+                all += __shfl_xor_sync(kFull, all, o);
+                before += __shfl_xor_sync(kFull, before, o);
+            }
+            at = small_scan<kWarps>(q == 0u ? all : 0u, s.warp_sum, &total);
+            at = __shfl_sync(kFull, at, 0, kParts) + before + upto - sum;
+        } else {
+            at = small_scan<kWarps>(sum, s.warp_sum, &total);
+        }
 #pragma unroll
         for (int w = 0; w < 8; ++w) {
             s.place[w0 + w][d] = (uint16_t)at;
@@ -949,12 +1050,24 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         for (int r = 0; r < ITEMS; ++r) {
             if (i0 + 32u * r < n) {
                 const uint32_t to = s.place[warp][(key[r] >> shift) & 255u] + (val_rank[r] >> 16);
-                s.key[to] = key[r];
-                s.val[to] = (uint16_t)val_rank[r];
+                const uint64_t item = (uint64_t)(val_rank[r] & 0xffffu) << 32 | key[r];
+                if constexpr (CLUSTER)
+                    asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(peer_address(
+                                     &s.item[to & ((1u << LOG) - 1u)], to >> LOG)),
+                                 "l"(item)
+                                 : "memory");
+                else
+                    s.item[to] = item;
             }
         }
-        __syncthreads();
+        if constexpr (CLUSTER) {
+            cluster_arrive();
+            cluster_wait();
+        } else {
+            __syncthreads();
+        }
     }
+    const ClusterCodes<LOG> codes{s.item, block};
     uint32_t count[ITEMS], sum = 0;
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
@@ -962,14 +1075,15 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         uint32_t cut = kNone;
         count[r] = 0;
         if (i < n) {
-            const uint32_t v = s.val[i];
+            const uint64_t item = s.item[i];
+            const uint32_t v = (uint32_t)(item >> 32);
             const float4 pm = *reinterpret_cast<const float4*>(sd.state + v);
-            keys[sd.off + i] = s.key[i];
-            sbody[sd.off + i] = make_float4(pm.x, pm.y, pm.z, __uint_as_float(v));
+            keys[sd.off + first + i] = (uint32_t)item;
+            sbody[sd.off + first + i] = make_float4(pm.x, pm.y, pm.z, __uint_as_float(v));
             if (SCAN) {
                 uint32_t dmin;
-                count[r] = chain_count(s.key, i, n, sd.bucket, sd.max_depth, &dmin);
-                cut = dmin << 16 | i;
+                count[r] = chain_count(codes, first + i, sd.n, sd.bucket, sd.max_depth, &dmin);
+                cut = dmin << 16 | (first + i);
             }
         }
         sum += count[r];
@@ -981,8 +1095,20 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     if constexpr (SCAN) {  // cells per position, scanned in position order
         uint32_t total;
         sum = __reduce_add_sync(kFull, sum);  // the warp's
-        uint32_t at = small_scan(lane ? 0u : sum, s.warp_sum, &total);
+        uint32_t at = small_scan<kWarps>(lane ? 0u : sum, s.warp_sum, &total);
         at = __shfl_sync(kFull, at, 0);
+        if constexpr (CLUSTER) {
+            if (t < blocks)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                                 peer_address(&s.cells[block], t)),
+                             "r"(total)
+                             : "memory");
+            cluster_arrive();  // also the last access to a peer's memory
+            cluster_wait();
+            const uint32_t v = lane < blocks ? s.cells[lane] : 0u;
+            at += __reduce_add_sync(kFull, lane < block ? v : 0u);
+            total = __reduce_add_sync(kFull, v);
+        }
 #pragma unroll
         for (int r = 0; r < ITEMS; ++r) {
             uint32_t x = count[r];
@@ -991,13 +1117,16 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
                 const uint32_t y = __shfl_up_sync(kFull, x, o);
                 if (lane >= (uint32_t)o) x += y;
             }
-            if (i0 + 32u * r < n) base[i0 + 32u * r] = at + x - count[r];
+            if (i0 + 32u * r < n) base[first + i0 + 32u * r] = at + x - count[r];
             at += __shfl_sync(kFull, x, 31);
         }
-        for (uint32_t p = n + t; p <= npos; p += kSmallThreads) base[p] = total;
-        if (t < plan.blocks) plan.cuts[t] = s.cut[t] & 0xffffu;
-        if (t == plan.blocks) plan.cuts[t] = npos;
-        if (t == 0) plan.inner_n[0] = 0;
+        if (block + 1u == blocks)
+            for (uint32_t p = sd.n + t; p <= npos; p += kSmallThreads) base[p] = total;
+        const uint32_t cut = first / kAggPositions + t;
+        if (t < (1u << LOG) / kAggPositions && cut < plan.blocks)
+            plan.cuts[cut] = s.cut[t] & 0xffffu;
+        if (block == 0 && t == 0) plan.cuts[plan.blocks] = npos;
+        if (block == 0 && t < plan.ranges) plan.inner_n[t] = 0;
     }
 }
 
@@ -2801,30 +2930,97 @@ static AggPlan agg_plan(const BatchBuffers& b) {
     return p;
 }
 
-// One block per simulation instead of Morton, radix and (for a single
-// simulation) scan launches, where every simulation is small enough for it (and
-// the caller has not asked for 4-bit digits).
-bool small_sort(const BatchBuffers& b) { return b.max_bodies <= kSmallSort && b.radix_bits == 8; }
-
-template <int ITEMS, bool SCAN>
-static cudaError_t sort_small(const BatchBuffers& b, cudaStream_t s) {
-    const cudaError_t e =
-        cudaFuncSetAttribute(k_sort_small<ITEMS, SCAN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SmallSort<ITEMS>));
-    if (e != cudaSuccess) return e;
-    return launch_step(k_sort_small<ITEMS, SCAN>, b.nsims, kSmallThreads, sizeof(SmallSort<ITEMS>),
-                       s, b.sims, b.minmax, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
+// Blocks that a cluster of the largest k_sort_small may have here: 16, or the
+// portable 8 where no part of the GPU holds 16 of them at once (a slice of it).
+static uint32_t sort_cluster_limit() {
+    static uint32_t cached[64] = {0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 8;
+    if (!cached[dev]) {
+        auto kernel = k_sort_small<12, true, true>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = kSmallBlocks;
+        cfg.blockDim = kSmallThreads;
+        cfg.dynamicSmemBytes = sizeof(SmallSort<12>);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kSmallBlocks;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        const bool fits =
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)sizeof(SmallSort<12>)) == cudaSuccess &&
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+                cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0;
+        if (!fits) cudaGetLastError();
+        cached[dev] = fits ? kSmallBlocks : 8u;
+    }
+    return cached[dev];
 }
 
-template <bool SCAN>
-static cudaError_t sort_small(const BatchBuffers& b, cudaStream_t s) {
-    if (b.max_bodies <= 1024) return sort_small<1, SCAN>(b, s);
-    if (b.max_bodies <= 2048) return sort_small<2, SCAN>(b, s);
-    return sort_small<4, SCAN>(b, s);
+// The form of k_sort_small that a batch gets: 2^log positions a block, `cluster`
+// blocks a simulation; log 0 for separate Morton, radix and scan launches (also
+// where the caller asked for 4-bit digits).  The fewest positions a block while
+// the batch has at most 64 blocks, since a block's time grows with them and the
+// chip has room: 8 simulations of 8,192 bodies 109, 114 and 125 us a step at 1,024,
+// 2,048 and 4,096; with 16 of them it is 149, 148 and 159, and 16 of 16,384 253, 243
+// and 243.  Not in clusters of two: 71 us against 70 in one block at 2,048 bodies.
+// With more than 64 blocks of 4,096 the chip is full, and clusters of 8 and 16,
+// partly idle where simulations differ, lose to the tiles of k_radix_pass: 16 of
+// 32,768 bodies 435 us against 421, 8 of 65,536 459 against 442, 96 of 2^10 to 2^16
+// 1,133 against 1,033; of at most 4 they do not (32 of 16,384 393 against 405).
+// No clusters where another stream keeps the GPU busy (b.clusters): one starts
+// when enough neighbouring multiprocessors have room at the same time, and twelve
+// requests' boundary solves beside the rounds of a server took 39 ms against 35.
+struct SortForm {
+    uint32_t log, cluster;
+};
+static SortForm sort_form(const BatchBuffers& b) {
+    constexpr uint32_t kRoom = 64;
+    if (b.radix_bits != 8 || b.max_bodies > kSmallSort) return {0, 0};
+    for (uint32_t log = 10; log <= 12; ++log) {
+        uint32_t cluster = 1;
+        while (cluster << log < b.max_bodies) cluster *= 2;
+        const uint64_t blocks = (uint64_t)cluster * b.nsims;
+        if (cluster > 1 && !b.clusters) continue;
+        if (cluster == 1 || (cluster > 2 && blocks <= kRoom && cluster <= sort_cluster_limit()) ||
+            (log == 12 && cluster <= 4))
+            return {log, cluster};
+    }
+    return {0, 0};
+}
+
+bool small_sort(const BatchBuffers& b) { return sort_form(b).log != 0; }
+
+template <int LOG, bool SCAN, bool CLUSTER>
+static cudaError_t sort_small(const BatchBuffers& b, uint32_t cluster, cudaStream_t s) {
+    auto kernel = k_sort_small<LOG, SCAN, CLUSTER>;
+    constexpr int bytes = (int)sizeof(SmallSort<LOG>);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && cluster > 8)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    return launch_clusters(kernel, cluster, b.nsims * cluster, kSmallThreads, bytes, s, b.sims,
+                           b.minmax, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
+}
+
+template <int LOG>
+static cudaError_t sort_small(const BatchBuffers& b, uint32_t cluster, cudaStream_t s) {
+    if (b.nsims == 1)
+        return cluster == 1 ? sort_small<LOG, true, false>(b, cluster, s)
+                            : sort_small<LOG, true, true>(b, cluster, s);
+    return cluster == 1 ? sort_small<LOG, false, false>(b, cluster, s)
+                        : sort_small<LOG, false, true>(b, cluster, s);
 }
 
 cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s) {
-    return b.nsims == 1 ? sort_small<true>(b, s) : sort_small<false>(b, s);
+    const SortForm f = sort_form(b);
+    return f.log == 10   ? sort_small<10>(b, f.cluster, s)
+           : f.log == 11 ? sort_small<11>(b, f.cluster, s)
+                         : sort_small<12>(b, f.cluster, s);
 }
 
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {

@@ -766,6 +766,38 @@ def test_one_block_sort_at_its_edges(gpu, rt, oracle, bucket):
         assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
 
 
+@pytest.mark.parametrize("n,copies", [(4097, 3), (8191, 2), (8193, 9), (16384, 5), (16385, 2),
+                                      (32768, 2), (32769, 2), (65535, 2), (65536, 3), (65537, 2)])
+def test_cluster_sort_at_its_edges(gpu, rt, oracle, n, copies):
+    """Up to 65,536 bodies are sorted by a cluster of 4 to 16 blocks of 1,024,
+    2,048 or 4,096 keys: sizes at those edges, half the bodies on a lattice of
+    equal codes (the stable order), alone and in batches with smaller members
+    (blocks without a key), whose copies decide the block's size.  Bit for bit,
+    so no tolerance."""
+    from galaxy_b200.batch import Batch
+    rng = np.random.default_rng(n)
+    cfg = Config(theta=0.7, softening_kpc=0.02, g=1.0, bucket=2, force_stats=False)
+    members, alone = [], []
+    for k in [n] * copies + [2, 1025, n // 2 + 1]:
+        bodies = np.zeros((k, 5))
+        bodies[:, :2] = rng.uniform(-1, 1, (k, 2))
+        half = k // 2
+        bodies[:half, :2] = rng.integers(0, 50, (half, 2)) / 49.0
+        bodies = bodies[rng.permutation(k)]
+        bodies[:, 4] = rng.uniform(0.5, 2.0, k) / k
+        ev, tree, evid, ot, b32, oc = build_both(gpu, rt, oracle, bodies, cfg)
+        if len(members) % copies == 0:
+            assert_tree_bit_exact(oracle, evid, ot, b32, oc, cfg)
+        rt.force(gpu, ev, tree, cfg)
+        alone.append(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32))
+        tree.close()
+        ev.close()
+        members.append(gpu.create_evolving_state(bodies)[0])
+    Batch(gpu, members, [cfg] * len(members)).solve()
+    for ev, want in zip(members, alone):
+        assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
+
+
 @pytest.mark.parametrize("n,probes", [(2, 1), (2047, 2), (2049, 8), (4097, 9), (30001, 64),
                                       (30001, 30001)])
 def test_direct_probes_in_slices(gpu, oracle, n, probes):
