@@ -959,7 +959,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
 
     b->h_sims.resize(count);
     b->h_chunk_sim.assign(L.nchunks, kNone);
-    uint32_t tile = 0;
+    uint32_t tile = 0, group = 0;
     for (uint32_t s = 0; s < count; ++s) {
         SimDesc& sd = b->h_sims[s];
         memset(&sd, 0, sizeof sd);
@@ -978,9 +978,12 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
             tl.sim = s;
             tl.start = L.off[s] + t0;
             tl.count = std::min<uint32_t>(kTile, counts[s] - t0);
+            // 4 KB per group of simulations above kTile bodies: agg_region has 96
+            tl.group = counts[s] <= kTile ? kNone : group + t0 / (kTile * kGroupTiles);
             b->h_tiles.push_back(tl);
             ++tile;
         }
+        if (counts[s] > kTile) group += (counts[s] + kTile * kGroupTiles - 1) / (kTile * kGroupTiles);
     }
     cudaStream_t st = dev->stream;
     if ((e = cudaMemcpyAsync(b->d_sims, b->h_sims.data(), sizeof(SimDesc) * count,

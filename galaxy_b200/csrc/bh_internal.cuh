@@ -16,6 +16,8 @@ constexpr int kSortItems = 16;
 constexpr uint32_t kTile = kSortThreads * kSortItems;  // keys per radix tile (4096)
 constexpr int kRadixDigits = 256;
 constexpr int kRadixPasses = 4;
+constexpr uint32_t kGroupTiles = 32;  // tiles whose digit counts are also summed together
+constexpr uint32_t kGroupStride = kRadixPasses * kRadixDigits;  // a group's words, all passes
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;  // 1024-position scan tiles: a shorter per-tile chain
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // positions per scan tile
@@ -74,7 +76,7 @@ struct Tile {
     uint32_t sim;
     uint32_t start;  // first position
     uint32_t count;  // keys in this tile (<= kTile)
-    uint32_t reserved;
+    uint32_t group;  // its group's words in the sort (kNone: its simulation's only tile)
 };
 
 // Device buffers of one batch (all sized from the batch layout).
@@ -114,7 +116,8 @@ struct BatchBuffers {
                         // root at slot 0 of group cell_capacity + s (traversal)
     double4* cell_d;    // com_x, com_y, mass (f64), then the f32 residuals of
                         // com_x, com_y (float2 bits): com - (float)com
-    void* agg_region;   // the aggregates' cuts and lists of cells across them
+    void* agg_region;   // during the sort the tile groups' digit counts, then the
+                        // aggregates' cuts and lists of cells across them
     // persistent
     uint32_t* err;                   // error bits
     unsigned long long* force_stats; // 4 counters

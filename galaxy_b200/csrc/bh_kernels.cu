@@ -8,7 +8,7 @@
 //   k_morton      f64 root bounds + 16-bit/axis quantization + Morton code
 //                 (nbody/src/lib.rs:137-154, nbody/src/flat.rs:67-94), fused
 //                 with the four 8-bit digit histograms of the radix sort
-//   k_radix_pass  one stable LSD pass (onesweep: decoupled look-back, warp
+//   k_radix_pass  one stable LSD pass (onesweep: look-back by tile groups, warp
 //                 match ranking, shared-memory staged scatter); the last pass
 //                 also gathers the bodies into Morton order
 //   k_sort_small  codes, sort, gather and chain scan of a simulation of at most
@@ -450,7 +450,8 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const SimDesc* __rest
                                                          const Tile* __restrict__ tiles,
                                                          const uint32_t* __restrict__ minmax,
                                                          uint32_t* __restrict__ keys,
-                                                         uint32_t* hist, SimOut* simout) {
+                                                         uint32_t* hist, uint32_t* group_words,
+                                                         SimOut* simout) {
     wait_for_predecessor();
     constexpr int kPasses = 32 / BITS;
     constexpr uint32_t kDig = 1u << BITS;
@@ -459,6 +460,9 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const SimDesc* __rest
     __syncthreads();
     const Tile t = tiles[blockIdx.x];
     const SimDesc& sd = sims[t.sim];
+    if (t.group != kNone && (t.start - sd.off) / kTile % kGroupTiles == 0u)
+        for (uint32_t k = threadIdx.x; k < kGroupStride; k += kMortonThreads)
+            group_words[(size_t)t.group * kGroupStride + k] = 0u;
     const RootBounds rb = root_bounds_from(minmax + 4 * t.sim);
     if (threadIdx.x == 0 && t.start == sd.off) {
         simout[t.sim].cx = rb.cx;
@@ -490,50 +494,55 @@ __global__ void __launch_bounds__(kMortonThreads) k_morton(const SimDesc* __rest
 // ============================================================== radix =====
 
 #ifndef GBH_LOOK_WINDOW
-#define GBH_LOOK_WINDOW 8
+#define GBH_LOOK_WINDOW 16
 #endif
-constexpr int kLookWindow = GBH_LOOK_WINDOW;  // predecessor flags loaded per look-back round trip
-constexpr uint32_t kFlagAgg = 1u << 30;
-constexpr uint32_t kFlagInc = 2u << 30;
-constexpr uint32_t kFlagMask = (1u << 30) - 1u;
+constexpr int kLookWindow = GBH_LOOK_WINDOW;  // counts loaded per look-back round trip
+// A published count: kGroupTiles << kCountBits | count.  A tile's word gets it at
+// once; its group's word, to which each of the kGroupTiles tiles adds 1 <<
+// kCountBits | count, once they all have.
+constexpr uint32_t kCountBits = 20;
+constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
+static_assert(kGroupTiles * kTile <= kCountMask, "a group's count fits its bits");
 
-// Decoupled look-back of tile t for one digit (flags[tile * stride] holds
-// that tile's state | count): the sum of the predecessors' counts back to the
-// nearest inclusive prefix, reading kLookWindow flags per round trip and
-// re-polling from the first tile that has not published yet.  The
-// simulation's first tile publishes an inclusive prefix at once, so the
-// window never needs tiles before it.  The wait is bounded: once `limit`
-// clock cycles have passed since it began and a round finds an unpublished
-// predecessor, it sets kErrLookbackTimeout and returns the partial sum, which
-// is at most the true prefix (the caller's writes stay in range).
-__device__ __forceinline__ uint32_t lookback_digit(const uint32_t* flags, uint32_t stride,
-                                                   uint32_t t, uint32_t first_tile,
-                                                   uint32_t* err, long long limit) {
+// Look-back for one digit: the counts of the `tiles` tiles of the group before
+// this one (tile_words[i * stride]) and of the `groups` groups before it
+// (group_words[i * kGroupStride]), kLookWindow loads per round trip, each window
+// polled until it is published.  No tile waits for another's look-back, only for
+// its count.  The wait is bounded: once `limit` clock cycles have passed since it
+// began and a count is missing, it sets kErrLookbackTimeout and returns the sum of
+// the windows before, which is at most the true prefix (the caller's writes stay
+// in range).
+__device__ __forceinline__ uint32_t lookback_digit(const uint32_t* tile_words, uint32_t stride,
+                                                   uint32_t tiles, const uint32_t* group_words,
+                                                   uint32_t groups, uint32_t* err,
+                                                   long long limit) {
     uint32_t excl = 0;
-    uint32_t tp = t - 1;
     const long long t0 = clock64();
-    while (true) {
-        uint32_t f[kLookWindow];
+    for (uint32_t i0 = 0; i0 < tiles + groups; i0 += kLookWindow) {
+        uint32_t sum;
+        bool all;
+        do {
+            uint32_t f[kLookWindow];
 #pragma unroll
-        for (int j = 0; j < kLookWindow; ++j)
-            f[j] = tp >= first_tile + j ? ld_volatile(flags + (size_t)(tp - j) * stride) : 0u;
-        bool done = false;
-        int used = 0;
+            for (int j = 0; j < kLookWindow; ++j) {
+                const uint32_t i = i0 + j;
+                f[j] = i < tiles            ? ld_volatile(tile_words + (size_t)i * stride)
+                       : i < tiles + groups ? ld_volatile(group_words + (size_t)(i - tiles) * kGroupStride)
+                                            : kGroupTiles << kCountBits;
+            }
+            sum = 0;
+            all = true;
 #pragma unroll
-        for (int j = 0; j < kLookWindow; ++j) {
-            if (done || used < j) continue;
-            const uint32_t st = f[j] & ~kFlagMask;
-            if (st == 0u) continue;
-            excl += f[j] & kFlagMask;
-            used = j + 1;
-            done = st == kFlagInc;
-        }
-        if (done) break;
-        tp -= used;
-        if (used < kLookWindow && clock64() - t0 > limit) {
-            set_err(err, kErrLookbackTimeout);
-            break;
-        }
+            for (int j = 0; j < kLookWindow; ++j) {
+                all = all && f[j] >> kCountBits == kGroupTiles;
+                sum += f[j] & kCountMask;
+            }
+            if (!all && clock64() - t0 > limit) {
+                set_err(err, kErrLookbackTimeout);
+                return excl;
+            }
+        } while (!all);
+        excl += sum;
     }
     return excl;
 }
@@ -545,22 +554,33 @@ __device__ __forceinline__ uint32_t lookback_digit(const uint32_t* flags, uint32
 __global__ void k_wait_probe(const uint32_t* flags, uint32_t* err, long long limit,
                              uint32_t* out) {
     const uint32_t d = threadIdx.x;
-    out[d] = lookback_digit(flags + d, kRadixDigits, 1u, 0u, err, limit);
+    out[d] = lookback_digit(flags + d, kRadixDigits, 1u, nullptr, 0u, err, limit);
 }
 
 // One stable BITS-wide LSD pass (BITS = 8: 4 passes, 4: 8 passes) over every
 // simulation's keys.  Tiles never cross simulations; within a simulation,
-// tile order is key order and the decoupled look-back adds the digit counts
-// of the preceding tiles.  Items are ranked warp by warp in key order (the
+// tile order is key order and the look-back adds the digit counts of the
+// preceding tiles.  Items are ranked warp by warp in key order (the
 // lanes sharing a digit found with one ballot per digit bit), so equal
 // digits keep their input order: the permutation equals a stable sort by
 // code, as Rust's sort_by_key (nbody/src/flat.rs:233-234).
+// A tile's counts go to its own words and, added, to those of its group of
+// kGroupTiles tiles, so its look-back reads at most 31 tiles and the groups before
+// it, 16 words a round trip, where a chain of tiles advanced 8 a round trip: 2^20
+// bodies' four passes 80 -> 74 us, 2^18 51 -> 47.  What is left, in cycles of a tile
+// at 2^20 (2 tiles an SM): loads 2,500, ranking 4,000 to 5,000, waiting for the
+// slowest of the tiles before it 5,000 to 9,000, scans and the local scatter 3,000,
+// stores 2,000, and in the last pass the gather of a random 32-byte sector a body,
+// 20,000 of them (with its loads issued together and no store of the values, which
+// the bodies' records carry, 74 -> 70 us).  Counting with shared atomics before the
+// ranking, to publish earlier, costs more than it saves (76 us; 2^18 57).
 // MINB tiles share an SM: 2 (up to 128 registers) for sorts of one wave,
 // 3 (80 registers) for sorts of many waves of tiles (large batches).
 template <int BITS, int PASS, bool LAST, int MINB>
 __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
     const SimDesc* __restrict__ sims, const Tile* __restrict__ tiles, uint32_t* tile_counter,
-    const uint32_t* __restrict__ hist, uint32_t* flags, const uint32_t* __restrict__ keys_in,
+    const uint32_t* __restrict__ hist, uint32_t* flags, uint32_t* group_words,
+    const uint32_t* __restrict__ keys_in,
     const uint32_t* __restrict__ vals_in, uint32_t* __restrict__ keys_out,
     uint32_t* __restrict__ vals_out, float4* __restrict__ sbody, uint32_t* err) {
     wait_for_predecessor();
@@ -629,13 +649,15 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
             run += c;
         }
     }
-    const bool first = (t == sd.first_tile);
-    uint32_t* my_flag = flags + (size_t)t * kDig + d;
-    if (owner) atomicExch(my_flag, (first ? kFlagInc : kFlagAgg) | run);
+    const uint32_t before = t - sd.first_tile, in_group = before % kGroupTiles;
     uint32_t excl = 0;
-    if (owner && !first) {
-        excl = lookback_digit(flags + d, kDig, t, sd.first_tile, err, kSpinCycles);
-        atomicExch(my_flag, kFlagInc | (excl + run));
+    if (owner && tl.group != kNone) {
+        uint32_t* group = group_words + (size_t)tl.group * kGroupStride + PASS * kDig + d;
+        atomicExch(flags + (size_t)t * kDig + d, kGroupTiles << kCountBits | run);
+        atomicAdd(group, 1u << kCountBits | run);
+        excl = lookback_digit(flags + (size_t)(t - in_group) * kDig + d, kDig, in_group,
+                              group - (size_t)(before / kGroupTiles) * kGroupStride,
+                              before / kGroupTiles, err, kSpinCycles);
     }
     uint32_t tot;
     const uint32_t h = owner ? hist[(size_t)tl.sim * kHistStride + PASS * kDig + d] : 0u;
@@ -657,18 +679,29 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
         }
     }
     __syncthreads();
+    // the gather's loads are issued four at a time
+    constexpr int kGather = LAST ? 4 : 1;
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t slot = k * kSortThreads + threadIdx.x;
-        if (slot < tl.count) {
-            const uint32_t kk = s_keys[slot];
-            const uint32_t vv = s_vals[slot];
-            const uint32_t dest = s_out[(kk >> shift) & (kDig - 1u)] + slot;
-            keys_out[dest] = kk;
-            vals_out[dest] = vv;
-            if (LAST) {
-                const float4 pm = *reinterpret_cast<const float4*>(sd.state + vv);
-                sbody[dest] = make_float4(pm.x, pm.y, pm.z, __uint_as_float(vv));
+    for (int k0 = 0; k0 < kSortItems; k0 += kGather) {
+        float4 pm[kGather];
+#pragma unroll
+        for (int k = 0; LAST && k < kGather; ++k) {
+            const uint32_t slot = (k0 + k) * kSortThreads + threadIdx.x;
+            if (slot < tl.count)
+                pm[k] = __ldcg(reinterpret_cast<const float4*>(sd.state + s_vals[slot]));
+        }
+#pragma unroll
+        for (int k = 0; k < kGather; ++k) {
+            const uint32_t slot = (k0 + k) * kSortThreads + threadIdx.x;
+            if (slot < tl.count) {
+                const uint32_t kk = s_keys[slot];
+                const uint32_t vv = s_vals[slot];
+                const uint32_t dest = s_out[(kk >> shift) & (kDig - 1u)] + slot;
+                keys_out[dest] = kk;
+                if (LAST)  // the values end in the bodies' records
+                    sbody[dest] = make_float4(pm[k].x, pm[k].y, pm[k].z, __uint_as_float(vv));
+                else
+                    vals_out[dest] = vv;
             }
         }
     }
@@ -1068,6 +1101,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         }
     }
     const ClusterCodes<LOG> codes{s.item, block};
+    float4 pm[ITEMS];  // the gather's loads are issued together
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        if (i0 + 32u * r < n)
+            pm[r] = __ldcg(reinterpret_cast<const float4*>(sd.state + (s.item[i0 + 32u * r] >> 32)));
     uint32_t count[ITEMS], sum = 0;
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
@@ -1077,9 +1115,8 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         if (i < n) {
             const uint64_t item = s.item[i];
             const uint32_t v = (uint32_t)(item >> 32);
-            const float4 pm = *reinterpret_cast<const float4*>(sd.state + v);
             keys[sd.off + first + i] = (uint32_t)item;
-            sbody[sd.off + first + i] = make_float4(pm.x, pm.y, pm.z, __uint_as_float(v));
+            sbody[sd.off + first + i] = make_float4(pm[r].x, pm[r].y, pm[r].z, __uint_as_float(v));
             if (SCAN) {
                 uint32_t dmin;
                 count[r] = chain_count(codes, first + i, sd.n, sd.bucket, sd.max_depth, &dmin);
@@ -2858,13 +2895,13 @@ cudaError_t launch_integrate(const BatchBuffers& b, int mode, cudaStream_t s) {
 cudaError_t launch_morton(const BatchBuffers& b, cudaStream_t s) {
     if (b.radix_bits == 4)
         return launch_step(k_morton<4>, b.ntiles, kMortonThreads, 0, s, b.sims, b.tiles, b.minmax,
-                           b.keys_a, b.hist, b.simout);
+                           b.keys_a, b.hist, (uint32_t*)b.agg_region, b.simout);
     return launch_step(k_morton<8>, b.ntiles, kMortonThreads, 0, s, b.sims, b.tiles, b.minmax,
-                       b.keys_a, b.hist, b.simout);
+                       b.keys_a, b.hist, (uint32_t*)b.agg_region, b.simout);
 }
 
 // Passes alternate a -> b -> a ...; an even pass count leaves the sorted keys
-// in keys_a / vals_a, and the last pass also gathers the sorted bodies.
+// in keys_a, and the last pass also gathers the sorted bodies (with their indices).
 // Streaming multiprocessors of the current device (cached per device).
 static int sm_count() {
     static int cached[64] = {0};
@@ -2892,11 +2929,11 @@ static cudaError_t radix_passes(const BatchBuffers& b, cudaStream_t s) {
     const cudaError_t e =
         many ? launch_step(k_radix_pass<BITS, PASS, PASS == kPasses - 1, 3>, b.ntiles,
                            kSortThreads, 0, s, b.sims, b.tiles, b.counters + PASS, b.hist,
-                           b.sort_flags + PASS * fstride, kin, PASS == 0 ? nullptr : vin, kout,
+                           b.sort_flags + PASS * fstride, (uint32_t*)b.agg_region, kin, PASS == 0 ? nullptr : vin, kout,
                            vout, b.sbody, b.err)
              : launch_step(k_radix_pass<BITS, PASS, PASS == kPasses - 1, 2>, b.ntiles,
                            kSortThreads, 0, s, b.sims, b.tiles, b.counters + PASS, b.hist,
-                           b.sort_flags + PASS * fstride, kin, PASS == 0 ? nullptr : vin, kout,
+                           b.sort_flags + PASS * fstride, (uint32_t*)b.agg_region, kin, PASS == 0 ? nullptr : vin, kout,
                            vout, b.sbody, b.err);
     if (e != cudaSuccess) return e;
     if constexpr (PASS + 1 < kPasses) return radix_passes<BITS, PASS + 1>(b, s);

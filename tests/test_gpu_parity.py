@@ -798,6 +798,36 @@ def test_cluster_sort_at_its_edges(gpu, rt, oracle, n, copies):
         assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
 
 
+@pytest.mark.parametrize("n", [131071, 131072, 131073, 262145])
+def test_radix_tile_groups_at_their_edges(gpu, rt, oracle, n):
+    """The sort adds digit counts by tiles of 4,096 keys and groups of 32 tiles:
+    sizes at a group's edges, half the bodies on a lattice of equal codes (the
+    stable order), alone and in a batch between simulations of one tile, two
+    tiles and other groups.  Bit for bit, so no tolerance."""
+    from galaxy_b200.batch import Batch
+    rng = np.random.default_rng(n)
+    cfg = Config(theta=0.8, softening_kpc=0.02, g=1.0, bucket=4, force_stats=False)
+    members, alone = [], []
+    for k in (4096, 131073, 5, n, 4097):
+        bodies = np.zeros((k, 5))
+        bodies[:, :2] = rng.uniform(-1, 1, (k, 2))
+        half = k // 2
+        bodies[:half, :2] = rng.integers(0, 50, (half, 2)) / 49.0
+        bodies = bodies[rng.permutation(k)]
+        bodies[:, 4] = rng.uniform(0.5, 2.0, k) / k
+        ev, tree, evid, ot, b32, oc = build_both(gpu, rt, oracle, bodies, cfg)
+        if k == n:
+            assert_tree_bit_exact(oracle, evid, ot, b32, oc, cfg)
+        rt.force(gpu, ev, tree, cfg)
+        alone.append(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32))
+        tree.close()
+        ev.close()
+        members.append(gpu.create_evolving_state(bodies)[0])
+    Batch(gpu, members, [cfg] * len(members)).solve()
+    for ev, want in zip(members, alone):
+        assert np.array_equal(gpu.read_evolving_accelerations_f32(ev)[0].view(np.uint32), want)
+
+
 @pytest.mark.parametrize("n,probes", [(2, 1), (2047, 2), (2049, 8), (4097, 9), (30001, 64),
                                       (30001, 30001)])
 def test_direct_probes_in_slices(gpu, oracle, n, probes):
