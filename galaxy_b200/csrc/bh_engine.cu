@@ -1032,15 +1032,16 @@ enum Stage { kStBounds, kStMorton, kStRadix, kStTopology, kStAggregate };
 static int enqueue_rebuild(Batch* b, int integrate_mode, cudaEvent_t* ev) {
     cudaStream_t s = b->dev->stream;
     if (ev) CK(cudaEventRecord(ev[0], s), "event");
-    CK(cudaMemsetAsync(b->control, 0, b->control_bytes, s), "control memset");
-    CK(launch_integrate(b->bb, integrate_mode, s), "integrate launch");
-    if (ev) CK(cudaEventRecord(ev[1], s), "event");
     const bool small = small_sort(b->bb);  // one launch, timed as the radix stage
+    const bool scanned = small && b->bb.nsims == 1;
+    if (!scanned) CK(cudaMemsetAsync(b->control, 0, b->control_bytes, s), "control memset");
+    if (!small) CK(launch_integrate(b->bb, integrate_mode, s), "integrate launch");
+    if (ev) CK(cudaEventRecord(ev[1], s), "event");
     if (!small) CK(launch_morton(b->bb, s), "morton launch");
     if (ev) CK(cudaEventRecord(ev[2], s), "event");
-    CK(small ? launch_sort_small(b->bb, s) : launch_radix(b->bb, s), "radix launch");
+    CK(small ? launch_sort_small(b->bb, integrate_mode, s) : launch_radix(b->bb, s), "radix launch");
     if (ev) CK(cudaEventRecord(ev[3], s), "event");
-    if (!small || b->bb.nsims > 1) CK(launch_count_scan(b->bb, s), "count/scan launch");
+    if (!scanned) CK(launch_count_scan(b->bb, s), "count/scan launch");
     if (ev) CK(cudaEventRecord(ev[4], s), "event");
     CK(launch_aggregate(b->bb, s), "aggregate launch");
     if (ev) CK(cudaEventRecord(ev[5], s), "event");

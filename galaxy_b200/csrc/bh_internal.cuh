@@ -128,10 +128,11 @@ struct BatchBuffers {
 cudaError_t launch_integrate(const BatchBuffers& b, int mode, cudaStream_t s);
 cudaError_t launch_morton(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s);
-// Whether Morton codes, sort and gather run as launch_sort_small (which also
-// does launch_count_scan's work for a single simulation).
+// Whether a step's integration and bounds (the mode of launch_integrate), Morton
+// codes, sort and gather run as launch_sort_small, which needs no zeroed control
+// block and also does launch_count_scan's work for a single simulation.
 bool small_sort(const BatchBuffers& b);
-cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s);
+cudaError_t launch_sort_small(const BatchBuffers& b, int mode, cudaStream_t s);
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s);
 // Recomputes G*m and the MAC bounds of simulation `sim` for new theta / G.

@@ -11,7 +11,7 @@
 //   k_radix_pass  one stable LSD pass (onesweep: look-back by tile groups, warp
 //                 match ranking, shared-memory staged scatter); the last pass
 //                 also gathers the bodies into Morton order
-//   k_sort_small  codes, sort, gather and chain scan of a simulation of at most
+//   k_sort_small  all of these and the chain scan of a simulation of at most
 //                 65,536 bodies in one block or cluster
 //   k_count_scan  cells per position + exclusive scan (cell numbering in the
 //                 reference's recursive preorder, nbody/src/flat.rs:127-177)
@@ -98,17 +98,18 @@ struct RootBounds {
 };
 
 // nbody/src/lib.rs:137-154 over the f32 min/max promoted to f64.
-__device__ __forceinline__ RootBounds root_bounds_from(const uint32_t* mm) {
-    double min_x = (double)dec_f32(~mm[0]);
-    double min_y = (double)dec_f32(~mm[1]);
-    double max_x = (double)dec_f32(mm[2]);
-    double max_y = (double)dec_f32(mm[3]);
+__device__ __forceinline__ RootBounds root_bounds(float mnx, float mny, float mxx, float mxy) {
+    const double min_x = mnx, min_y = mny, max_x = mxx, max_y = mxy;
     double span = fmax(fmax(__dsub_rn(max_x, min_x), __dsub_rn(max_y, min_y)), 1e-12);
     RootBounds r;
     r.cx = __dmul_rn(__dadd_rn(min_x, max_x), 0.5);
     r.cy = __dmul_rn(__dadd_rn(min_y, max_y), 0.5);
     r.half = __dadd_rn(__dmul_rn(span, 0.500000000001), 1e-12);
     return r;
+}
+
+__device__ __forceinline__ RootBounds root_bounds_from(const uint32_t* mm) {
+    return root_bounds(dec_f32(~mm[0]), dec_f32(~mm[1]), dec_f32(mm[2]), dec_f32(mm[3]));
 }
 
 // Root width / theta, +inf at theta = 0 (every cell opens).
@@ -254,6 +255,22 @@ constexpr long long kSpinCycles = 2000000000ll;
 // chunks whose loads a warp keeps in flight (modes with the bounds reduction)
 constexpr int kIntegrateUnrollBounds = GBH_INTEGRATE_UNROLL;
 
+// The kick / drift of one record.
+__device__ __forceinline__ void integrate(int mode, float dt, float4& pm, float4& v,
+                                          const float4& a) {
+    const float hdt = __fmul_rn(0.5f, dt);
+    if (mode == 2 || mode == 3) {
+        v.x = __fadd_rn(v.x, __fmul_rn(hdt, a.x));
+        v.y = __fadd_rn(v.y, __fmul_rn(hdt, a.y));
+    }
+    if (mode == 1 || mode == 3) {
+        v.x = __fadd_rn(v.x, __fmul_rn(hdt, a.x));
+        v.y = __fadd_rn(v.y, __fmul_rn(hdt, a.y));
+        pm.x = __fadd_rn(pm.x, __fmul_rn(dt, v.x));
+        pm.y = __fadd_rn(pm.y, __fmul_rn(dt, v.y));
+    }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(256) k_integrate(const SimDesc* __restrict__ sims,
                                                    const uint32_t* __restrict__ chunk_sim,
@@ -309,20 +326,7 @@ __global__ void __launch_bounds__(256) k_integrate(const SimDesc* __restrict__ s
         n = sd.n;
         dt = sd.dt;
     };
-    // the kick / drift of one record, with its bounds
-    auto update = [&](float4& pm, float4& v, const float4& a) {
-        const float hdt = __fmul_rn(0.5f, dt);
-        if (MODE == 2 || MODE == 3) {
-            v.x = __fadd_rn(v.x, __fmul_rn(hdt, a.x));
-            v.y = __fadd_rn(v.y, __fmul_rn(hdt, a.y));
-        }
-        if (MODE == 1 || MODE == 3) {
-            v.x = __fadd_rn(v.x, __fmul_rn(hdt, a.x));
-            v.y = __fadd_rn(v.y, __fmul_rn(hdt, a.y));
-            pm.x = __fadd_rn(pm.x, __fmul_rn(dt, v.x));
-            pm.y = __fadd_rn(pm.y, __fmul_rn(dt, v.y));
-        }
-    };
+    auto update = [&](float4& pm, float4& v, const float4& a) { integrate(MODE, dt, pm, v, a); };
     auto bound = [&](const float4& pm) {
         if (kBounds) {
             mnx = fminf(mnx, pm.x);
@@ -867,9 +871,10 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(
 // ========================================================= small sort =====
 
 // A simulation of at most kSmallSort bodies in one block or one cluster of up to
-// 16: Morton codes, the four stable 8-bit passes in shared memory (a cluster's
-// blocks write one another's), the gather into Morton order and, where the batch
-// is that one simulation (SCAN), the chain counts and their scan.  Separate
+// 16: the step's integration (mode as k_integrate) and bounds, Morton codes, the
+// four stable 8-bit passes in shared memory (a cluster's blocks write one
+// another's), the gather into Morton order and, where the batch is that one
+// simulation (SCAN), the chain counts and their scan.  Separate
 // launches cost 10 us for the codes, 7 to 10 a pass and 10 for the scan however
 // few keys they have: a launch, a chain of loads, a look-back, global stores.  A
 // warp ranks its positions in order as k_radix_pass does (the lanes that share a
@@ -885,7 +890,10 @@ __global__ void __launch_bounds__(kScanThreads) k_count_scan(
 // shorter chains than 256: 92.6, 93.6 and 92.9 us a step at 16,384 bodies, 145, 146
 // and 156 at 65,536.  Steps against separate launches: 4,096 bodies 121 -> 80 us (one
 // block of 1,024 threads: 88), 8,192 112 -> 84, 16,384 117 -> 91, 32,768 128 -> 109,
-// 65,536 154 -> 145.
+// 65,536 154 -> 145.  With the integration and the bounds here too, and so no
+// memset and no second reading of the positions, a rebuild takes 8 us less, a step
+// 1,024 bodies 58 -> 56, 16,384 93 -> 92, 65,536 147 -> 148, 64 simulations of 16,384
+// in a batch 705 -> 669.
 constexpr int kSmallThreads = 512;
 constexpr uint32_t kSmallBlocks = 16;  // most blocks of a cluster
 static_assert(kSmallSort == kSmallBlocks * 4096u && kSmallSort <= 65536u,
@@ -898,6 +906,8 @@ struct SmallSort {
     // threads of a digit read rows 8 apart, in different banks)
     uint16_t place[kSmallThreads / 32][258];
     uint32_t digits[kSmallBlocks][264];  // the blocks' digit counts (padded likewise)
+    float4 block_bounds[kSmallBlocks];   // the blocks' (min x, min y, max x, max y)
+    float4 bounds[kSmallThreads / 32];   // the warps'
     uint32_t cells[kSmallBlocks];        // the blocks' chain counts
     uint32_t warp_sum[32];
     uint32_t cut[(1 << LOG) / kAggPositions];  // least dmin << 16 | position of the cut windows
@@ -958,11 +968,10 @@ __device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t* warp_sum, u
 
 template <int LOG, bool SCAN, bool CLUSTER>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
-    const SimDesc* __restrict__ sims, const uint32_t* __restrict__ minmax, uint32_t npos,
-    uint32_t* __restrict__ keys, float4* __restrict__ sbody, uint32_t* __restrict__ base,
-    const AggPlan plan, SimOut* simout) {
+    const SimDesc* __restrict__ sims, int mode, uint32_t npos, uint32_t* __restrict__ keys,
+    float4* __restrict__ sbody, uint32_t* __restrict__ base, const AggPlan plan, SimOut* simout) {
     wait_for_predecessor();
-    extern __shared__ unsigned long long small_shared[];
+    extern __shared__ float4 small_shared[];
     SmallSort<LOG>& s = *reinterpret_cast<SmallSort<LOG>*>(small_shared);
     constexpr int ITEMS = (1 << LOG) / kSmallThreads;
     constexpr int kWarps = kSmallThreads / 32;
@@ -983,7 +992,72 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     if (CLUSTER) cluster_arrive();
     const uint32_t i0 = warp * (ITEMS * 32u) + lane;  // this thread's positions: i0 + 32 r
     if (SCAN && t < (1u << LOG) / kAggPositions) s.cut[t] = kNone;
-    const RootBounds rb = root_bounds_from(minmax + 4 * sim);
+    // the bodies moved (as k_integrate) and bounded, kBatch loads at a time
+    constexpr int kBatch = ITEMS < 4 ? ITEMS : 4;
+    float2 xy[ITEMS];
+    float mnx = INFINITY, mny = INFINITY, mxx = -INFINITY, mxy = -INFINITY;
+#pragma unroll
+    for (int r0 = 0; r0 < ITEMS; r0 += kBatch) {
+        float4 pm[kBatch], v[kBatch], acc[kBatch];
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const uint32_t i = i0 + 32u * (r0 + r);
+            if (i >= n) continue;
+            const float4* st = reinterpret_cast<const float4*>(sd.state + first + i);
+            pm[r] = st[0];
+            if (mode != 0) {
+                v[r] = st[1];
+                acc[r] = sd.accel[first + i];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < kBatch; ++r) {
+            const uint32_t i = i0 + 32u * (r0 + r);
+            if (i >= n) continue;
+            if (mode != 0) {
+                integrate(mode, sd.dt, pm[r], v[r], acc[r]);
+                float4* st = reinterpret_cast<float4*>(sd.state + first + i);
+                st[0] = pm[r];
+                st[1] = v[r];
+            }
+            xy[r0 + r] = make_float2(pm[r].x, pm[r].y);
+            mnx = fminf(mnx, pm[r].x);
+            mny = fminf(mny, pm[r].y);
+            mxx = fmaxf(mxx, pm[r].x);
+            mxy = fmaxf(mxy, pm[r].y);
+        }
+    }
+    auto reduce = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mnx = fminf(mnx, __shfl_xor_sync(kFull, mnx, o));
+            mny = fminf(mny, __shfl_xor_sync(kFull, mny, o));
+            mxx = fmaxf(mxx, __shfl_xor_sync(kFull, mxx, o));
+            mxy = fmaxf(mxy, __shfl_xor_sync(kFull, mxy, o));
+        }
+    };
+    auto gather = [&](const float4* bounds, uint32_t count) {  // each lane one, then all
+        const float4 b = lane < count ? bounds[lane]
+                                      : make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
+        mnx = b.x, mny = b.y, mxx = b.z, mxy = b.w;
+        reduce();
+    };
+    reduce();
+    if (lane == 0) s.bounds[warp] = make_float4(mnx, mny, mxx, mxy);
+    __syncthreads();
+    gather(s.bounds, kWarps);
+    if constexpr (CLUSTER) {
+        cluster_wait();  // every block runs: its shared memory may be written
+        if (t < blocks)
+            asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(
+                             peer_address(&s.block_bounds[block], t)),
+                         "f"(mnx), "f"(mny), "f"(mxx), "f"(mxy)
+                         : "memory");
+        cluster_arrive();
+        cluster_wait();
+        gather(s.block_bounds, blocks);
+    }
+    const RootBounds rb = root_bounds(mnx, mny, mxx, mxy);
     if (t == 0 && block == 0) {
         simout[sim].cx = rb.cx;
         simout[sim].cy = rb.cy;
@@ -993,14 +1067,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
         const uint32_t i = i0 + 32u * r;
-        if (i < n) {
-            const float2 xy = *reinterpret_cast<const float2*>(sd.state + first + i);
+        if (i < n)
             s.item[i] = (uint64_t)(first + i) << 32 |
-                        morton2(quantize_axis((double)xy.x, rb.cx, rb.half),
-                                quantize_axis((double)xy.y, rb.cy, rb.half));
-        }
+                        morton2(quantize_axis((double)xy[r].x, rb.cx, rb.half),
+                                quantize_axis((double)xy[r].y, rb.cy, rb.half));
     }
-    if (CLUSTER) cluster_wait();  // every block runs: its shared memory may be written
     // a warp reads back only its own positions until the places are known
 #pragma unroll 1
     for (uint32_t shift = 0; shift < 32u; shift += 8u) {
@@ -1164,6 +1235,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
             plan.cuts[cut] = s.cut[t] & 0xffffu;
         if (block == 0 && t == 0) plan.cuts[plan.blocks] = npos;
         if (block == 0 && t < plan.ranges) plan.inner_n[t] = 0;
+        if (block == 0 && t == 0) *plan.outer_n = 0;
     }
 }
 
@@ -3045,7 +3117,7 @@ static SortForm sort_form(const BatchBuffers& b) {
 bool small_sort(const BatchBuffers& b) { return sort_form(b).log != 0; }
 
 template <int LOG, bool SCAN, bool CLUSTER>
-static cudaError_t sort_small(const BatchBuffers& b, uint32_t cluster, cudaStream_t s) {
+static cudaError_t sort_small(const BatchBuffers& b, int mode, uint32_t cluster, cudaStream_t s) {
     auto kernel = k_sort_small<LOG, SCAN, CLUSTER>;
     constexpr int bytes = (int)sizeof(SmallSort<LOG>);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
@@ -3053,23 +3125,23 @@ static cudaError_t sort_small(const BatchBuffers& b, uint32_t cluster, cudaStrea
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     return launch_clusters(kernel, cluster, b.nsims * cluster, kSmallThreads, bytes, s, b.sims,
-                           b.minmax, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
+                           mode, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
 }
 
 template <int LOG>
-static cudaError_t sort_small(const BatchBuffers& b, uint32_t cluster, cudaStream_t s) {
+static cudaError_t sort_small(const BatchBuffers& b, int mode, uint32_t cluster, cudaStream_t s) {
     if (b.nsims == 1)
-        return cluster == 1 ? sort_small<LOG, true, false>(b, cluster, s)
-                            : sort_small<LOG, true, true>(b, cluster, s);
-    return cluster == 1 ? sort_small<LOG, false, false>(b, cluster, s)
-                        : sort_small<LOG, false, true>(b, cluster, s);
+        return cluster == 1 ? sort_small<LOG, true, false>(b, mode, cluster, s)
+                            : sort_small<LOG, true, true>(b, mode, cluster, s);
+    return cluster == 1 ? sort_small<LOG, false, false>(b, mode, cluster, s)
+                        : sort_small<LOG, false, true>(b, mode, cluster, s);
 }
 
-cudaError_t launch_sort_small(const BatchBuffers& b, cudaStream_t s) {
+cudaError_t launch_sort_small(const BatchBuffers& b, int mode, cudaStream_t s) {
     const SortForm f = sort_form(b);
-    return f.log == 10   ? sort_small<10>(b, f.cluster, s)
-           : f.log == 11 ? sort_small<11>(b, f.cluster, s)
-                         : sort_small<12>(b, f.cluster, s);
+    return f.log == 10   ? sort_small<10>(b, mode, f.cluster, s)
+           : f.log == 11 ? sort_small<11>(b, mode, f.cluster, s)
+                         : sort_small<12>(b, mode, f.cluster, s);
 }
 
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
