@@ -978,7 +978,7 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
             tl.sim = s;
             tl.start = L.off[s] + t0;
             tl.count = std::min<uint32_t>(kTile, counts[s] - t0);
-            // 4 KB per group of simulations above kTile bodies: agg_region has 96
+            // 8 KB per group of simulations above kTile bodies: agg_region has 96
             tl.group = counts[s] <= kTile ? kNone : group + t0 / (kTile * kGroupTiles);
             b->h_tiles.push_back(tl);
             ++tile;
@@ -1219,6 +1219,7 @@ static int tree_fit(bh_tree* tree, const bh_config* cfg) {
     if ((rc = batch_build(tree->dev, &tree->st, cfg, 1, &nb))) return rc;
     nb->bb.radix_bits = tree->batch->bb.radix_bits;  // keep the tree's tuning
     nb->bb.trav_warps = tree->batch->bb.trav_warps;
+    nb->bb.clusters = tree->batch->bb.clusters;
     delete tree->batch;
     tree->batch = nb;
     tree->built = false;

@@ -17,7 +17,8 @@ constexpr uint32_t kTile = kSortThreads * kSortItems;  // keys per radix tile (4
 constexpr int kRadixDigits = 256;
 constexpr int kRadixPasses = 4;
 constexpr uint32_t kGroupTiles = 32;  // tiles whose digit counts are also summed together
-constexpr uint32_t kGroupStride = kRadixPasses * kRadixDigits;  // a group's words, all passes
+constexpr uint32_t kGroupWords = kRadixPasses * kRadixDigits;  // a group's counts, all passes
+constexpr uint32_t kGroupStride = 2u * kGroupWords;  // and the sums through it
 constexpr int kScanThreads = 256;
 constexpr int kScanItems = 4;  // 1024-position scan tiles: a shorter per-tile chain
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // positions per scan tile

@@ -507,33 +507,31 @@ constexpr int kLookWindow = GBH_LOOK_WINDOW;  // counts loaded per look-back rou
 constexpr uint32_t kCountBits = 20;
 constexpr uint32_t kCountMask = (1u << kCountBits) - 1u;
 static_assert(kGroupTiles * kTile <= kCountMask, "a group's count fits its bits");
+constexpr uint32_t kPrefix = 1u << 31;  // marks a published prefix
 
 // Look-back for one digit: the counts of the `tiles` tiles of the group before
-// this one (tile_words[i * stride]) and of the `groups` groups before it
-// (group_words[i * kGroupStride]), kLookWindow loads per round trip, each window
-// polled until it is published.  No tile waits for another's look-back, only for
-// its count.  The wait is bounded: once `limit` clock cycles have passed since it
-// began and a count is missing, it sets kErrLookbackTimeout and returns the sum of
-// the windows before, which is at most the true prefix (the caller's writes stay
-// in range).
+// this one (tile_words[i * stride]), then of the `groups` groups before it, the
+// nearest first (group_words[-i * kGroupStride], i from 1), up to the first whose
+// last tile has published the sum through it (kPrefix | sum, kGroupWords further).
+// kLookWindow loads per round trip, polled until they are published.  The wait is
+// bounded: once `limit` clock cycles have passed since it began and a count is
+// missing, it sets kErrLookbackTimeout and returns the sum so far, which is at most
+// the true prefix (the caller's writes stay in range).
 __device__ __forceinline__ uint32_t lookback_digit(const uint32_t* tile_words, uint32_t stride,
                                                    uint32_t tiles, const uint32_t* group_words,
                                                    uint32_t groups, uint32_t* err,
                                                    long long limit) {
     uint32_t excl = 0;
     const long long t0 = clock64();
-    for (uint32_t i0 = 0; i0 < tiles + groups; i0 += kLookWindow) {
+    for (uint32_t i0 = 0; i0 < tiles; i0 += kLookWindow) {
         uint32_t sum;
         bool all;
         do {
             uint32_t f[kLookWindow];
 #pragma unroll
-            for (int j = 0; j < kLookWindow; ++j) {
-                const uint32_t i = i0 + j;
-                f[j] = i < tiles            ? ld_volatile(tile_words + (size_t)i * stride)
-                       : i < tiles + groups ? ld_volatile(group_words + (size_t)(i - tiles) * kGroupStride)
-                                            : kGroupTiles << kCountBits;
-            }
+            for (int j = 0; j < kLookWindow; ++j)
+                f[j] = i0 + j < tiles ? ld_volatile(tile_words + (size_t)(i0 + j) * stride)
+                                      : kGroupTiles << kCountBits;
             sum = 0;
             all = true;
 #pragma unroll
@@ -547,6 +545,32 @@ __device__ __forceinline__ uint32_t lookback_digit(const uint32_t* tile_words, u
             }
         } while (!all);
         excl += sum;
+    }
+    constexpr int kGroupWindow = kLookWindow / 2;
+    for (uint32_t i0 = 1; i0 <= groups;) {
+        uint32_t f[kGroupWindow], prefix[kGroupWindow];
+#pragma unroll
+        for (int j = 0; j < kGroupWindow; ++j) {
+            const uint32_t* at = group_words - (size_t)min(i0 + j, groups) * kGroupStride;
+            f[j] = ld_volatile(at);
+            prefix[j] = ld_volatile(at + kGroupWords);
+        }
+        bool ready = true, done = false;
+        uint32_t used = 0;
+#pragma unroll
+        for (int j = 0; j < kGroupWindow; ++j) {
+            if (done || !ready || i0 + j > groups) continue;
+            done = (prefix[j] & kPrefix) != 0u;
+            ready = done || f[j] >> kCountBits == kGroupTiles;
+            if (ready) excl += done ? prefix[j] & ~kPrefix : f[j] & kCountMask;
+            used += ready;
+        }
+        if (done) break;
+        i0 += used;
+        if (!ready && clock64() - t0 > limit) {
+            set_err(err, kErrLookbackTimeout);
+            break;
+        }
     }
     return excl;
 }
@@ -570,14 +594,16 @@ __global__ void k_wait_probe(const uint32_t* flags, uint32_t* err, long long lim
 // code, as Rust's sort_by_key (nbody/src/flat.rs:233-234).
 // A tile's counts go to its own words and, added, to those of its group of
 // kGroupTiles tiles, so its look-back reads at most 31 tiles and the groups before
-// it, 16 words a round trip, where a chain of tiles advanced 8 a round trip: 2^20
-// bodies' four passes 80 -> 74 us, 2^18 51 -> 47.  What is left, in cycles of a tile
-// at 2^20 (2 tiles an SM): loads 2,500, ranking 4,000 to 5,000, waiting for the
-// slowest of the tiles before it 5,000 to 9,000, scans and the local scatter 3,000,
-// stores 2,000, and in the last pass the gather of a random 32-byte sector a body,
-// 20,000 of them (with its loads issued together and no store of the values, which
-// the bodies' records carry, 74 -> 70 us).  Counting with shared atomics before the
-// ranking, to publish earlier, costs more than it saves (76 us; 2^18 57).
+// it up to a known prefix, 16 words a round trip, where a chain of tiles advanced 8
+// a round trip: 2^20 bodies' four passes 80 -> 74 us, 2^18 51 -> 47, 2^24 1,030 ->
+// 935 (1,062 without the groups' prefixes, and 1.5 us less then at 2^20).  What is
+// left, in cycles of a tile at 2^20 (2 tiles an SM): loads 2,500, ranking 4,000 to
+// 5,000, waiting for the slowest of the tiles before it 5,000 to 9,000, scans and
+// the local scatter 3,000, stores 2,000, and in the last pass the gather of a random
+// 32-byte sector a body, 20,000 (with its loads issued together and no store of the
+// values, which the bodies' records carry, 74 -> 71 us).  Counting with shared
+// atomics before the ranking, to publish earlier, costs more than it saves (76 us;
+// 2^18 57).
 // MINB tiles share an SM: 2 (up to 128 registers) for sorts of one wave,
 // 3 (80 registers) for sorts of many waves of tiles (large batches).
 template <int BITS, int PASS, bool LAST, int MINB>
@@ -660,8 +686,8 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
         atomicExch(flags + (size_t)t * kDig + d, kGroupTiles << kCountBits | run);
         atomicAdd(group, 1u << kCountBits | run);
         excl = lookback_digit(flags + (size_t)(t - in_group) * kDig + d, kDig, in_group,
-                              group - (size_t)(before / kGroupTiles) * kGroupStride,
-                              before / kGroupTiles, err, kSpinCycles);
+                              group, before / kGroupTiles, err, kSpinCycles);
+        if (in_group == kGroupTiles - 1u) atomicExch(group + kGroupWords, kPrefix | (excl + run));
     }
     uint32_t tot;
     const uint32_t h = owner ? hist[(size_t)tl.sim * kHistStride + PASS * kDig + d] : 0u;
