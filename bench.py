@@ -36,10 +36,10 @@ N_BODIES = 1 << 20
 THETA, EPS, G, BUCKET, DT, SEED = 0.5, 0.005, 1.0, 1, 5e-4, 7
 METRIC = "particle-steps/s"
 # DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) of integrate,
-# Morton, 4 radix passes, count/scan, cells and aggregate for one step at
+# Morton, 4 radix passes, count/scan and the aggregate kernels for one step at
 # N=2^20, from one capture of this bench's workload; re-measured whenever one
 # of those kernels changes
-BUILD_DRAM_BYTES_PER_STEP = 465.5e6
+BUILD_DRAM_BYTES_PER_STEP = 316.0e6
 WORKLOAD = "cold-collapse uniform disc N=2^20, eps=0.005, theta=0.5, bucket=1, dt=5e-4, seed 7"
 
 def algorithmic_bytes(c: float) -> dict:
@@ -54,10 +54,11 @@ def algorithmic_bytes(c: float) -> dict:
         # 4 stable 8-bit passes (4 + 4x16) plus positions and the sorted
         # gather (read 4 + 32, write 4 + 16), which the last pass performs
         "radix": 68.0 + 56.0,
-        # topology: read 4 B codes, write 64 B per cell
-        "topology": 4.0 + 64.0 * c,
-        # aggregates: read 64 B per cell + 16 B sorted body, write 32 B per cell
-        "aggregate": 16.0 + 96.0 * c,
+        # topology (cells per position and their scan): read 4 B codes
+        "topology": 4.0,
+        # cells and aggregates in one kernel: write 64 B per cell, read them and
+        # a 16 B sorted body, write 32 B per cell
+        "aggregate": 16.0 + 160.0 * c,
     }
 
 
@@ -754,7 +755,7 @@ def run_engine(args, world, rank, local, pg):
                                        "step's sort, build and leapfrog kernels on this workload "
                                        "(one capture, per step)",
                      "kernels": "sort/build/leapfrog (integrate+bounds, morton, 4 radix "
-                                "passes, count/scan, cells, aggregate)",
+                                "passes, count/scan, aggregates)",
                      "peak_source": peaks["source"],
                      "algorithmic_bytes_per_body": {k: round(v, 1) for k, v in ab.items()},
                      "stage_ms": {k: round(v * 1e3, 4) for k, v in stage.items()},
@@ -766,7 +767,7 @@ def run_engine(args, world, rank, local, pg):
                 "host_numa": numa.summary(), "wall_s": e2e_wall},
         "cpu_baseline": cpu,
         "clocks": clk,
-        "gpu_launches": 10 * args.steps + 1,
+        "gpu_launches": 11 * args.steps + 1,
         "summary": summary,
     }
     print(json.dumps(line), flush=True)
