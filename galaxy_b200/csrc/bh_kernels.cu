@@ -785,21 +785,21 @@ static_assert(kAggCutWindow == 32u * kScanItems && kAggPositions == 2u * kAggCut
               "the warps of k_count_scan find the cuts");
 // The cuts (one more than blocks, found with the chain counts) and the internal
 // cells that span one (from k_aggregate), as (cell, depth << 26 | simulation,
-// first position), at most one per cut and depth.  Every kAggRange-th cut is an outer cut: a list per range
-// between two of them, and one of the cells that span an outer cut.
-#ifndef GBH_AGG_RANGE
-#define GBH_AGG_RANGE 128
-#endif
-constexpr uint32_t kAggRange = GBH_AGG_RANGE;
-constexpr uint32_t kAggRangeCells = 16u * kAggRange;
+// first position), at most one per cut and depth.  Every range-th cut is an outer
+// cut: a list per `range` blocks between two of them, and one of the cells that span
+// an outer cut, which a single block combines.  128 blocks a range, but 256 above
+// 2^21 bodies or so, where that single block is the longer part: the aggregates of
+// 2^22 bodies 380 -> 359 us, of 2^24 1,385 -> 1,334, of 2^18 44 -> 46, of 700,001 95
+// -> 97.
+static uint32_t agg_range(uint32_t blocks) { return blocks > 8192u ? 256u : 128u; }
 struct AggPlan {
     uint32_t* cuts;
     uint32_t* inner_n;  // [range], zeroed with the chain counts
     uint32_t* outer_n;  // zeroed with the control block
-    uint4* inner;       // [range][kAggRangeCells]
+    uint4* inner;       // [range][16 blocks of a range]
     uint4* outer;       // [16 ranges]
     struct SpanCell* outer_cells;  // [16 ranges], with their links
-    uint32_t blocks, ranges;
+    uint32_t blocks, range, ranges;
 };
 
 constexpr unsigned long long kScanAgg = 1ull << 62;
@@ -1393,8 +1393,10 @@ __device__ __forceinline__ float2 store_cell(double4* cell_d, uint32_t k, const 
 // per SM.  Links and values read from global memory per cell, with a climb
 // through an acquire-release counter wherever a parent crossed a block, took
 // 156 us at 2^20 bodies (458 at 2^22, 61 at 2^14, 45 at 2^10); this and
-// the spanning cells' passes take 110 (331, 28, 20).  256 threads: 130 us at 2^20, 64:
-// 140; four lanes per cell: 168; cut windows of 64 and 256 positions: 112, 118.
+// the spanning cells' passes took 110 (331, 28, 20), and with the links as well,
+// for which a cells kernel took another 64 (239), 122 (361, 32, 22).  Before the
+// links, 256 threads: 130 us at 2^20, 64: 140; four lanes per cell: 168; cut windows
+// of 64 and 256 positions: 112, 118.
 #ifndef GBH_AGG_THREADS
 #define GBH_AGG_THREADS 128
 #endif
@@ -1499,8 +1501,8 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
     if (t <= (R1 - 1u) / 32u - chunk0) s.sim[t] = agg_sim(a, a.chunk_sim[chunk0 + t]);
     const uint32_t before = R0 > 0u ? a.codes[R0 - 1u] : 0u;
     const uint32_t after = R1 < npos ? a.codes[R1] : 0u;
-    const uint32_t range = blockIdx.x / kAggRange;
-    const uint32_t R2 = plan.cuts[min((range + 1u) * kAggRange, plan.blocks)];  // the outer cut
+    const uint32_t range = blockIdx.x / plan.range;
+    const uint32_t R2 = plan.cuts[min((range + 1u) * plan.range, plan.blocks)];  // the outer cut
     const uint32_t beyond = R2 < npos ? a.codes[R2] : 0u;
     if (t == 0) {
         s.depths = 0;
@@ -1537,7 +1539,7 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
                 if (si.end > R2 && shared_levels(code, beyond) >= d)
                     plan.outer[atomicAdd(plan.outer_n, 1u)] = rec;
                 else
-                    plan.inner[(size_t)range * kAggRangeCells + atomicAdd(plan.inner_n + range, 1u)] =
+                    plan.inner[(size_t)range * 16u * plan.range + atomicAdd(plan.inner_n + range, 1u)] =
                         rec;
             }
         }
@@ -1826,10 +1828,10 @@ __global__ void __launch_bounds__(kSpanThreads) k_aggregate_inner(const AggArgs 
         if (i < n) plan.outer_cells[i].load(a, plan.outer[i], kNone);
         return;
     }
-    const uint4* list = plan.inner + (size_t)r * kAggRangeCells;
-    const uint32_t n = min(plan.inner_n[r], kAggRangeCells);
+    const uint4* list = plan.inner + (size_t)r * 16u * plan.range;
+    const uint32_t n = min(plan.inner_n[r], 16u * plan.range);
     if (n == 0u) return;
-    const uint32_t outer_cut = plan.cuts[min((r + 1u) * kAggRange, plan.blocks)];
+    const uint32_t outer_cut = plan.cuts[min((r + 1u) * plan.range, plan.blocks)];
     combine_spans(a, n, [&](uint32_t i, SpanCell* c) { c->load(a, list[i], outer_cut); });
 }
 
@@ -3060,7 +3062,8 @@ cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s) {
 static AggPlan agg_plan(const BatchBuffers& b) {
     AggPlan p;
     p.blocks = (b.npos + kAggPositions - 1) / kAggPositions;
-    p.ranges = (p.blocks + kAggRange - 1) / kAggRange;
+    p.range = agg_range(p.blocks);
+    p.ranges = (p.blocks + p.range - 1) / p.range;
     p.outer_n = b.counters + 16;
     char* at = (char*)b.agg_region;
     auto take = [&](size_t bytes) {
