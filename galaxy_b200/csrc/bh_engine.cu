@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -78,7 +79,8 @@ extern "C" uint32_t galaxy_bh_abi_version(void) { return GALAXY_BH_ABI_VERSION; 
 // its first copy that uses them (about 8 ms, once).  Arrays that are pinned
 // already are copied as they are, and so are those below 16 MB: from 4 to 8 MB
 // the threads cost up to a fifth more than they save, at 12 MB 10 % less, and a
-// handle that moves no more than that need not pay for the slots.
+// handle that moves no more than that need not pay for the slots.  Two host
+// threads that copy their own states through one handle take the slots in turn.
 class HostCopies {
 public:
     // Returns once a device-to-host copy is complete; a host-to-device one may
@@ -90,7 +92,10 @@ public:
         const bool pageable = cudaPointerGetAttributes(&at, host) != cudaSuccess ||
                               at.type == cudaMemoryTypeUnregistered;
         cudaGetLastError();
-        if (!pageable || bytes < kStagedBytes || !ready())
+        const bool staged = pageable && bytes >= kStagedBytes;
+        std::unique_lock<std::mutex> slots(in_use_, std::defer_lock);
+        if (staged) slots.lock();
+        if (!staged || !ready())
             return cudaMemcpyAsync(dst, src, bytes,
                                    to_host ? cudaMemcpyDeviceToHost : cudaMemcpyHostToDevice, stream);
         const size_t chunks = (bytes + kChunk - 1) / kChunk;
@@ -123,7 +128,8 @@ public:
         for (auto& s : slots_)
             if (s.done) cudaEventDestroy(s.done);
         if (pinned_) cudaFreeHost(pinned_);
-        *this = HostCopies();
+        pinned_ = nullptr;
+        for (auto& s : slots_) s = Slot();
     }
 
 private:
@@ -193,6 +199,7 @@ private:
         return cudaSuccess;
     }
 
+    std::mutex in_use_;  // one copy at a time has the slots
     char* pinned_ = nullptr;
     Slot slots_[2 * kWorkers];
 };

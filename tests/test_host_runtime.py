@@ -1,0 +1,74 @@
+"""The engine's host side (bh_engine.cu) on a CPU: compiled as C++ against a fake
+CUDA runtime (fake_cuda.cpp), so that failing calls, error words and threads can
+be tried without a GPU."""
+import ctypes as C
+import os
+import subprocess
+import threading
+
+import numpy as np
+import pytest
+
+from galaxy_b200 import _lib, build
+from galaxy_b200.nbody_gpu import Config
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("fake") / "libhost.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread", "-I" + include,
+                    "-x", "c++", os.path.join(build.CSRC, "bh_engine.cu"),
+                    os.path.join(HERE, "fake_cuda.cpp"), "-o", so], check=True)
+    lib = C.CDLL(so)
+    for name, (res, args) in _lib.SIGNATURES.items():
+        if hasattr(lib, name):
+            fn = getattr(lib, name)
+            fn.restype, fn.argtypes = res, args
+    lib.fake_queued.restype = C.c_uint64
+    return lib
+
+
+@pytest.fixture
+def device(fake):
+    fake.fake_reset()
+    dev = C.c_void_p()
+    assert fake.galaxy_bh_device_open(0, C.byref(dev)) == _lib.BH_OK
+    yield dev
+    fake.fake_reset()
+    fake.galaxy_bh_device_close(dev)
+
+
+def new_state(fake, dev, records):
+    st = C.c_void_p()
+    assert fake.galaxy_bh_state_create(dev, _lib.ptr(records), len(records), C.byref(st),
+                                       None) == _lib.BH_OK
+    return st
+
+
+def test_two_threads_on_one_handle_read_their_own_states(fake, device):
+    """Large pageable arrays go through the handle's pinned slots: two threads
+    that read two states at once through one handle each get their own."""
+    n = (16 << 20) // 32 + 5
+    records = [np.zeros((n, 8), np.float32) for _ in range(2)]
+    for k, r in enumerate(records):
+        r[:] = 1.0 + k + np.arange(n, dtype=np.float32)[:, None] / n
+    states = [new_state(fake, device, r) for r in records]
+    wrong = [0, 0]
+
+    def read(k):
+        out = np.empty_like(records[k])
+        for _ in range(6):
+            assert fake.galaxy_bh_read_state(device, states[k], _lib.ptr(out), n, None) == 0
+            wrong[k] += not np.array_equal(out, records[k])
+
+    threads = [threading.Thread(target=read, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for st in states:
+        fake.galaxy_bh_state_destroy(st)
+    assert wrong == [0, 0]
