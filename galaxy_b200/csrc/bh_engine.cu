@@ -1332,6 +1332,50 @@ extern "C" int galaxy_bh_force_f64(bh_device* dev, bh_state* st, bh_tree* tree,
     return BH_OK;
 }
 
+// The rest of a step behind a wait that gave up, on a small simulation: its tree
+// is sound when the error word is set, so what runs reads nothing out of place, but
+// a rebuild has to leave the cells alone and a force to find nothing to sum.
+static int probe_stalled_step(bh_device* dev) {
+    constexpr uint32_t kBodies = 70000;  // sorted by tiles, with cells across outer cuts
+    std::vector<GpuEvolveState> records(kBodies);
+    for (uint32_t i = 0; i < kBodies; ++i) {
+        records[i] = GpuEvolveState{};
+        records[i].position_mass[0] = (float)(i * 2654435761u >> 8);
+        records[i].position_mass[1] = (float)(i * 40503u % 65536u);
+        records[i].position_mass[2] = 1.f;
+    }
+    const bh_config cfg{0.5, 1.0, 1.0, 4, 16, BH_FLAG_NO_STATS, 0};
+    bh_state* st = nullptr;
+    bh_tree* tree = nullptr;
+    int rc = galaxy_bh_state_create(dev, records.data(), kBodies, &st, nullptr);
+    if (!rc) rc = galaxy_bh_tree_create(dev, st, &cfg, &tree);
+    if (!rc) rc = galaxy_bh_tree_rebuild(dev, st, tree, &cfg, nullptr);
+    if (!rc) rc = galaxy_bh_force(dev, st, tree, &cfg, nullptr);
+    std::vector<uint32_t> accel(4 * (size_t)kBodies), cells(4 * (size_t)kBodies);
+    if (!rc) {
+        Batch* b = tree->batch;
+        cudaStream_t s = dev->stream;
+        const size_t bytes = 16ull * kBodies;
+        const uint32_t bits = kErrLookbackTimeout;
+        cudaError_t e;
+        if ((e = cudaMemsetAsync(b->bb.cell_u, 0x5a, bytes, s)) ||
+            (e = cudaMemcpyAsync(b->bb.err, &bits, 4, cudaMemcpyHostToDevice, s)))
+            rc = cuda_fail(e, "wait probe");
+        if (!rc) rc = enqueue_rebuild(b, 0, nullptr);
+        if (!rc) rc = enqueue_force(b, false);
+        if (!rc && ((e = cudaMemcpyAsync(accel.data(), st->d_accel, bytes, cudaMemcpyDeviceToHost, s)) ||
+                    (e = cudaMemcpyAsync(cells.data(), b->bb.cell_u, bytes, cudaMemcpyDeviceToHost, s))))
+            rc = cuda_fail(e, "wait probe");
+        if (!rc) rc = check_device_errors(b);
+        for (size_t k = 0; rc == BH_TIMEOUT && k < cells.size(); ++k)
+            if (cells[k] != 0x5a5a5a5au || accel[k] != 0u)
+                rc = set_error(BH_CUDA_ERROR, "wait probe: a step went on behind a wait that gave up");
+    }
+    if (tree) galaxy_bh_tree_destroy(tree);
+    if (st) galaxy_bh_state_destroy(st);
+    return rc;
+}
+
 extern "C" int galaxy_bh_wait_probe(bh_device* dev, uint64_t spin_cycles) {
     int rc = enter(dev);
     if (rc) return rc;
@@ -1351,9 +1395,11 @@ extern "C" int galaxy_bh_wait_probe(bh_device* dev, uint64_t spin_cycles) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
     cudaFree(d);
     if (e != cudaSuccess) return cuda_fail(e, "wait probe");
-    if (err & kErrLookbackTimeout)
-        return set_error(BH_TIMEOUT, "device wait (look-back) timed out (error bits 0x%x)", err);
-    return set_error(BH_CUDA_ERROR, "wait probe: the bounded wait did not report its timeout");
+    if (!(err & kErrLookbackTimeout))
+        return set_error(BH_CUDA_ERROR, "wait probe: the bounded wait did not report its timeout");
+    if ((rc = probe_stalled_step(dev)) != BH_TIMEOUT)
+        return rc ? rc : set_error(BH_CUDA_ERROR, "wait probe: a stalled step reported no timeout");
+    return set_error(BH_TIMEOUT, "device wait (look-back) timed out (error bits 0x%x)", err);
 }
 
 extern "C" int galaxy_bh_read_tree_evidence(bh_device* dev, bh_tree* tree, TreeMeta* meta,

@@ -83,6 +83,13 @@ __device__ __forceinline__ void wait_for_predecessor() {
 #endif
 }
 
+// Whether a wait of the step ran out.  The codes may be unsorted then and the
+// chains' sums short, and what the sort's passes and the aggregates read and write
+// by them could lie outside their arrays.
+__device__ __forceinline__ bool gave_up(const uint32_t* err) {
+    return (*err & kErrLookbackTimeout) != 0u;
+}
+
 // Order-preserving float <-> uint mapping (for integer atomics on floats).
 __device__ __forceinline__ uint32_t enc_f32(float f) {
     uint32_t u = __float_as_uint(f);
@@ -616,6 +623,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
     wait_for_predecessor();
     constexpr uint32_t kDig = 1u << BITS;
     __shared__ uint32_t s_tile;
+    __shared__ bool s_stop;
     __shared__ uint32_t s_whist[8][kDig];
     __shared__ uint32_t s_tprefix[kDig];
     __shared__ uint32_t s_out[kDig];
@@ -624,9 +632,14 @@ __global__ void __launch_bounds__(kSortThreads, MINB) k_radix_pass(
     __shared__ uint32_t s_scan[8];
 
     const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+    if (threadIdx.x == 0) {
+        s_tile = atomicAdd(tile_counter, 1u);
+        // in an earlier pass, or a tile of this one: read once, for the whole block
+        s_stop = gave_up(err);
+    }
     for (int k = threadIdx.x; k < 8 * (int)kDig; k += kSortThreads) (&s_whist[0][0])[k] = 0;
     __syncthreads();
+    if (s_stop) return;
     const uint32_t t = s_tile;
     const Tile tl = tiles[t];
     const SimDesc& sd = sims[tl.sim];
@@ -1334,6 +1347,7 @@ struct AggArgs {
     uint4* cell_u;
     double4* cell_d;
     CellRec* groups;
+    uint32_t nsims;
 };
 
 // The simulation a chunk of 32 positions belongs to, as the aggregates need it.
@@ -1486,6 +1500,7 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
     wait_for_predecessor();
     __shared__ AggShared s;
     const uint32_t t = threadIdx.x, lane = lane_id(), warp = t >> 5;
+    const bool stop = gave_up(err);  // (no block of this kernel sets that bit)
     const uint32_t R0 = plan.cuts[blockIdx.x], R1 = plan.cuts[blockIdx.x + 1u];
     const uint32_t npos = plan.cuts[plan.blocks];
     const uint32_t n = R1 - R0;
@@ -1510,6 +1525,14 @@ __global__ void __launch_bounds__(kAggThreads, GBH_AGG_MIN_BLOCKS)
         s.base[n] = a.base[R1];
     }
     __syncthreads();
+    if (stop) {
+        // no cells and no lists (the list passes find them empty), and root groups
+        // without a root: the traversal then has nothing to read
+        if (blockIdx.x == 0)
+            for (uint32_t k = t; k < 4u * a.nsims; k += kAggThreads)
+                a.groups[4ull * a.capacity + k].u = make_uint4(0u, 0u, 0u, kNone);
+        return;
+    }
     if (s.base[n] > a.capacity) {  // cannot be: the capacity bounds every tree
         if (t == 0) set_err(err, kErrCapacity);
         return;
@@ -3180,7 +3203,7 @@ cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
 
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s) {
     const AggArgs a{b.sims,          b.simout, b.chunk_sim, b.sbody,  b.keys_a,
-                    b.cell_capacity, b.base,   b.cell_u,    b.cell_d, b.groups};
+                    b.cell_capacity, b.base,   b.cell_u,    b.cell_d, b.groups, b.nsims};
     const AggPlan plan = agg_plan(b);
     cudaError_t e = launch_step(k_aggregate, plan.blocks, kAggThreads, 0, s, a, plan, b.err);
     if (e == cudaSuccess && plan.blocks > 1) {
