@@ -1239,6 +1239,7 @@ extern "C" int galaxy_bh_tree_rebuild(bh_device* dev, bh_state* st, bh_tree* tre
     if (rc) return rc;
     if ((rc = tree_fit(tree, cfg))) return rc;
     if ((rc = apply_configs(tree->batch, cfg, true))) return rc;
+    tree->built = false;  // until this rebuild has ended without an error
     if ((rc = enqueue_rebuild(tree->batch, 0, dev->ev))) return rc;
     CK(cudaStreamSynchronize(dev->stream), "rebuild");
     if ((rc = check_device_errors(tree->batch))) return rc;
@@ -1484,7 +1485,9 @@ extern "C" int galaxy_bh_step(bh_device* dev, bh_state* st, bh_tree* tree, const
     if ((rc = apply_configs(tree->batch, cfg, true))) return rc;
     tree->batch->built_theta = cfg->theta;
     tree->batch->built_g = cfg->g;
-    return run_graphs(tree->batch, nsteps);
+    rc = run_graphs(tree->batch, nsteps);
+    tree->built = rc == BH_OK;
+    return rc;
 }
 
 // ----------------------------------------------------------- packed (2B1) --

@@ -47,6 +47,7 @@ bool g_all_pinned = false, g_capturing = false;
 int g_fail_after = -1;       // fallible calls until one fails (-1: none does)
 uint32_t g_rebuild_err = 0;  // error bits that the next sorts set
 uint32_t g_packed_err = 0;   // and the packed walks
+uint32_t* g_step_err = nullptr;  // the error word of the steps captured last
 
 Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 
@@ -78,6 +79,7 @@ void fake_reset() {
     g_all_pinned = false;
     g_fail_after = -1;
     g_rebuild_err = g_packed_err = 0;
+    g_step_err = nullptr;
 }
 void fake_all_pinned(int on) { g_all_pinned = on != 0; }
 void fake_fail_after(int calls) { g_fail_after = calls; }
@@ -180,7 +182,11 @@ cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t* g) {
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t* g, cudaGraph_t, unsigned long long) {
     return *g = reinterpret_cast<cudaGraphExec_t>(1), cudaSuccess;
 }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) { return kernel(s); }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t s) {
+    return kernel(s, [] {
+        if (g_step_err) *g_step_err |= g_rebuild_err;
+    });
+}
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 }  // extern "C"
@@ -193,6 +199,7 @@ uint32_t conservation_blocks(uint32_t) { return 1; }
 cudaError_t launch_integrate(const BatchBuffers&, int, cudaStream_t s) { return kernel(s); }
 cudaError_t launch_morton(const BatchBuffers&, cudaStream_t s) { return kernel(s); }
 cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s) {
+    if (g_capturing) g_step_err = b.err;
     return kernel(s, [err = b.err] { *err |= g_rebuild_err; });
 }
 cudaError_t launch_sort_small(const BatchBuffers&, int, cudaStream_t s) { return kernel(s); }

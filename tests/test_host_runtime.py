@@ -72,3 +72,29 @@ def test_two_threads_on_one_handle_read_their_own_states(fake, device):
     for st in states:
         fake.galaxy_bh_state_destroy(st)
     assert wrong == [0, 0]
+
+
+def test_a_failed_rebuild_or_step_leaves_no_tree_to_use(fake, device):
+    """After a rebuild or a step that ended in an error the cells are not those of
+    the sums and codes beside them: nothing walks them until a rebuild succeeds."""
+    records = np.ones((100, 8), np.float32)
+    st, tree, cfg = new_state(fake, device, records), C.c_void_p(), C.byref(Config().to_c())
+    assert fake.galaxy_bh_tree_create(device, st, cfg, C.byref(tree)) == _lib.BH_OK
+    accel = np.zeros((100, 2))
+
+    def uses():
+        return [fake.galaxy_bh_force(device, st, tree, cfg, None),
+                fake.galaxy_bh_force_f64(device, st, tree, cfg, _lib.ptr(accel), None, None),
+                fake.galaxy_bh_read_tree_evidence(device, tree, None, None, None, 0, None, 0, None),
+                fake.galaxy_bh_step(device, st, tree, cfg, 1e-3, 1)]
+
+    for fail in (lambda: fake.galaxy_bh_tree_rebuild(device, st, tree, cfg, None),
+                 lambda: fake.galaxy_bh_step(device, st, tree, cfg, 1e-3, 1)):
+        assert fake.galaxy_bh_tree_rebuild(device, st, tree, cfg, None) == _lib.BH_OK
+        assert uses() == [_lib.BH_OK] * 4
+        fake.fake_rebuild_error(1)  # the sort's wait gave up
+        assert fail() == _lib.BH_TIMEOUT
+        fake.fake_rebuild_error(0)
+        assert uses() == [_lib.BH_INVALID_ARG] * 4
+    fake.galaxy_bh_tree_destroy(tree)
+    fake.galaxy_bh_state_destroy(st)
