@@ -1382,25 +1382,30 @@ extern "C" int galaxy_bh_wait_probe(bh_device* dev, uint64_t spin_cycles) {
     if (rc) return rc;
     if (spin_cycles > (uint64_t)4000000000ull)
         return set_error(BH_INVALID_ARG, "spin_cycles above 4e9 (about two seconds)");
-    // flags of the never-published first tile, the error word, the results
-    constexpr size_t kWords = 2 * kRadixDigits + 1;
-    uint32_t* d = nullptr;
-    CK(cudaMalloc(&d, kWords * 4), "probe allocation");
-    cudaError_t e = cudaMemsetAsync(d, 0, kWords * 4, dev->stream);
+    // the words of the tile and of the groups before, two error words, the results
+    constexpr size_t kBefore = kRadixDigits + 2 * kGroupStride, kResults = 2 * kRadixDigits;
+    PoolBlock block(dev);
+    CK(block.get((kBefore + 2 + kResults) * 4), "probe allocation");
+    uint32_t* d = reinterpret_cast<uint32_t*>(block.at);
+    cudaError_t e = cudaMemsetAsync(d, 0, (kBefore + 2 + kResults) * 4, dev->stream);
     if (e == cudaSuccess)
-        e = launch_wait_probe(d, d + kRadixDigits, (long long)spin_cycles, d + kRadixDigits + 1,
-                              dev->stream);
-    uint32_t err = 0;
+        e = launch_wait_probe(d, d + kBefore, (long long)spin_cycles, d + kBefore + 2, dev->stream);
+    uint32_t got[2 + kResults] = {};
     if (e == cudaSuccess)
-        e = cudaMemcpyAsync(&err, d + kRadixDigits, 4, cudaMemcpyDeviceToHost, dev->stream);
+        e = cudaMemcpyAsync(got, d + kBefore, sizeof got, cudaMemcpyDeviceToHost, dev->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
-    cudaFree(d);
     if (e != cudaSuccess) return cuda_fail(e, "wait probe");
-    if (!(err & kErrLookbackTimeout))
-        return set_error(BH_CUDA_ERROR, "wait probe: the bounded wait did not report its timeout");
+    const uint32_t err = got[0] & got[1];
+    bool sums = true;  // each wait returns what had been published: nothing, and 1 a digit
+    for (size_t k = 0; k < kResults; ++k) sums = sums && got[2 + k] == k / kRadixDigits;
+    if (!(err & kErrLookbackTimeout) || !sums)
+        return set_error(BH_CUDA_ERROR, "wait probe: a bounded wait did not report its timeout");
     if ((rc = probe_stalled_step(dev)) != BH_TIMEOUT)
         return rc ? rc : set_error(BH_CUDA_ERROR, "wait probe: a stalled step reported no timeout");
-    return set_error(BH_TIMEOUT, "device wait (look-back) timed out (error bits 0x%x)", err);
+    return set_error(BH_TIMEOUT,
+                     "device waits (look-back over tiles, over tile groups) timed out (error bits "
+                     "0x%x)",
+                     err);
 }
 
 extern "C" int galaxy_bh_read_tree_evidence(bh_device* dev, bh_tree* tree, TreeMeta* meta,

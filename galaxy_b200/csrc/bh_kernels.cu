@@ -582,14 +582,21 @@ __device__ __forceinline__ uint32_t lookback_digit(const uint32_t* tile_words, u
     return excl;
 }
 
-// Failure-detection probe: the sort's look-back wait run as tile 1 of a
-// simulation whose first tile never publishes (flags all zero), one thread
-// per digit, so every thread must give up after `limit` cycles and report
-// the timeout.
-__global__ void k_wait_probe(const uint32_t* flags, uint32_t* err, long long limit,
-                             uint32_t* out) {
+// Failure-detection probe: the sort's look-back wait, one thread per digit, so
+// every thread must give up after `limit` cycles and report the timeout.  Block 0
+// waits as tile 1 of a simulation whose first tile never publishes, block 1 as the
+// first tile of the third group, behind a group that has published a count of 1 a
+// digit and one that never does.  words: zeros, kRadixDigits for the tile and
+// kGroupStride for each group; err and out: a word, and kRadixDigits, a block.
+__global__ void k_wait_probe(uint32_t* words, uint32_t* err, long long limit, uint32_t* out) {
     const uint32_t d = threadIdx.x;
-    out[d] = lookback_digit(flags + d, kRadixDigits, 1u, nullptr, 0u, err, limit);
+    if (blockIdx.x == 0) {
+        out[d] = lookback_digit(words + d, kRadixDigits, 1u, nullptr, 0u, err, limit);
+    } else {
+        uint32_t* group = words + kRadixDigits + 2u * kGroupStride + d;
+        atomicExch(group - kGroupStride, kGroupTiles << kCountBits | 1u);
+        out[kRadixDigits + d] = lookback_digit(nullptr, 0u, 0u, group, 2u, err + 1, limit);
+    }
 }
 
 // One stable BITS-wide LSD pass (BITS = 8: 4 passes, 4: 8 passes) over every
@@ -3216,9 +3223,9 @@ cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s) {
     return e;
 }
 
-cudaError_t launch_wait_probe(const uint32_t* flags, uint32_t* err, long long limit,
-                              uint32_t* out, cudaStream_t s) {
-    k_wait_probe<<<1, kRadixDigits, 0, s>>>(flags, err, limit > 0 ? limit : kSpinCycles, out);
+cudaError_t launch_wait_probe(uint32_t* words, uint32_t* err, long long limit, uint32_t* out,
+                              cudaStream_t s) {
+    k_wait_probe<<<2, kRadixDigits, 0, s>>>(words, err, limit > 0 ? limit : kSpinCycles, out);
     return cudaGetLastError();
 }
 

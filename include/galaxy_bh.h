@@ -128,15 +128,15 @@ typedef struct bh_batch bh_batch;
 
 /* Copies the calling thread's last error message; returns its length. */
 size_t galaxy_bh_last_error(char* buf, size_t len);
-/* Failure-detection probe (no reference counterpart): runs the sort's
- * bounded look-back wait against a predecessor that never publishes, with a
- * limit of spin_cycles GPU clock cycles (0 = the production limit of 2e9,
- * about one second; at most 4e9), and then a rebuild and a force of a small
- * simulation of its own as they run behind a wait that gave up, which must
- * leave its cells alone and find nothing to sum.  Returns BH_TIMEOUT with the same
- * message a stalled sort reports, and leaves the device handle usable; any
- * other status means that the wait did not give up, or the step did not stop,
- * as designed. */
+/* Failure-detection probe (no reference counterpart): runs the sort's bounded
+ * look-back waits, for a tile and for a group of tiles, against predecessors
+ * that never publish, with a limit of spin_cycles GPU clock cycles (0 = the
+ * production limit of 2e9, about one second; at most 4e9), and then a rebuild
+ * and a force of a small simulation of its own as they run behind a wait that
+ * gave up, which must leave its cells alone and find nothing to sum.  Returns
+ * BH_TIMEOUT, as a stalled sort does, and leaves the device handle usable; any
+ * other status means that a wait did not give up, or the step did not stop, as
+ * designed. */
 int galaxy_bh_wait_probe(bh_device* dev, uint64_t spin_cycles);
 uint32_t galaxy_bh_abi_version(void);
 

@@ -211,7 +211,7 @@ cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
 }
 cudaError_t launch_aggregate(const BatchBuffers&, cudaStream_t s) { return kernel(s); }
 cudaError_t launch_refresh_mac(const BatchBuffers&, uint32_t, cudaStream_t s) { return kernel(s); }
-cudaError_t launch_wait_probe(const uint32_t*, uint32_t*, long long, uint32_t*, cudaStream_t s) {
+cudaError_t launch_wait_probe(uint32_t*, uint32_t*, long long, uint32_t*, cudaStream_t s) {
     return kernel(s);
 }
 cudaError_t launch_traverse(const BatchBuffers&, bool, bool, bool, bool, cudaStream_t s) {
