@@ -1545,18 +1545,23 @@ static int run_packed(bh_device* dev, const BhSettings* settings, const GpuBody*
     if ((e = launch_traverse_packed(d_s, d_b, d_e, d_c, n, cell_count, d_out, d_err, s)))
         return cuda_fail(e, "packed traversal");
     cudaEventRecord(dev->ev[2], s);
-    if (out && ((e = launch_check_records(d_out, 1, n, d_err + 2, s)) ||
-                (e = copy_down(dev, out, d_out, out_bytes))))
-        return cuda_fail(e, "acceleration readback");
-    cudaEventRecord(dev->ev[3], s);
+    if (out && (e = launch_check_records(d_out, 1, n, d_err + 2, s)))
+        return cuda_fail(e, "packed traversal");
+    // the error words first: a walk that failed leaves the caller's array alone
     if ((e = cudaMemcpyAsync(err, d_err, sizeof err, cudaMemcpyDeviceToHost, s)) ||
         (e = cudaStreamSynchronize(s)))
         return cuda_fail(e, "packed traversal");
+    float up = 0.f, walk = 0.f, down = 0.f;
+    if (out && !err[0]) {
+        cudaEventRecord(dev->ev[3], s);
+        if ((e = copy_down(dev, out, d_out, out_bytes))) return cuda_fail(e, "acceleration readback");
+        cudaEventRecord(dev->ev[4], s);
+        if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "acceleration readback");
+        cudaEventElapsedTime(&down, dev->ev[3], dev->ev[4]);
+    }
     if (timing) {
-        float up = 0.f, walk = 0.f, down = 0.f;
         cudaEventElapsedTime(&up, dev->ev[0], dev->ev[1]);
         cudaEventElapsedTime(&walk, dev->ev[1], dev->ev[2]);
-        if (out) cudaEventElapsedTime(&down, dev->ev[2], dev->ev[3]);
         *timing = bh_stage_timing{up * 1e-3, walk * 1e-3, down * 1e-3};
     }
     if (err[0] & kErrPackedStack)

@@ -98,3 +98,25 @@ def test_a_failed_rebuild_or_step_leaves_no_tree_to_use(fake, device):
         assert uses() == [_lib.BH_INVALID_ARG] * 4
     fake.galaxy_bh_tree_destroy(tree)
     fake.galaxy_bh_state_destroy(st)
+
+
+@pytest.mark.parametrize("bits,status", [(8, _lib.BH_CAPACITY_OVERFLOW), (16, _lib.BH_INVALID_ARG)])
+def test_a_refused_packed_tree_leaves_the_output_alone(fake, device, bits, status):
+    """A walk that meets its stack's end or an index out of range gives no result."""
+    n = 40
+    settings = np.zeros(1, _lib.BH_SETTINGS_DTYPE)
+    settings["info"][0, 0] = n
+    bodies, entries = np.zeros(n, _lib.GPU_BODY_DTYPE), np.zeros(n, _lib.GPU_ENTRY_DTYPE)
+    cells, out = np.zeros(3, _lib.GPU_CELL_DTYPE), np.full((n, 4), 7.0, np.float32)
+
+    def traverse():
+        return fake.galaxy_bh_traverse_packed(device, _lib.ptr(settings), _lib.ptr(bodies), n,
+                                              _lib.ptr(entries), _lib.ptr(cells), len(cells),
+                                              _lib.ptr(out), None)
+
+    fake.fake_packed_error(bits)
+    assert traverse() == status
+    assert (out == 7.0).all()
+    fake.fake_packed_error(0)
+    assert traverse() == _lib.BH_OK
+    assert (out == 0.0).all()
