@@ -231,9 +231,12 @@ static cudaError_t copy_up(bh_device* dev, void* device, const void* host, size_
 
 // Device memory of one call from the handle's pool (no device-wide
 // synchronisation, as cudaMalloc and cudaFree have), given back in stream order.
+// A call that returns before wait() has ended well (an error on the way) waits
+// here: what it has queued may still read or write the caller's arrays.
 struct PoolBlock {
     bh_device* dev;
     char* at = nullptr;
+    bool idle = false;  // nothing of the call is queued any more
     explicit PoolBlock(bh_device* d) : dev(d) {}
     PoolBlock(const PoolBlock&) = delete;
     PoolBlock& operator=(const PoolBlock&) = delete;
@@ -249,8 +252,15 @@ struct PoolBlock {
         if (e != cudaSuccess) at = nullptr;
         return e;
     }
+    cudaError_t wait() {
+        const cudaError_t e = cudaStreamSynchronize(dev->stream);
+        idle = e == cudaSuccess;
+        return e;
+    }
     ~PoolBlock() {
-        if (at) cudaFreeAsync(at, dev->stream);
+        if (!at) return;
+        cudaFreeAsync(at, dev->stream);
+        if (!idle) cudaStreamSynchronize(dev->stream);
     }
 };
 
@@ -720,7 +730,7 @@ extern "C" int galaxy_bh_direct_probes(bh_device* dev, bh_state* st, const bh_co
         e = launch_direct_probes(st->d_state, st->n, d_p, nprobes, cfg->softening, cfg->g, d_o,
                                  dev->stream);
     if (!e) e = copy_down(dev, out, d_o, 16ull * nprobes);
-    if (!e) e = cudaStreamSynchronize(dev->stream);
+    if (!e) e = block.wait();
     if (e) return cuda_fail(e, "direct probes");
     return BH_OK;
 }
@@ -1322,7 +1332,7 @@ extern "C" int galaxy_bh_force_f64(bh_device* dev, bh_state* st, bh_tree* tree,
     if (!e) e = copy_down(dev, accel, d_acc, 16 * n);
     if (!e && abs_sum) e = copy_down(dev, abs_sum, d_abs, 8 * n);
     if (!e) e = cudaMemcpyAsync(h_stats, d_stats, 24, cudaMemcpyDeviceToHost, dev->stream);
-    if (!e) e = cudaStreamSynchronize(dev->stream);
+    if (!e) e = block.wait();
     if (e) return cuda_fail(e, "f64 traversal");
     if (stats) {
         *stats = bh_force_stats{};
@@ -1393,7 +1403,7 @@ extern "C" int galaxy_bh_wait_probe(bh_device* dev, uint64_t spin_cycles) {
     uint32_t got[2 + kResults] = {};
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(got, d + kBefore, sizeof got, cudaMemcpyDeviceToHost, dev->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(dev->stream);
+    if (e == cudaSuccess) e = block.wait();
     if (e != cudaSuccess) return cuda_fail(e, "wait probe");
     const uint32_t err = got[0] & got[1];
     bool sums = true;  // each wait returns what had been published: nothing, and 1 a digit
@@ -1457,7 +1467,7 @@ extern "C" int galaxy_bh_read_tree_evidence(bh_device* dev, bh_tree* tree, TreeM
     if (!e && entries_bytes) e = copy_down(dev, entries, d_e, entries_bytes);
     if (!e && bodies_bytes) e = copy_down(dev, bodies, d_b, bodies_bytes);
     if (!e && cells_bytes) e = copy_down(dev, cells, d_c, cells_bytes);
-    if (!e) e = cudaStreamSynchronize(s);
+    if (!e) e = block.wait();
     if (e) return cuda_fail(e, "tree evidence");
     return BH_OK;
 }
@@ -1549,14 +1559,15 @@ static int run_packed(bh_device* dev, const BhSettings* settings, const GpuBody*
         return cuda_fail(e, "packed traversal");
     // the error words first: a walk that failed leaves the caller's array alone
     if ((e = cudaMemcpyAsync(err, d_err, sizeof err, cudaMemcpyDeviceToHost, s)) ||
-        (e = cudaStreamSynchronize(s)))
+        (e = block.wait()))
         return cuda_fail(e, "packed traversal");
     float up = 0.f, walk = 0.f, down = 0.f;
     if (out && !err[0]) {
+        block.idle = false;
         cudaEventRecord(dev->ev[3], s);
         if ((e = copy_down(dev, out, d_out, out_bytes))) return cuda_fail(e, "acceleration readback");
         cudaEventRecord(dev->ev[4], s);
-        if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "acceleration readback");
+        if ((e = block.wait())) return cuda_fail(e, "acceleration readback");
         cudaEventElapsedTime(&down, dev->ev[3], dev->ev[4]);
     }
     if (timing) {

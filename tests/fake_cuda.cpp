@@ -6,6 +6,7 @@
 // do nothing but set the error words that a test asks for.
 #include <cuda_runtime_api.h>
 
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <deque>
@@ -41,9 +42,9 @@ struct Event {
 };
 
 std::mutex g_mu;
-std::map<const char*, size_t> g_pinned;  // cudaMallocHost blocks
-std::deque<Stream*> g_streams;
-bool g_all_pinned = false, g_capturing = false;
+std::map<const char*, size_t> g_pinned;  // cudaMallocHost blocks, and a test's arrays
+bool g_capturing = false;
+std::atomic<int> g_transfers{0};  // queued copies from or to host memory
 int g_fail_after = -1;       // fallible calls until one fails (-1: none does)
 uint32_t g_rebuild_err = 0;  // error bits that the next sorts set
 uint32_t g_packed_err = 0;   // and the packed walks
@@ -53,7 +54,6 @@ Stream* of(cudaStream_t s) { return reinterpret_cast<Stream*>(s); }
 
 bool pinned(const void* p) {
     std::lock_guard<std::mutex> lk(g_mu);
-    if (g_all_pinned) return true;
     auto it = g_pinned.upper_bound(static_cast<const char*>(p));
     if (it == g_pinned.begin()) return false;
     --it;
@@ -76,21 +76,17 @@ cudaError_t kernel(cudaStream_t s, std::function<void()> op = [] {}) {
 // -- controls of the tests ----------------------------------------------------
 extern "C" {
 void fake_reset() {
-    g_all_pinned = false;
     g_fail_after = -1;
     g_rebuild_err = g_packed_err = 0;
     g_step_err = nullptr;
 }
-void fake_all_pinned(int on) { g_all_pinned = on != 0; }
+void fake_pin(const char* p, size_t n) { g_pinned[p] = n; }
+void fake_unpin(const char* p) { g_pinned.erase(p); }
 void fake_fail_after(int calls) { g_fail_after = calls; }
 int fake_failed() { return g_fail_after == -1; }  // after fake_fail_after: whether it did
 void fake_rebuild_error(uint32_t bits) { g_rebuild_err = bits; }
 void fake_packed_error(uint32_t bits) { g_packed_err = bits; }
-uint64_t fake_queued() {
-    uint64_t n = 0;
-    for (Stream* s : g_streams) n += s->ops.size();
-    return n;
-}
+int fake_transfers() { return g_transfers; }
 
 // -- the runtime ----------------------------------------------------------------
 cudaError_t cudaDriverGetVersion(int* v) { return *v = 0, cudaSuccess; }
@@ -134,8 +130,7 @@ cudaError_t cudaFreeAsync(void* p, cudaStream_t s) {
     return of(s)->add([p] { free(p); }), cudaSuccess;
 }
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
-    g_streams.push_back(new Stream());
-    return *s = reinterpret_cast<cudaStream_t>(g_streams.back()), cudaSuccess;
+    return *s = reinterpret_cast<cudaStream_t>(new Stream()), cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { return of(s)->run(~0ull), cudaSuccess; }
@@ -165,7 +160,11 @@ cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind
                             cudaStream_t s) {
     const cudaError_t e = fallible();
     if (e != cudaSuccess) return e;
-    of(s)->add([=] { memcpy(dst, src, n); });
+    ++g_transfers;
+    of(s)->add([=] {
+        memcpy(dst, src, n);
+        --g_transfers;
+    });
     if (kind != cudaMemcpyDeviceToDevice && !pinned(kind == cudaMemcpyHostToDevice ? src : dst))
         of(s)->run(~0ull);
     return cudaSuccess;

@@ -27,7 +27,7 @@ def fake(tmp_path_factory):
         if hasattr(lib, name):
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
-    lib.fake_queued.restype = C.c_uint64
+    lib.fake_pin.argtypes, lib.fake_unpin.argtypes = [C.c_void_p, C.c_size_t], [C.c_void_p]
     return lib
 
 
@@ -120,3 +120,49 @@ def test_a_refused_packed_tree_leaves_the_output_alone(fake, device, bits, statu
     fake.fake_packed_error(0)
     assert traverse() == _lib.BH_OK
     assert (out == 0.0).all()
+
+
+@pytest.mark.parametrize("name", ["packed", "into", "evidence", "f64", "probes"])
+def test_a_call_that_fails_leaves_no_transfer_behind(fake, device, name):
+    """Whichever CUDA call fails in one that takes device memory for its own length,
+    it returns with nothing queued that still reads or writes the caller's pinned
+    arrays."""
+    n, cfg = 64, Config().to_c()
+    st, tree, p = new_state(fake, device, np.ones((n, 8), np.float32)), C.c_void_p(), _lib.ptr
+    assert fake.galaxy_bh_tree_create(device, st, C.byref(cfg), C.byref(tree)) == _lib.BH_OK
+    assert fake.galaxy_bh_tree_rebuild(device, st, tree, C.byref(cfg), None) == _lib.BH_OK
+    settings = np.zeros(1, _lib.BH_SETTINGS_DTYPE)
+    settings["info"][0, 0] = n
+    bodies, entries = np.zeros(n, _lib.GPU_BODY_DTYPE), np.zeros(n, _lib.GPU_ENTRY_DTYPE)
+    cells, accel = np.zeros(n, _lib.GPU_CELL_DTYPE), np.zeros((n, 4), np.float32)
+    f64, abs_sum, probes = np.zeros((n, 2)), np.zeros(n), np.arange(n, dtype=np.uint32)
+    call = {
+        "packed": lambda: fake.galaxy_bh_traverse_packed(
+            device, p(settings), p(bodies), n, p(entries), p(cells), n, p(accel), None),
+        "into": lambda: fake.galaxy_bh_force_into(
+            device, st, p(settings), p(bodies), p(entries), p(cells), n, None),
+        "evidence": lambda: fake.galaxy_bh_read_tree_evidence(
+            device, tree, None, p(entries), p(bodies), n, p(cells), n, None),
+        "f64": lambda: fake.galaxy_bh_force_f64(device, st, tree, C.byref(cfg), p(f64),
+                                                p(abs_sum), None),
+        "probes": lambda: fake.galaxy_bh_direct_probes(device, st, C.byref(cfg), p(probes), n,
+                                                       p(f64)),
+    }[name]
+    arrays = [settings, bodies, entries, cells, accel, f64, abs_sum, probes]
+    for a in arrays:
+        fake.fake_pin(a.ctypes.data, a.nbytes)
+    assert (call(), fake.fake_transfers()) == (_lib.BH_OK, 0)
+    seen = []  # status and transfers left, by the call that failed
+    fake.fake_fail_after(0)
+    while True:
+        got = (call(), fake.fake_transfers())
+        if not fake.fake_failed():  # there are no more
+            break
+        seen.append(got)
+        fake.fake_fail_after(len(seen))
+    for a in arrays:
+        fake.fake_unpin(a.ctypes.data)
+    fake.galaxy_bh_tree_destroy(tree)
+    fake.galaxy_bh_state_destroy(st)
+    assert got == (_lib.BH_OK, 0)
+    assert len(seen) >= 3 and seen == [(_lib.BH_CUDA_ERROR, 0)] * len(seen)
