@@ -219,8 +219,27 @@ struct bh_device {
     // unmaps pages, which cost a serving loop seconds per burst of finished
     // requests and would stall it on its stager's work.
     cudaMemPool_t pool = nullptr;
+    // Memory that single calls take for their own length (PoolBlock).  It keeps at
+    // most kScratchKept of it: an export of 2^22 bodies takes 660 MB once.
+    cudaMemPool_t scratch = nullptr;
     HostCopies copies;
 };
+constexpr uint64_t kScratchKept = 256ull << 20;
+
+// Memory from one of the handle's pools; when it runs short, what they keep unused
+// is given back and tried again.
+static cudaError_t pool_alloc(bh_device* dev, cudaMemPool_t pool, void** at, size_t bytes) {
+    cudaError_t e = cudaMallocFromPoolAsync(at, bytes, pool, dev->stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        cudaStreamSynchronize(dev->stream);
+        cudaMemPoolTrimTo(dev->pool, 0);
+        cudaMemPoolTrimTo(dev->scratch, 0);
+        e = cudaMallocFromPoolAsync(at, bytes, pool, dev->stream);
+    }
+    if (e != cudaSuccess) *at = nullptr;
+    return e;
+}
 
 static cudaError_t copy_down(bh_device* dev, void* host, const void* device, size_t bytes) {
     return dev->copies.run(host, device, bytes, true, dev->stream, dev->ordinal);
@@ -229,7 +248,7 @@ static cudaError_t copy_up(bh_device* dev, void* device, const void* host, size_
     return dev->copies.run(device, host, bytes, false, dev->stream, dev->ordinal);
 }
 
-// Device memory of one call from the handle's pool (no device-wide
+// Device memory of one call from the handle's scratch pool (no device-wide
 // synchronisation, as cudaMalloc and cudaFree have), given back in stream order.
 // A call that returns before wait() has ended well (an error on the way) waits
 // here: what it has queued may still read or write the caller's arrays.
@@ -237,20 +256,13 @@ struct PoolBlock {
     bh_device* dev;
     char* at = nullptr;
     bool idle = false;  // nothing of the call is queued any more
+    bool large = false;  // more than the pool keeps: it gives memory back when waited for
     explicit PoolBlock(bh_device* d) : dev(d) {}
     PoolBlock(const PoolBlock&) = delete;
     PoolBlock& operator=(const PoolBlock&) = delete;
     cudaError_t get(size_t bytes) {
-        cudaError_t e = cudaMallocFromPoolAsync((void**)&at, bytes, dev->pool, dev->stream);
-        if (e == cudaErrorMemoryAllocation) {
-            // give back what the pool keeps unused, then retry
-            cudaGetLastError();
-            cudaStreamSynchronize(dev->stream);
-            cudaMemPoolTrimTo(dev->pool, 0);
-            e = cudaMallocFromPoolAsync((void**)&at, bytes, dev->pool, dev->stream);
-        }
-        if (e != cudaSuccess) at = nullptr;
-        return e;
+        large = bytes > kScratchKept;
+        return pool_alloc(dev, dev->scratch, (void**)&at, bytes);
     }
     cudaError_t wait() {
         const cudaError_t e = cudaStreamSynchronize(dev->stream);
@@ -260,7 +272,7 @@ struct PoolBlock {
     ~PoolBlock() {
         if (!at) return;
         cudaFreeAsync(at, dev->stream);
-        if (!idle) cudaStreamSynchronize(dev->stream);
+        if (!idle || large) cudaStreamSynchronize(dev->stream);
     }
 };
 
@@ -269,6 +281,7 @@ static void device_free(bh_device* dev) {
     cudaStreamSynchronize(dev->stream);
     dev->copies.release();
     if (dev->pool) cudaMemPoolDestroy(dev->pool);
+    if (dev->scratch) cudaMemPoolDestroy(dev->scratch);
     for (auto& ev : dev->ev) cudaEventDestroy(ev);
     cudaStreamDestroy(dev->stream);
     delete dev;
@@ -308,14 +321,18 @@ extern "C" int galaxy_bh_device_open(int ordinal, bh_device** out) {
     pool_props.allocType = cudaMemAllocationTypePinned;
     pool_props.location.type = cudaMemLocationTypeDevice;
     pool_props.location.id = ordinal;
-    const uint64_t keep = ~0ull;
+    const uint64_t keep = ~0ull, scratch_keep = kScratchKept;
     if ((e = cudaSetDevice(ordinal)) != cudaSuccess ||
         (e = cudaGetDeviceProperties(&d->prop, ordinal)) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaMemPoolCreate(&d->pool, &pool_props)) != cudaSuccess ||
         (e = cudaMemPoolSetAttribute(d->pool, cudaMemPoolAttrReleaseThreshold,
-                                     (void*)&keep)) != cudaSuccess) {
+                                     (void*)&keep)) != cudaSuccess ||
+        (e = cudaMemPoolCreate(&d->scratch, &pool_props)) != cudaSuccess ||
+        (e = cudaMemPoolSetAttribute(d->scratch, cudaMemPoolAttrReleaseThreshold,
+                                     (void*)&scratch_keep)) != cudaSuccess) {
         if (d->pool) cudaMemPoolDestroy(d->pool);
+        if (d->scratch) cudaMemPoolDestroy(d->scratch);
         if (d->stream) cudaStreamDestroy(d->stream);
         delete d;
         return cuda_fail(e, "device open");
@@ -457,22 +474,14 @@ extern "C" int galaxy_bh_state_create(bh_device* dev, const GpuEvolveState* host
     cudaEventRecord(dev->ev[0], dev->stream);
     cudaError_t e;
     std::vector<uint32_t> chunk(st->nchunks, 0u);
-    auto pool_alloc = [&](auto** ptr, size_t bytes) {
-        cudaError_t r = cudaMallocFromPoolAsync((void**)ptr, bytes, dev->pool, dev->stream);
-        if (r == cudaErrorMemoryAllocation) {
-            // give back what the pool keeps unused, then retry
-            cudaGetLastError();
-            cudaStreamSynchronize(dev->stream);
-            cudaMemPoolTrimTo(dev->pool, 0);
-            r = cudaMallocFromPoolAsync((void**)ptr, bytes, dev->pool, dev->stream);
-        }
-        return r;
+    auto take = [&](auto** ptr, size_t bytes) {
+        return pool_alloc(dev, dev->pool, (void**)ptr, bytes);
     };
-    if ((e = pool_alloc(&st->d_state, sizeof(GpuEvolveState) * (size_t)n)) ||
-        (e = pool_alloc(&st->d_accel, sizeof(float4) * (size_t)n)) ||
-        (e = pool_alloc(&st->d_sim, sizeof(SimDesc))) ||
-        (e = pool_alloc(&st->d_chunk_sim, sizeof(uint32_t) * st->nchunks)) ||
-        (e = pool_alloc(&st->d_minmax, 16)) || (e = pool_alloc(&st->d_check, 16))) {
+    if ((e = take(&st->d_state, sizeof(GpuEvolveState) * (size_t)n)) ||
+        (e = take(&st->d_accel, sizeof(float4) * (size_t)n)) ||
+        (e = take(&st->d_sim, sizeof(SimDesc))) ||
+        (e = take(&st->d_chunk_sim, sizeof(uint32_t) * st->nchunks)) ||
+        (e = take(&st->d_minmax, 16)) || (e = take(&st->d_check, 16))) {
         galaxy_bh_state_destroy(st);
         return cuda_fail(e, "evolving state allocation");
     }
@@ -910,18 +919,10 @@ static int batch_build(bh_device* dev, bh_state* const* states, const bh_config*
     // the arena comes from the device handle's stream-ordered pool, which
     // keeps released arenas and state buffers for reuse
     if (!b->arena) {
-        e = cudaMallocFromPoolAsync(&b->arena, b->arena_bytes, dev->pool, dev->stream);
-        if (e == cudaErrorMemoryAllocation) {
-            // give back what the pool keeps, then retry
-            cudaGetLastError();
-            cudaStreamSynchronize(dev->stream);
-            cudaMemPoolTrimTo(dev->pool, 0);
-            e = cudaMallocFromPoolAsync(&b->arena, b->arena_bytes, dev->pool, dev->stream);
-        }
+        e = pool_alloc(dev, dev->pool, &b->arena, b->arena_bytes);
         b->arena_capacity = b->arena_bytes;
     }
     if (e != cudaSuccess) {
-        b->arena = nullptr;
         delete b;
         return cuda_fail(e, "batch arena allocation");
     }
