@@ -3265,14 +3265,20 @@ static cudaError_t traverse_launch(const BatchBuffers& b, bool compensated, bool
 #undef GBH_TRAVERSE
 }
 
-// A softening whose square is subnormal (or zero) in some simulation of the
-// batch: the general form, at one block size.
+template <bool NORMAL>
+static cudaError_t traverse_warps(const BatchBuffers& b, bool compensated, bool potential,
+                                  bool stats, cudaStream_t s) {
+    if (b.trav_warps == 2) return traverse_launch<2, NORMAL>(b, compensated, potential, stats, s);
+    if (b.trav_warps == 4) return traverse_launch<4, NORMAL>(b, compensated, potential, stats, s);
+    return traverse_launch<kTravWarps, NORMAL>(b, compensated, potential, stats, s);
+}
+
+// The general form where the softening's square is subnormal (or zero) in some
+// simulation of the batch.
 static cudaError_t traverse_form(const BatchBuffers& b, bool compensated, bool potential,
                                  bool stats, cudaStream_t s) {
-    if (!b.normal_eps2) return traverse_launch<4, false>(b, compensated, potential, stats, s);
-    if (b.trav_warps == 2) return traverse_launch<2, true>(b, compensated, potential, stats, s);
-    if (b.trav_warps == 4) return traverse_launch<4, true>(b, compensated, potential, stats, s);
-    return traverse_launch<kTravWarps, true>(b, compensated, potential, stats, s);
+    return b.normal_eps2 ? traverse_warps<true>(b, compensated, potential, stats, s)
+                         : traverse_warps<false>(b, compensated, potential, stats, s);
 }
 
 cudaError_t launch_traverse(const BatchBuffers& b, bool compensated, bool plain, bool potential,
