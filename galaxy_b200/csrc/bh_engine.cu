@@ -1028,11 +1028,16 @@ static int upload_sims(Batch* b) {
     return BH_OK;
 }
 
-// Reads (and clears) the device error word; maps bits to a status.
-static int check_device_errors(Batch* b) {
-    uint32_t err = 0;
-    CK(cudaMemcpyAsync(&err, b->bb.err, 4, cudaMemcpyDeviceToHost, b->dev->stream), "readback");
+// Reads (and clears) the device error word; maps bits to a status.  stage_cycles
+// (or null): kStages words, as the last timed small sort left them.
+static int check_device_errors(Batch* b, uint32_t* stage_cycles = nullptr) {
+    uint32_t words[kStageCycles + kStages] = {};
+    CK(cudaMemcpyAsync(words, b->bb.err, stage_cycles ? sizeof words : 4, cudaMemcpyDeviceToHost,
+                       b->dev->stream),
+       "readback");
     CK(cudaStreamSynchronize(b->dev->stream), "stream synchronize");
+    const uint32_t err = words[0];
+    if (stage_cycles) std::copy_n(words + kStageCycles, kStages, stage_cycles);
     if (!err) return BH_OK;
     cudaMemsetAsync(b->bb.err, 0, 4, b->dev->stream);
     cudaStreamSynchronize(b->dev->stream);
@@ -1050,14 +1055,14 @@ enum Stage { kStBounds, kStMorton, kStRadix, kStTopology, kStAggregate };
 static int enqueue_rebuild(Batch* b, int integrate_mode, cudaEvent_t* ev) {
     cudaStream_t s = b->dev->stream;
     if (ev) CK(cudaEventRecord(ev[0], s), "event");
-    const bool small = small_sort(b->bb);  // one launch, timed as the radix stage
+    const bool small = small_sort(b->bb);  // one launch
     const bool scanned = small && b->bb.nsims == 1;
     if (!scanned) CK(cudaMemsetAsync(b->control, 0, b->control_bytes, s), "control memset");
     if (!small) CK(launch_integrate(b->bb, integrate_mode, s), "integrate launch");
     if (ev) CK(cudaEventRecord(ev[1], s), "event");
     if (!small) CK(launch_morton(b->bb, s), "morton launch");
     if (ev) CK(cudaEventRecord(ev[2], s), "event");
-    CK(small ? launch_sort_small(b->bb, integrate_mode, s) : launch_radix(b->bb, s), "radix launch");
+    CK(small ? launch_sort_small(b->bb, integrate_mode, ev != nullptr, s) : launch_radix(b->bb, s), "radix launch");
     if (ev) CK(cudaEventRecord(ev[3], s), "event");
     if (!scanned) CK(launch_count_scan(b->bb, s), "count/scan launch");
     if (ev) CK(cudaEventRecord(ev[4], s), "event");
@@ -1251,12 +1256,20 @@ extern "C" int galaxy_bh_tree_rebuild(bh_device* dev, bh_state* st, bh_tree* tre
     if ((rc = tree_fit(tree, cfg))) return rc;
     if ((rc = apply_configs(tree->batch, cfg, true))) return rc;
     tree->built = false;  // until this rebuild has ended without an error
-    if ((rc = enqueue_rebuild(tree->batch, 0, dev->ev))) return rc;
+    if ((rc = enqueue_rebuild(tree->batch, 0, timing ? dev->ev : nullptr))) return rc;
     CK(cudaStreamSynchronize(dev->stream), "rebuild");
-    if ((rc = check_device_errors(tree->batch))) return rc;
+    uint32_t cycles[kStages];
+    if ((rc = check_device_errors(tree->batch, cycles))) return rc;
     if (timing) {
         float ms[5];
         for (int k = 0; k < 5; ++k) cudaEventElapsedTime(&ms[k], dev->ev[k], dev->ev[k + 1]);
+        if (small_sort(tree->batch->bb)) {  // one launch: divided as its own cycles are
+            const float launch = ms[0] + ms[1] + ms[2] + ms[3];
+            double all = 0.0;
+            for (uint32_t c : cycles) all += c;
+            for (uint32_t k = 0; k < kStages; ++k)
+                ms[k] = all > 0.0 ? (float)(launch * (cycles[k] / all)) : 0.f;
+        }
         timing->bounds_seconds = ms[0] * 1e-3;
         timing->morton_seconds = ms[1] * 1e-3;
         timing->radix_seconds = ms[2] * 1e-3;

@@ -33,6 +33,9 @@ enum : uint32_t {
     kErrPackedStack = 8u,
     kErrPackedIndex = 16u,
 };
+// Words of the error region that follow the error word: the cycles of the four
+// stages that a timed k_sort_small does for a single simulation.
+constexpr uint32_t kStageCycles = 4, kStages = 4;
 
 // One simulation of a batch (the plain path is a batch of one).
 struct SimDesc {
@@ -133,7 +136,9 @@ cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s);
 // codes, sort and gather run as launch_sort_small, which needs no zeroed control
 // block and also does launch_count_scan's work for a single simulation.
 bool small_sort(const BatchBuffers& b);
-cudaError_t launch_sort_small(const BatchBuffers& b, int mode, cudaStream_t s);
+// timed: it also leaves the cycles of a single simulation's stages behind the
+// error word (kStageCycles).
+cudaError_t launch_sort_small(const BatchBuffers& b, int mode, bool timed, cudaStream_t s);
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s);
 cudaError_t launch_aggregate(const BatchBuffers& b, cudaStream_t s);
 // Recomputes G*m and the MAC bounds of simulation `sim` for new theta / G.

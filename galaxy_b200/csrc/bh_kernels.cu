@@ -1012,11 +1012,24 @@ __device__ __forceinline__ uint32_t small_scan(uint32_t v, uint32_t* warp_sum, u
     return x - v + (warp ? before : 0u);
 }
 
-template <int LOG, bool SCAN, bool CLUSTER>
+template <int LOG, bool SCAN, bool CLUSTER, bool TIMED>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     const SimDesc* __restrict__ sims, int mode, uint32_t npos, uint32_t* __restrict__ keys,
-    float4* __restrict__ sbody, uint32_t* __restrict__ base, const AggPlan plan, SimOut* simout) {
+    float4* __restrict__ sbody, uint32_t* __restrict__ base, const AggPlan plan, SimOut* simout,
+    uint32_t* __restrict__ stage_cycles) {
     wait_for_predecessor();
+    // TIMED: the stages in cycles of one thread: bounds, codes, sort with its
+    // gather, chain counts with their scan.  A form of its own, for rebuilds whose
+    // caller asks for times: the marks, and the gather done before the chain counts
+    // start, cost a step 0.2 to 0.8 us (16,384 bodies 91.7 -> 92.2).
+    uint32_t mark = TIMED ? (uint32_t)clock() : 0u;
+    auto stage_done = [&](int stage) {
+        if (TIMED && blockIdx.x == 0 && threadIdx.x == 0) {
+            const uint32_t now = (uint32_t)clock();
+            stage_cycles[stage] = now - mark;
+            mark = now;
+        }
+    };
     extern __shared__ float4 small_shared[];
     SmallSort<LOG>& s = *reinterpret_cast<SmallSort<LOG>*>(small_shared);
     constexpr int ITEMS = (1 << LOG) / kSmallThreads;
@@ -1104,6 +1117,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         gather(s.block_bounds, blocks);
     }
     const RootBounds rb = root_bounds(mnx, mny, mxx, mxy);
+    stage_done(0);
     if (t == 0 && block == 0) {
         simout[sim].cx = rb.cx;
         simout[sim].cy = rb.cy;
@@ -1118,6 +1132,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
                         morton2(quantize_axis((double)xy[r].x, rb.cx, rb.half),
                                 quantize_axis((double)xy[r].y, rb.cy, rb.half));
     }
+    stage_done(1);
     // a warp reads back only its own positions until the places are known
 #pragma unroll 1
     for (uint32_t shift = 0; shift < 32u; shift += 8u) {
@@ -1223,6 +1238,18 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
     for (int r = 0; r < ITEMS; ++r)
         if (i0 + 32u * r < n)
             pm[r] = __ldcg(reinterpret_cast<const float4*>(sd.state + (s.item[i0 + 32u * r] >> 32)));
+    auto store = [&](int r, uint32_t i) {
+        const uint64_t item = s.item[i];
+        keys[sd.off + first + i] = (uint32_t)item;
+        sbody[sd.off + first + i] =
+            make_float4(pm[r].x, pm[r].y, pm[r].z, __uint_as_float((uint32_t)(item >> 32)));
+    };
+    if constexpr (TIMED) {
+#pragma unroll
+        for (int r = 0; r < ITEMS; ++r)
+            if (i0 + 32u * r < n) store(r, i0 + 32u * r);
+        stage_done(2);
+    }
     uint32_t count[ITEMS], sum = 0;
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
@@ -1230,10 +1257,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         uint32_t cut = kNone;
         count[r] = 0;
         if (i < n) {
-            const uint64_t item = s.item[i];
-            const uint32_t v = (uint32_t)(item >> 32);
-            keys[sd.off + first + i] = (uint32_t)item;
-            sbody[sd.off + first + i] = make_float4(pm[r].x, pm[r].y, pm[r].z, __uint_as_float(v));
+            if (!TIMED) store(r, i);
             if (SCAN) {
                 uint32_t dmin;
                 count[r] = chain_count(codes, first + i, sd.n, sd.bucket, sd.max_depth, &dmin);
@@ -1283,6 +1307,7 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
         if (block == 0 && t < plan.ranges) plan.inner_n[t] = 0;
         if (block == 0 && t == 0) *plan.outer_n = 0;
     }
+    stage_done(3);
 }
 
 // =========================================================== aggregate ====
@@ -3117,7 +3142,7 @@ static uint32_t sort_cluster_limit() {
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 8;
     if (!cached[dev]) {
-        auto kernel = k_sort_small<12, true, true>;
+        auto kernel = k_sort_small<12, true, true, false>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = kSmallBlocks;
         cfg.blockDim = kSmallThreads;
@@ -3175,20 +3200,25 @@ static SortForm sort_form(const BatchBuffers& b) {
 
 bool small_sort(const BatchBuffers& b) { return sort_form(b).log != 0; }
 
-template <int LOG, bool SCAN, bool CLUSTER>
+template <int LOG, bool SCAN, bool CLUSTER, bool TIMED = false>
 static cudaError_t sort_small(const BatchBuffers& b, int mode, uint32_t cluster, cudaStream_t s) {
-    auto kernel = k_sort_small<LOG, SCAN, CLUSTER>;
+    auto kernel = k_sort_small<LOG, SCAN, CLUSTER, TIMED>;
     constexpr int bytes = (int)sizeof(SmallSort<LOG>);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e == cudaSuccess && cluster > 8)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     return launch_clusters(kernel, cluster, b.nsims * cluster, kSmallThreads, bytes, s, b.sims,
-                           mode, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout);
+                           mode, b.npos, b.keys_a, b.sbody, b.base, agg_plan(b), b.simout,
+                           b.err + kStageCycles);
 }
 
 template <int LOG>
-static cudaError_t sort_small(const BatchBuffers& b, int mode, uint32_t cluster, cudaStream_t s) {
+static cudaError_t sort_small(const BatchBuffers& b, int mode, bool timed, uint32_t cluster,
+                              cudaStream_t s) {
+    if (b.nsims == 1 && timed)
+        return cluster == 1 ? sort_small<LOG, true, false, true>(b, mode, cluster, s)
+                            : sort_small<LOG, true, true, true>(b, mode, cluster, s);
     if (b.nsims == 1)
         return cluster == 1 ? sort_small<LOG, true, false>(b, mode, cluster, s)
                             : sort_small<LOG, true, true>(b, mode, cluster, s);
@@ -3196,11 +3226,11 @@ static cudaError_t sort_small(const BatchBuffers& b, int mode, uint32_t cluster,
                         : sort_small<LOG, false, true>(b, mode, cluster, s);
 }
 
-cudaError_t launch_sort_small(const BatchBuffers& b, int mode, cudaStream_t s) {
+cudaError_t launch_sort_small(const BatchBuffers& b, int mode, bool timed, cudaStream_t s) {
     const SortForm f = sort_form(b);
-    return f.log == 10   ? sort_small<10>(b, mode, f.cluster, s)
-           : f.log == 11 ? sort_small<11>(b, mode, f.cluster, s)
-                         : sort_small<12>(b, mode, f.cluster, s);
+    return f.log == 10   ? sort_small<10>(b, mode, timed, f.cluster, s)
+           : f.log == 11 ? sort_small<11>(b, mode, timed, f.cluster, s)
+                         : sort_small<12>(b, mode, timed, f.cluster, s);
 }
 
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {

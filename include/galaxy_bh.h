@@ -98,7 +98,9 @@ typedef struct {
 } bh_stage_timing;
 
 /* ParallelTreeBuildTiming of nbody_parallel.rs:45-53 (seconds, device time
- * measured with CUDA events per stage). */
+ * measured with CUDA events per stage).  Up to 65,536 bodies one launch does the
+ * stages before the aggregates: its time is divided as the cycles that one of
+ * its threads spends in each. */
 typedef struct {
     double bounds_seconds;
     double morton_seconds;

@@ -201,7 +201,7 @@ cudaError_t launch_radix(const BatchBuffers& b, cudaStream_t s) {
     if (g_capturing) g_step_err = b.err;
     return kernel(s, [err = b.err] { *err |= g_rebuild_err; });
 }
-cudaError_t launch_sort_small(const BatchBuffers&, int, cudaStream_t s) { return kernel(s); }
+cudaError_t launch_sort_small(const BatchBuffers&, int, bool, cudaStream_t s) { return kernel(s); }
 cudaError_t launch_count_scan(const BatchBuffers& b, cudaStream_t s) {
     // every position a cell of its own
     return kernel(s, [base = b.base, n = b.npos] {
