@@ -1322,7 +1322,9 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
 // 4x margin and 1e-4 relative slack); in between the traversal decides in f64.
 // With r = u C/crit + 4 u the slack 4 r + 1e-4 on crit^2 and 4 u C crit beside
 // it make crit^2 (16 u + 1e-4) + 8 u C crit on either side of crit^2; here in
-// f32 with every rounding away from crit^2, so the band only widens.
+// f32 with every rounding away from crit^2, so the band only widens (checked in
+// exact arithmetic: it contains the band of the same formula in f64 for 200,000
+// critical distances of 1e-30 to 1e19 and centres of as many magnitudes).
 struct Crit {
     float up, down;  // width/theta rounded up and down; +inf at theta = 0
 };
@@ -1336,7 +1338,9 @@ __device__ __forceinline__ void mac_band(Crit root, uint32_t depth, float com_x,
     const float up2 = __fmul_ru(up, up);
     const float wide = __fmul_ru(__fmul_ru(up, 4.76837159e-7f), __fadd_ru(fabsf(com_x), fabsf(com_y)));
     const float down2 = __fmul_rd(down, down);
-    const bool always_open = !(down2 < 1e38f);  // beyond any f32 distance
+    // theta = 0.  (Past f32's end up2 is +inf and down2 its largest number: a
+    // smaller d2 opens, one that overflows is decided in f64.)
+    const bool always_open = down == INFINITY;
     *hi = always_open ? INFINITY : __fmaf_ru(up2, 1.000101f, wide);
     *lo = always_open ? INFINITY : __fmaf_rd(down2, 0.999899f, -wide);
 }
