@@ -1338,9 +1338,9 @@ __device__ __forceinline__ void mac_band(Crit root, uint32_t depth, float com_x,
     const float up2 = __fmul_ru(up, up);
     const float wide = __fmul_ru(__fmul_ru(up, 4.76837159e-7f), __fadd_ru(fabsf(com_x), fabsf(com_y)));
     const float down2 = __fmul_rd(down, down);
-    // theta = 0.  (Past f32's end up2 is +inf and down2 its largest number: a
-    // smaller d2 opens, one that overflows is decided in f64.)
-    const bool always_open = down == INFINITY;
+    // theta = 0.  (Past f32's end up2 is +inf, but down2, rounded down, its largest
+    // number: a smaller d2 opens, one that overflows is decided in f64.)
+    const bool always_open = !(down2 < INFINITY);
     *hi = always_open ? INFINITY : __fmaf_ru(up2, 1.000101f, wide);
     *lo = always_open ? INFINITY : __fmaf_rd(down2, 0.999899f, -wide);
 }
