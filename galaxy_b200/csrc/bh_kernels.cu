@@ -2765,9 +2765,10 @@ constexpr int kProbesPerBlock = 8;
 // nbody/src/lib.rs:315-329, over the f32 state promoted to f64): every term
 // is that of nbody/src/lib.rs:247-255 in f64, with the reciprocal square root and
 // fused multiply-adds where the reference divides 1 by a square root and rounds
-// each product (1 ulp either way); each thread sums a strided share of a slice of the sources, the block adds
-// the shares in a fixed order and k_add_slices the slices.  The slices (grid.y)
-// fill the chip whatever the number of probes: with every source in one block
+// each product: the root is within 1 ulp and enters three times, so a term differs
+// by a few ulp.  Each thread sums a strided share of a slice of the sources, the
+// block adds the shares in a fixed order and k_add_slices the slices.  The slices
+// (grid.y) fill the chip whatever the number of probes: with every source in one block
 // 4,096 probes were 512 blocks, 1.15 waves of the 444 resident ones, and 12
 // probes 2 blocks; 4,096 probes of 2^20 bodies, a whole call, 16.3 -> 10.0 ms.
 // The f64 pipe bounds it: with rsqrt for a square root and a division 9.1 -> 5.4 ms.
@@ -2832,9 +2833,10 @@ __global__ void __launch_bounds__(kProbeThreads) k_direct_probes(
 }
 
 // out[i] = the sum of the slices' values, in slice order; values[0] may be out.
-// Up to 512 of them one after the other would cost more than the rest of the sum
-// together (6e-16 against 4e-16 of the result), so each addition's rounding is
-// kept and added at the end (Knuth's two-sum).
+// There are up to 4,440 (512 with few probes of 2^20 bodies, 2,048 of 2^22), and one
+// after the other already 512 cost more than the rest of the sum together (6e-16
+// against 4e-16 of the result), so each addition's rounding is kept and added at the
+// end (Knuth's two-sum).
 __global__ void __launch_bounds__(256) k_add_slices(const double* values, uint32_t count,
                                                     uint32_t slices, double* out) {
     const uint32_t i = blockIdx.x * 256u + threadIdx.x;

@@ -260,10 +260,11 @@ int galaxy_bh_step(bh_device* dev, bh_state* st, bh_tree* tree, const bh_config*
 
 /* ---- FP64 direct-sum probes ---------------------------------------------------
  * direct_acceleration_for (nbody/src/lib.rs:315-329) on the device for
- * nprobes body indices of the resident state, in f64 with the reference's
- * per-term arithmetic (only the summation order is parallel).  out receives
- * ax, ay per probe (2*nprobes doubles, host memory); cfg supplies softening
- * and G.  The reference runs these probes on the CPU (probe_error,
+ * nprobes body indices of the resident state, in f64: the reference's formula
+ * per term, with a reciprocal square root (1 ulp) for its division by a square
+ * root and fused multiply-adds, so a term differs by a few ulp, and the terms
+ * summed in parallel.  out receives ax, ay per probe (2*nprobes doubles, host
+ * memory); cfg supplies softening and G.  The reference runs these probes on the CPU (probe_error,
  * nbody/src/lib.rs:370-395); the engine uses them to state the FP64 error of
  * every run. */
 int galaxy_bh_direct_probes(bh_device* dev, bh_state* st, const bh_config* cfg,
