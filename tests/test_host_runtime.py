@@ -19,7 +19,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 def fake(tmp_path_factory):
     so = str(tmp_path_factory.mktemp("fake") / "libhost.so")
     include = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread", "-I" + include,
+    # (-Bsymbolic: its own runtime, whatever other one the process has loaded)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-pthread",
+                    "-Wl,-Bsymbolic", "-I" + include,
                     "-x", "c++", os.path.join(build.CSRC, "bh_engine.cu"),
                     os.path.join(HERE, "fake_cuda.cpp"), "-o", so], check=True)
     lib = C.CDLL(so)
