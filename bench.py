@@ -39,13 +39,13 @@ METRIC = "particle-steps/s"
 # Morton, 4 radix passes, count/scan and the aggregate kernels for one step at
 # N=2^20, from one capture of this bench's workload; re-measured whenever one
 # of those kernels changes
-BUILD_DRAM_BYTES_PER_STEP = 316.0e6
+BUILD_DRAM_BYTES_PER_STEP = 322.0e6
 WORKLOAD = "cold-collapse uniform disc N=2^20, eps=0.005, theta=0.5, bucket=1, dt=5e-4, seed 7"
 
 def algorithmic_bytes(c: float) -> dict:
     """Bytes per body-step each HBM-bound stage must move (reads + writes) in
     the reference's record layout (32 B state, 16 B accel, 8 B key+index,
-    64 B cells); c = cells per body (measured).  Total 264 + 160c."""
+    64 B cells); c = cells per body (measured).  Total 264 + 96c."""
     return {
         # fused leapfrog + bounds partials: read 32 B state + 16 B accel, write 32 B
         "integrate": 80.0,
@@ -56,9 +56,9 @@ def algorithmic_bytes(c: float) -> dict:
         "radix": 68.0 + 56.0,
         # topology (cells per position and their scan): read 4 B codes
         "topology": 4.0,
-        # cells and aggregates in one kernel: write 64 B per cell, read them and
-        # a 16 B sorted body, write 32 B per cell
-        "aggregate": 16.0 + 160.0 * c,
+        # cells and aggregates in one kernel, the cells in shared memory between the
+        # two: read a 16 B sorted body, write 64 B and 32 B per cell
+        "aggregate": 16.0 + 96.0 * c,
     }
 
 
