@@ -219,12 +219,14 @@ struct bh_device {
     // unmaps pages, which cost a serving loop seconds per burst of finished
     // requests and would stall it on its stager's work.
     cudaMemPool_t pool = nullptr;
-    // Memory that single calls take for their own length (PoolBlock).  It keeps at
-    // most kScratchKept of it: an export of 2^22 bodies takes 660 MB once.
+    // Blocks above kSmallBlock that single calls take for their own length
+    // (PoolBlock): it keeps at most kScratchKept, an export of 2^22 bodies takes 660
+    // MB once.  Smaller ones come from `pool`, which mostly has room: a handle's
+    // first few probes would take 300 us longer from a pool that has none yet.
     cudaMemPool_t scratch = nullptr;
     HostCopies copies;
 };
-constexpr uint64_t kScratchKept = 256ull << 20;
+constexpr uint64_t kSmallBlock = 32ull << 20, kScratchKept = 256ull << 20;
 
 // Memory from one of the handle's pools; when it runs short, what they keep unused
 // is given back and tried again.
@@ -248,7 +250,7 @@ static cudaError_t copy_up(bh_device* dev, void* device, const void* host, size_
     return dev->copies.run(device, host, bytes, false, dev->stream, dev->ordinal);
 }
 
-// Device memory of one call from the handle's scratch pool (no device-wide
+// Device memory of one call from the handle's pools (no device-wide
 // synchronisation, as cudaMalloc and cudaFree have), given back in stream order.
 // A call that returns before wait() has ended well (an error on the way) waits
 // here: what it has queued may still read or write the caller's arrays.
@@ -262,7 +264,7 @@ struct PoolBlock {
     PoolBlock& operator=(const PoolBlock&) = delete;
     cudaError_t get(size_t bytes) {
         large = bytes > kScratchKept;
-        return pool_alloc(dev, dev->scratch, (void**)&at, bytes);
+        return pool_alloc(dev, bytes > kSmallBlock ? dev->scratch : dev->pool, (void**)&at, bytes);
     }
     cudaError_t wait() {
         const cudaError_t e = cudaStreamSynchronize(dev->stream);
