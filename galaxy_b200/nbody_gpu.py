@@ -85,7 +85,9 @@ class StageTiming:
 
 @dataclass
 class ParallelTreeBuildTiming:
-    """nbody_parallel.rs:45-64 (device stage times from CUDA events)."""
+    """nbody_parallel.rs:45-64 (device stage times from CUDA events; up to 65,536
+    bodies one launch does the stages before the aggregates, and its time is
+    divided as the cycles that one of its threads spends in each)."""
 
     bounds_seconds: float = 0.0
     morton_seconds: float = 0.0
