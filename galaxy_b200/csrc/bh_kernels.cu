@@ -1326,10 +1326,11 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(
 // exact arithmetic: it contains the band of the same formula in f64 for 200,000
 // critical distances of 1e-30 to 1e19 and centres of as many magnitudes).
 struct Crit {
-    float up, down;  // width/theta rounded up and down; +inf at theta = 0
+    float up, down;  // width/theta rounded up and down; +inf at theta = 0 and beyond f32
 };
 __device__ __forceinline__ Crit crit_f32(double crit) {
-    return Crit{__double2float_ru(crit), __double2float_rd(crit)};
+    const float up = __double2float_ru(crit);
+    return Crit{up, up < INFINITY ? __double2float_rd(crit) : INFINITY};
 }
 __device__ __forceinline__ void mac_band(Crit root, uint32_t depth, float com_x, float com_y,
                                          float* lo, float* hi) {
@@ -1338,8 +1339,9 @@ __device__ __forceinline__ void mac_band(Crit root, uint32_t depth, float com_x,
     const float up2 = __fmul_ru(up, up);
     const float wide = __fmul_ru(__fmul_ru(up, 4.76837159e-7f), __fadd_ru(fabsf(com_x), fabsf(com_y)));
     const float down2 = __fmul_rd(down, down);
-    // theta = 0.  (Past f32's end up2 is +inf, but down2, rounded down, its largest
-    // number: a smaller d2 opens, one that overflows is decided in f64.)
+    // theta = 0, or a root's width/theta beyond f32: every finite d2 opens.  (Past
+    // f32's end up2 is +inf, but down2, rounded down, its largest number: a smaller
+    // d2 opens.  One that overflows is decided in f64 in either case.)
     const bool always_open = !(down2 < INFINITY);
     *hi = always_open ? INFINITY : __fmaf_ru(up2, 1.000101f, wide);
     *lo = always_open ? INFINITY : __fmaf_rd(down2, 0.999899f, -wide);

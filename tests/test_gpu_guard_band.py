@@ -31,3 +31,22 @@ def test_decisions_equal_the_reference_near_the_end_of_f32(oracle, crit):
     want = oracle.flat_accelerations(b32, oracle.build_flat_tree(b32, oc), oc)[1]
     for key in ("visited_nodes", "approximated_cells", "direct_terms"):
         assert got[key] == want[key], key
+
+
+@pytest.mark.parametrize("theta", [1e-20, 1e-38, 1e-39, 1e-44])
+def test_tiny_angles_open_every_cell_without_the_f64_test(theta):
+    """A critical distance far beyond every body's, also beyond f32, opens each cell as
+    theta = 0 does, and no decision is left to f64."""
+    gpu = NbodyGpu("0")
+    rt = ParallelTreeRuntime(gpu)
+    bodies = scenarios.exponential_disc(2000, 5)
+    ev, _ = gpu.create_evolving_state(bodies)
+    got = []
+    for angle in (0.0, theta):
+        cfg = Config(theta=angle, softening_kpc=0.01, g=1.0, bucket=1)
+        tree = rt.create_tree(gpu, ev, cfg)
+        rt.rebuild(gpu, ev, tree, cfg)
+        rt.force(gpu, ev, tree, cfg)
+        got.append((rt.force_stats(gpu, tree), gpu.read_evolving_accelerations_f32(ev)[0].tobytes()))
+    assert got[0][0]["exact_mac_fallbacks"] == 0
+    assert got[0] == got[1]
